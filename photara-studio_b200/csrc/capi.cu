@@ -32,10 +32,14 @@ using namespace gsb;
 using namespace gsb::host;
 
 // Automatic compositing schedule: one pixel per thread up to this many 16x16
-// tiles, two up to kAutoPx2Tiles, four above (measured on B200: 256 tiles,
-// 1,200 tiles and 8,160 tiles).
+// tiles, then two, four, and eight (a warp per tile) above. Forward + adjoint,
+// us, at 1 / 2 / 4 / 8 pixels per thread: 256 tiles 158 / 233 / 290 / 488,
+// 690 tiles 161 / 152 / 161 / 214, 1,200 tiles 366 / 300 / 294 / 376, 3,600
+// tiles 732 / 553 / 461 / 480, 5,130 tiles 872 / 639 / 510 / 494, 8,160 tiles
+// 1205 / 860 / 665 / 602.
 constexpr int kAutoPx1Tiles = 600;
-constexpr int kAutoPx2Tiles = 2400;
+constexpr int kAutoPx2Tiles = 1000;
+constexpr int kAutoPx4Tiles = 4800;
 
 struct gs_context {
     int device = 0;
@@ -69,7 +73,8 @@ struct gs_context {
     float* pix_T = nullptr;
     unsigned* pix_last = nullptr;
     float* pix_dtdt = nullptr; // dT/dt at the median depth (geometry training forwards)
-    unsigned* tile_order = nullptr; // the last colour training forward's tiles, heaviest first
+    unsigned* work_lists = nullptr; // the last colour training forward's strips by adjoint work
+    int work_px = 0;                // its pixels per thread (the strips' shape)
     bool geometry = false;     // the last forward rendered the median-depth / normal channels
     const float* fwd_depth = nullptr;  // its median-depth and normal outputs (caller memory)
     const float* fwd_normal = nullptr;
@@ -121,14 +126,14 @@ template <typename F> gs_status guarded(gs_context* ctx, F&& f) {
 // Stage k: 0 preprocess, 1 depth sort + offset scan, 2 emit, 3 tile sort,
 // 4 ranges, 5 composite, 6 composite backward, 7 gaussian backward (+Adam).
 // Pixels per thread of the compositing kernels. Automatic (0): a frame's
-// compositing time is the longest tile's serial walk when there are too few
+// compositing time is the longest strip's serial walk when there are too few
 // tiles to fill the GPU, and fewer pixels per thread shorten that walk (more
-// threads share each tile); with many tiles, four pixels per thread amortise
-// the staging and the per-Gaussian setup best.
+// warps share each tile); with many tiles, more pixels per thread amortise the
+// per-Gaussian set-up and the adjoint's warp reduction best.
 int compositing_px(const gs_context* c, int tiles) {
     if (c->pixels_per_thread > 0)
         return c->pixels_per_thread;
-    return tiles <= kAutoPx1Tiles ? 1 : tiles <= kAutoPx2Tiles ? 2 : 4;
+    return tiles <= kAutoPx1Tiles ? 1 : tiles <= kAutoPx2Tiles ? 2 : tiles <= kAutoPx4Tiles ? 4 : 8;
 }
 
 void mark(gs_context* c, int stage, bool end) {
@@ -446,19 +451,19 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
         const size_t o_scan = carve(scan_status_bytes(n));
         const size_t o_dsort = carve(sort_status_bytes(size_t(n), 4));
         const size_t o_ctr = carve(16 * sizeof(unsigned));
-        // per-tile adjoint work (accumulated by the compositing) and the
-        // backward's tile order (heaviest first)
-        const size_t o_work = carve(size_t(tiles) * sizeof(unsigned));
-        const size_t o_order = carve(size_t(tiles) * sizeof(unsigned));
+        const int ppt = compositing_px(c, tiles);
+        // the strips by adjoint work, listed by the compositing; only the
+        // class counts at its start are zeroed
+        const size_t o_work = carve(kWorkListZeroed * sizeof(unsigned));
+        const size_t zeroed = frame;
+        frame = o_work + align_up(strip_order_words(tiles, ppt) * sizeof(unsigned));
         char* fb = c->ranges.ensure(frame, st);
-        unsigned* tile_work = reinterpret_cast<unsigned*>(fb + o_work);
-        unsigned* tile_order = reinterpret_cast<unsigned*>(fb + o_order);
-        c->tile_order = nullptr; // set below once the order is computed
+        c->work_lists = nullptr; // set below by a colour training forward
         unsigned* fctr = reinterpret_cast<unsigned*>(fb + o_ctr); // [0] compaction [1] scan
                                                                   // [2..6) depth sort passes
         unsigned* hist = reinterpret_cast<unsigned*>(fb + o_hist_d);
         mark(c, 1, false);
-        ck(cudaMemsetAsync(fb, 0, frame, st), "frame reset");
+        ck(cudaMemsetAsync(fb, 0, zeroed, st), "frame reset");
         launch_depth_compact(st, n, c->st, counters, c->dkeys[0], c->dvals[0], hist,
                              reinterpret_cast<unsigned long long*>(fb + o_compact), fctr + 0,
                              counters + 2, /*zeroed=*/true);
@@ -548,15 +553,14 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
                                       out->visibility, out->median_depth, out->normal);
         else {
             const bool train = s->record_backward_state != 0;
-            launch_composite_forward(st, tiles, reinterpret_cast<const uint2*>(c->ranges.p),
-                                     c->vals[cur], c->st, K, bg, out->color, out->alpha,
-                                     c->pix_T, c->pix_last, out->visibility,
-                                     compositing_px(c, tiles), record_staging(c),
-                                     train ? tile_work : nullptr);
             if (train) {
-                launch_tile_order(st, tile_work, tiles, tile_order);
-                c->tile_order = tile_order;
+                c->work_lists = reinterpret_cast<unsigned*>(fb + o_work);
+                c->work_px = ppt;
             }
+            launch_composite_forward(st, tiles, reinterpret_cast<const uint2*>(c->ranges.p),
+                                     c->vals[cur], K, bg, out->color, out->alpha, c->pix_T,
+                                     c->pix_last, out->visibility, ppt, record_staging(c),
+                                     c->work_lists);
         }
         ck(cudaGetLastError(), "composite launch");
         mark(c, 5, true);
@@ -642,8 +646,8 @@ gs_status gs_backward(gs_context* c, const float* fwd_alpha, const int* fwd_radi
                                       c->vals[c->sorted_buf], c->st, c->K, c->bg, c->pix_T,
                                       c->pix_last, dL->color, dL->alpha, dL->densify_map,
                                       grads && grads->refine_weight ? 1 : 0,
-                                      compositing_px(c, c->tiles), record_staging(c),
-                                      c->tile_order);
+                                      c->work_lists ? c->work_px : compositing_px(c, c->tiles),
+                                      record_staging(c), c->work_lists);
         ck(cudaGetLastError(), "composite backward launch");
         mark(c, 6, true);
         mark(c, 7, false);
@@ -916,8 +920,8 @@ gs_status gs_forward_colors(gs_context* c, const float* colors, const gs_outputs
         c->g.colors = colors;
         // empty tiles (ranges zeroed by the forward) composite the background
         launch_composite_forward(c->stream, c->tiles, reinterpret_cast<const uint2*>(c->ranges.p),
-                                 c->vals[c->sorted_buf], c->st, c->K, c->bg, out->color,
-                                 out->alpha, c->pix_T, c->pix_last, out->visibility,
+                                 c->vals[c->sorted_buf], c->K, c->bg, out->color, out->alpha,
+                                 c->pix_T, c->pix_last, out->visibility,
                                  compositing_px(c, c->tiles), record_staging(c));
         ck(cudaGetLastError(), "colour reuse composite launch");
     });

@@ -1,129 +1,71 @@
-// Single-view compositing kernels: one CTA per reference 16x16 tile running
-// the per-tile forward / adjoint of composite.cuh (numerics and organisation
+// Single-view compositing kernels: one warp per strip of a reference 16x16
+// tile running the forward / adjoint of strip.cuh (numerics and organisation
 // described there; reference: third_party/splat_drender/src/render_forward.cu
 // :341-416, :508-525 and render_backward.cu:156-519).
-#include "composite.cuh"
 #include "kernels.h"
+#include "strip.cuh"
 
 namespace gsb {
 
-// Single view: one CTA per reference 16x16 tile. kCount: the same forward
-// that also counts its evaluated pairs into *pairs.
-// The Gaussians of each batch are staged by TMA gathers of their 64-byte
-// records (`map`: the record array as a [rows][16] float tensor).
+// Resident warps per SM that the strip kernels are compiled for: the register
+// budget of each pixels-per-thread count without spills.
+template <int PX> constexpr int kForwardCtas = PX == 8 ? 20 : PX == 4 ? 28 : 32;
+template <int PX> constexpr int kBackwardCtas = PX == 8 ? 16 : PX == 4 ? 20 : 24;
+
+// One warp per strip of a reference 16x16 tile (256 / (32 PX) strips per
+// tile). kCount: the same forward that also counts its evaluated pairs.
 template <int PX, bool kCount = false>
-__global__ void __launch_bounds__(TileGeom<kTileW, kTileH, PX>::kThreads) composite_forward_kernel(
+__global__ void __launch_bounds__(32, kForwardCtas<PX>) composite_forward_kernel(
     const __grid_constant__ CUtensorMap map, unsigned* __restrict__ err,
-    const uint2* __restrict__ ranges, const unsigned* __restrict__ order, GaussianState st,
-    const Camera K, float3 bg, float* __restrict__ out_color, float* __restrict__ out_alpha,
+    const uint2* __restrict__ ranges, const unsigned* __restrict__ order, const Camera K,
+    float3 bg, float* __restrict__ out_color, float* __restrict__ out_alpha,
     float* __restrict__ pix_T, unsigned* __restrict__ pix_last, float* __restrict__ visibility,
-    unsigned* __restrict__ tile_work, unsigned long long* __restrict__ pairs = nullptr) {
-    using G = TileGeom<kTileW, kTileH, PX>;
-    __shared__ RecStage<G::kBatch> s;
-    __shared__ unsigned char s_vis[G::kBatch];
-    for (int k = threadIdx.x; k < G::kBatch; k += G::kThreads)
-        s_vis[k] = 0;
-    if (threadIdx.x == 0)
-        mbar_init(&s.bar, 1);
-    __syncthreads();
-    TmaGather g{&map, err, 0u};
-    const int tile = blockIdx.x;
+    StripOrder sched, unsigned long long* __restrict__ pairs = nullptr) {
+    constexpr int kStrips = kTileH / StripGeom<kTileW, PX>::kRows;
+    __shared__ StripStage s;
+    StripFeed feed{s, &map, err};
+    feed.init();
+    const int tile = int(blockIdx.x) / kStrips, strip = int(blockIdx.x) % kStrips;
     const ViewTarget o{K.width, K.height, K.alpha_clip, bg, out_color, out_alpha, pix_T, pix_last};
-    composite_forward_tile<kTileW, kTileH, PX, kCount>(s, s_vis, tile % K.grid_x,
-                                                       tile / K.grid_x, ranges[tile], order, st,
-                                                       o, visibility, pairs, &g,
-                                                       tile_work ? tile_work + tile : nullptr);
+    composite_forward_strip<kTileW, PX, kCount>(
+        feed, (tile % K.grid_x) * kTileW,
+        (tile / K.grid_x) * kTileH + strip * StripGeom<kTileW, PX>::kRows, ranges[tile], order, o,
+        visibility, sched, blockIdx.x, pairs);
 }
 
-// Four pixels per thread: capped at 96 registers (no spills) for 10 resident
-// CTAs per SM instead of 8 (0.700 -> 0.684 ms at 1M Gaussians, 1080p; the
-// 80-register cap for 12 CTAs spills and measured slower).
 template <int PX, bool kRefine, bool kDensify, bool kCount = false>
-__global__ void __launch_bounds__(TileGeom<kTileW, kTileH, PX>::kThreads, PX == 4 ? 10 : 1)
-    composite_backward_kernel(
+__global__ void __launch_bounds__(32, kBackwardCtas<PX>) composite_backward_kernel(
     const __grid_constant__ CUtensorMap map, unsigned* __restrict__ err,
-    const uint2* __restrict__ ranges, const unsigned* __restrict__ order, GaussianState st,
+    const uint2* __restrict__ ranges, const unsigned* __restrict__ order, float4* __restrict__ grad,
     const Camera K, float3 bg, const float* __restrict__ pix_T,
     const unsigned* __restrict__ pix_last, const float* __restrict__ dL_color,
-    const float* __restrict__ dL_alpha, const float* __restrict__ densify_map,
-    const unsigned* __restrict__ tile_order, unsigned long long* __restrict__ pairs = nullptr) {
-    using G = TileGeom<kTileW, kTileH, PX>;
-    using Stage = RecStage<G::kBatch>;
-    __shared__ BackStage<G::kBatch, Stage> sb;
-    __shared__ unsigned s_wmax[G::kWarps];
-    for (int k = threadIdx.x; k < G::kBatch * 12; k += G::kThreads)
-        (&sb.acc[0][0])[k] = 0.f;
-    if (threadIdx.x == 0)
-        mbar_init(&sb.s.bar, 1);
-    __syncthreads();
-    TmaGather g{&map, err, 0u};
-    // heaviest tiles first (tile_order: tiles by descending adjoint work),
-    // so the kernel's tail is made of the shortest tiles
-    const int tile = tile_order ? int(tile_order[blockIdx.x]) : int(blockIdx.x);
+    const float* __restrict__ dL_alpha, const float* __restrict__ densify_map, StripOrder sched,
+    unsigned long long* __restrict__ pairs = nullptr) {
+    constexpr int kStrips = kTileH / StripGeom<kTileW, PX>::kRows;
+    __shared__ StripStage s;
+    StripFeed feed{s, &map, err};
+    feed.init();
+    // heaviest strips first where the forward listed them
+    const unsigned at = sched.count ? strip_order_get(sched, blockIdx.x) : blockIdx.x;
+    if (at == 0xffffffffu)
+        return;
+    const int tile = int(at) / kStrips, strip = int(at) % kStrips;
     const ViewGrads o{K.width, K.height, K.alpha_clip, bg, pix_T, pix_last, dL_color, dL_alpha,
                       densify_map};
-    composite_backward_tile<kTileW, kTileH, PX, kRefine, kDensify, kCount, Stage>(
-        sb, s_wmax, tile % K.grid_x, tile / K.grid_x, ranges[tile], order, st, o, pairs, &g);
+    composite_backward_strip<kTileW, PX, kRefine, kDensify, kCount>(
+        feed, (tile % K.grid_x) * kTileW,
+        (tile / K.grid_x) * kTileH + strip * StripGeom<kTileW, PX>::kRows, ranges[tile], order, o,
+        grad, pairs);
 }
 
-// Tiles by descending adjoint work (a permutation of [0, tiles) whatever the
-// work values): one block, a counting sort on the work clamped to 4095.
-__global__ void __launch_bounds__(1024) tile_order_kernel(const unsigned* __restrict__ work,
-                                                          int tiles,
-                                                          unsigned* __restrict__ order) {
-    constexpr int kKeys = 4096;
-    __shared__ unsigned s_cnt[kKeys];
-    for (int k = threadIdx.x; k < kKeys; k += 1024)
-        s_cnt[k] = 0;
-    __syncthreads();
-    for (int t = threadIdx.x; t < tiles; t += 1024)
-        atomicAdd(&s_cnt[kKeys - 1 - min(work[t], unsigned(kKeys - 1))], 1u);
-    __syncthreads();
-    // exclusive scan of the 4096 counts (descending work first), four per thread
-    __shared__ unsigned s_warp[32];
-    unsigned v[4], sum = 0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        v[q] = s_cnt[4 * threadIdx.x + q];
-        sum += v[q];
-    }
-    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    unsigned incl = sum;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const unsigned y = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= unsigned(off))
-            incl += y;
-    }
-    if (lane == 31)
-        s_warp[w] = incl;
-    __syncthreads();
-    if (w == 0) {
-        unsigned x = s_warp[lane];
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= unsigned(off))
-                x += y;
-        }
-        s_warp[lane] = x;
-    }
-    __syncthreads();
-    unsigned run = incl - sum + (w ? s_warp[w - 1] : 0u);
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        s_cnt[4 * threadIdx.x + q] = run;
-        run += v[q];
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < tiles; t += 1024)
-        order[atomicAdd(&s_cnt[kKeys - 1 - min(work[t], unsigned(kKeys - 1))], 1u)] = unsigned(t);
+size_t strip_order_words(int tiles, int pixels_per_thread) {
+    return kWorkClasses * (1 + size_t(tiles) * size_t(8 / pixels_per_thread));
 }
 
-void launch_tile_order(cudaStream_t s, const unsigned* work, int tiles, unsigned* order) {
-    if (tiles > 0)
-        tile_order_kernel<<<1, 1024, 0, s>>>(work, tiles, order);
+static StripOrder strip_order(unsigned* words, int tiles, int pixels_per_thread) {
+    if (!words)
+        return {};
+    return {words, words + kWorkClasses, unsigned(tiles) * unsigned(8 / pixels_per_thread)};
 }
 
 // Test hook for the staging wait: one CTA announces 256 bytes on its
@@ -156,24 +98,24 @@ void launch_composite_count_pairs(cudaStream_t s, int tiles, const uint2* ranges
                                   const float* pix_T, const unsigned* pix_last,
                                   int pixels_per_thread, unsigned long long* pairs,
                                   const RecStaging& rs) {
-    // the forward writes pix_T / pix_last again with identical values; the
-    // count run leaves them as they were only if given the same buffers, so
-    // it writes no per-pixel state (NULL) and no visibility
+    // the count run writes no per-pixel state (NULL) and no visibility
     auto count = [&]<int PX>() {
-        constexpr int T = TileGeom<kTileW, kTileH, PX>::kThreads;
-        composite_forward_kernel<PX, true><<<tiles, T, 0, s>>>(
-            rs.map, rs.err, ranges, order, st, K, bg, color, alpha, nullptr, nullptr, nullptr,
-            nullptr, pairs);
-        composite_backward_kernel<PX, false, false, true><<<tiles, T, 0, s>>>(
-            rs.map, rs.err, ranges, order, st, K, bg, pix_T, pix_last, color, nullptr, nullptr,
-            nullptr, pairs + 1);
+        const int blocks = tiles * (8 / PX);
+        composite_forward_kernel<PX, true><<<blocks, 32, 0, s>>>(
+            rs.map, rs.err, ranges, order, K, bg, color, alpha, nullptr, nullptr, nullptr, {},
+            pairs);
+        composite_backward_kernel<PX, false, false, true><<<blocks, 32, 0, s>>>(
+            rs.map, rs.err, ranges, order, st.grad, K, bg, pix_T, pix_last, color, nullptr,
+            nullptr, {}, pairs + 1);
     };
     if (pixels_per_thread == 1)
         count.template operator()<1>();
     else if (pixels_per_thread == 2)
         count.template operator()<2>();
-    else
+    else if (pixels_per_thread == 4)
         count.template operator()<4>();
+    else
+        count.template operator()<8>();
 }
 
 // ------------------------------------------------- geometry channels ----
@@ -768,42 +710,23 @@ void launch_composite_backward_geometry(cudaStream_t s, int tiles, const uint2* 
 }
 
 void launch_composite_forward(cudaStream_t s, int tiles, const uint2* ranges,
-                              const unsigned* order, const GaussianState& st, const Camera& K,
-                              float3 bg, float* color, float* alpha, float* pix_T,
-                              unsigned* pix_last, float* visibility, int pixels_per_thread,
-                              const RecStaging& rs, unsigned* tile_work) {
+                              const unsigned* order, const Camera& K, float3 bg, float* color,
+                              float* alpha, float* pix_T, unsigned* pix_last, float* visibility,
+                              int pixels_per_thread, const RecStaging& rs, unsigned* work_lists) {
+    const StripOrder sched = strip_order(work_lists, tiles, pixels_per_thread);
     auto fwd = [&]<int PX>() {
-        composite_forward_kernel<PX><<<tiles, TileGeom<kTileW, kTileH, PX>::kThreads, 0, s>>>(
-            rs.map, rs.err, ranges, order, st, K, bg, color, alpha, pix_T, pix_last, visibility,
-            tile_work);
+        composite_forward_kernel<PX><<<tiles * (8 / PX), 32, 0, s>>>(
+            rs.map, rs.err, ranges, order, K, bg, color, alpha, pix_T, pix_last, visibility,
+            sched);
     };
     if (pixels_per_thread == 1)
         fwd.template operator()<1>();
     else if (pixels_per_thread == 2)
         fwd.template operator()<2>();
-    else if (pixels_per_thread == 8)
-        fwd.template operator()<8>();
-    else
+    else if (pixels_per_thread == 4)
         fwd.template operator()<4>();
-}
-
-template <int PX>
-static void launch_backward_px(cudaStream_t s, int tiles, const uint2* ranges,
-                               const unsigned* order, const GaussianState& st, const Camera& K,
-                               float3 bg, const float* pix_T, const unsigned* pix_last,
-                               const float* dL_color, const float* dL_alpha,
-                               const float* densify_map, int want_refine,
-                               const RecStaging& rs, const unsigned* tile_order) {
-    const int T = TileGeom<kTileW, kTileH, PX>::kThreads;
-#define GSB_BWD(R, D)                                                                            \
-    composite_backward_kernel<PX, R, D><<<tiles, T, 0, s>>>(rs.map, rs.err, ranges, order, st,   \
-                                                            K, bg, pix_T, pix_last, dL_color,    \
-                                                            dL_alpha, densify_map, tile_order)
-    if (want_refine && densify_map) GSB_BWD(true, true);
-    else if (want_refine) GSB_BWD(true, false);
-    else if (densify_map) GSB_BWD(false, true);
-    else GSB_BWD(false, false);
-#undef GSB_BWD
+    else
+        fwd.template operator()<8>();
 }
 
 void launch_composite_backward(cudaStream_t s, int tiles, const uint2* ranges,
@@ -811,23 +734,31 @@ void launch_composite_backward(cudaStream_t s, int tiles, const uint2* ranges,
                                float3 bg, const float* pix_T, const unsigned* pix_last,
                                const float* dL_color, const float* dL_alpha,
                                const float* densify_map, int want_refine, int pixels_per_thread,
-                               const RecStaging& rs, const unsigned* tile_order) {
+                               const RecStaging& rs, unsigned* work_lists) {
+    const StripOrder sched = strip_order(work_lists, tiles, pixels_per_thread);
+    auto bwd = [&]<int PX>() {
+        auto go = [&](auto kernel) {
+            kernel<<<tiles * (8 / PX), 32, 0, s>>>(rs.map, rs.err, ranges, order, st.grad, K, bg,
+                                                   pix_T, pix_last, dL_color, dL_alpha,
+                                                   densify_map, sched, nullptr);
+        };
+        if (want_refine && densify_map)
+            go(composite_backward_kernel<PX, true, true>);
+        else if (want_refine)
+            go(composite_backward_kernel<PX, true, false>);
+        else if (densify_map)
+            go(composite_backward_kernel<PX, false, true>);
+        else
+            go(composite_backward_kernel<PX, false, false>);
+    };
     if (pixels_per_thread == 1)
-        launch_backward_px<1>(s, tiles, ranges, order, st, K, bg, pix_T, pix_last, dL_color,
-                              dL_alpha, densify_map, want_refine, rs,
-                              tile_order);
+        bwd.template operator()<1>();
     else if (pixels_per_thread == 2)
-        launch_backward_px<2>(s, tiles, ranges, order, st, K, bg, pix_T, pix_last, dL_color,
-                              dL_alpha, densify_map, want_refine, rs,
-                              tile_order);
-    else if (pixels_per_thread == 8)
-        launch_backward_px<8>(s, tiles, ranges, order, st, K, bg, pix_T, pix_last, dL_color,
-                              dL_alpha, densify_map, want_refine, rs,
-                              tile_order);
+        bwd.template operator()<2>();
+    else if (pixels_per_thread == 4)
+        bwd.template operator()<4>();
     else
-        launch_backward_px<4>(s, tiles, ranges, order, st, K, bg, pix_T, pix_last, dL_color,
-                              dL_alpha, densify_map, want_refine, rs,
-                              tile_order);
+        bwd.template operator()<8>();
 }
 
 } // namespace gsb

@@ -202,14 +202,17 @@ struct RecStaging {
 // kDevStageTimeout in *err.
 void launch_stage_probe(cudaStream_t s, unsigned limit, unsigned* err);
 
+// Compositing forward over 16x16 tiles (strip.cuh). work_lists (may be NULL):
+// strip_order_words() words that receive the strips by adjoint work, the first
+// kWorkListZeroed of them zeroed before the call; launch_composite_backward
+// takes them with the same pixels_per_thread.
+constexpr int kWorkListZeroed = 64;
+size_t strip_order_words(int tiles, int pixels_per_thread);
 void launch_composite_forward(cudaStream_t s, int tiles, const uint2* ranges,
-                              const unsigned* order, const GaussianState& st, const Camera& K,
-                              float3 bg, float* color, float* alpha, float* pix_T,
-                              unsigned* pix_last, float* visibility, int pixels_per_thread,
-                              const RecStaging& rs, unsigned* tile_work = nullptr);
-// Tiles by descending adjoint work (tile_work from launch_composite_forward,
-// zeroed before it): a permutation of [0, tiles) into order.
-void launch_tile_order(cudaStream_t s, const unsigned* work, int tiles, unsigned* order);
+                              const unsigned* order, const Camera& K, float3 bg, float* color,
+                              float* alpha, float* pix_T, unsigned* pix_last, float* visibility,
+                              int pixels_per_thread, const RecStaging& rs,
+                              unsigned* work_lists = nullptr);
 // Fused L1 + SSIM loss: grad += dL/dpred, *loss_out (may be NULL) = L;
 // Training-loss terms of one view (image_loss.cu); field meanings as the
 // C ABI's gs_loss_images / gs_loss_options / gs_loss_outputs.
@@ -325,7 +328,7 @@ void launch_composite_backward(cudaStream_t s, int tiles, const uint2* ranges,
                                const float* dL_color, const float* dL_alpha,
                                const float* densify_map, int want_refine,
                                int pixels_per_thread, const RecStaging& rs,
-                               const unsigned* tile_order = nullptr);
+                               unsigned* work_lists = nullptr);
 
 cudaError_t launch_pruning_scores(cudaStream_t s, int tiles, const uint2* ranges,
                                   const unsigned* order, const GaussianState& st, const Camera& K,
