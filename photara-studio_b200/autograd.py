@@ -9,6 +9,7 @@ path stays on `Rasterizer.backward(..., structure_adam=, sh_adam=)`.
 """
 from __future__ import annotations
 
+from dataclasses import replace
 from typing import Optional
 
 import torch
@@ -26,7 +27,13 @@ class RasterizeGaussians(torch.autograd.Function):
                               sh_degree)
         rendered = Rasterizer().forward(model, camera, options)
         ctx.model = model
-        ctx.rendered = rendered
+        # Without the output tensors themselves: they point back at this node,
+        # and the cycle kept the native context and its workspace until a
+        # garbage collection, so every pass made new ones (300K Gaussians at
+        # 1237x823: 4.3 ms a pass, 0.9 ms with the context back at the end of
+        # the pass).
+        ctx.rendered = replace(rendered, color=rendered.color.detach(),
+                               alpha=rendered.alpha.detach())
         ctx.logit_shape = opacity_logits.shape
         ctx.mark_non_differentiable(rendered.radii)
         return rendered.color, rendered.alpha, rendered.radii

@@ -76,3 +76,38 @@ def test_autograd_matches_cpu_oracle_raw_gradients():
         a = p.grad.detach().cpu().double().numpy().ravel()
         b = np.asarray(ref, np.float64).ravel()
         assert np.linalg.norm(a - b) / np.linalg.norm(b) < 1e-3
+
+
+def test_autograd_passes_reuse_one_context(monkeypatch):
+    """A pass gives its native context back when its graph is freed, without a
+    garbage collection, on whichever stream the next pass runs."""
+    import gc
+    params, cam = _params()
+    params = [p.requires_grad_(True) for p in params]
+    made = []
+    create = gsb.rasterizer._Context.__init__
+    monkeypatch.setattr(gsb.rasterizer._Context, "__init__",
+                        lambda self, pool: (made.append(1), create(self, pool))[1])
+
+    def step():
+        color, alpha, _ = gsb.rasterize_gaussians(*params, cam)
+        return torch.autograd.grad(color.sum() + alpha.sum(), params)
+
+    first = step()
+    side = torch.cuda.Stream()
+    gc.disable()
+    try:
+        before = len(made)
+        for _ in range(3):
+            again = step()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            other = step()
+        torch.cuda.current_stream().wait_stream(side)
+        assert len(made) == before
+    finally:
+        gc.enable()
+    for a, b, c in zip(first, again, other):
+        scale = float(a.abs().max())  # float atomics: the last bits may differ
+        assert float((a - b).abs().max()) <= 1e-5 * scale
+        assert float((a - c).abs().max()) <= 1e-5 * scale
