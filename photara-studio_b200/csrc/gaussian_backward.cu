@@ -18,12 +18,15 @@
 // the structure Adam from registers. The SH adjoint leaves the row's basis
 // values and clamped colour gradient in shared memory (19 words instead of the
 // 48 coefficient gradients: each gradient is one product of the two).
-// Phase 2, the quantized SH Adam: degree-3 rows one thread per row (new
-// parameters straight to HBM as 16-byte row segments, log-second values in
-// the parameters' shared slots, first moments and codes in place and written
-// back coalesced); other strides one half-warp per row. 440 bytes of shared
-// memory per Gaussian and a 128-register bound give 4 CTAs (16 warps) per SM
-// (the thread-per-row layout with a gradient row took 544 bytes: 3 CTAs).
+// Phase 2, the quantized SH Adam: degree-3 rows one thread per row on f32x2
+// pairs (only the parameters staged; 284 bytes of shared memory per Gaussian
+// and 96 registers give 5 CTAs, 20 warps, per SM); other strides and degrees
+// one half-warp per row with everything staged (440 bytes: 4 CTAs).
+// Bound: the latency of its loads and of the codec's chains at 20 warps per
+// SM, half issue; it moves its algorithmic bytes. 1M / 1080p 306 -> 268 us,
+// 8.4M / 2160p 2,364 -> 2,006 us (4.4 TB/s) against the layout with every row
+// staged at 4 CTAs; 4 CTAs 275 us, 6 CTAs (80 registers, spills) 308 us, CTAs
+// of 64 and 32 rows 267 and 286 us (2,040 and 2,209 us at 8.4M).
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -371,17 +374,13 @@ __device__ __forceinline__ float code_to_float(unsigned code) {
 }
 
 // roundf(255 * (value - lo) * inv_range) clamped to [0, 255], as an integer:
-// adding 2^23 rounds a value in [0, 256) to the nearest integer (ties to
-// even) and leaves it in the low mantissa bits; a tie that went down is then
-// moved up, which is roundf's ties-away-from-zero for non-negative values.
-// Clamping before rounding gives the same integer (the bounds are integers).
+// floats in [2^22, 2^23) are multiples of a half, so y + (2^22 + 1/2) rounded
+// toward zero holds floor(2 y + 1) in its low mantissa bits, and half of that
+// is floor(y + 1/2), which is roundf for non-negative values. Clamping before
+// rounding gives the same integer (the bounds are integers).
 __device__ __forceinline__ unsigned codec_encode_int(float value, float lo, float inv_range) {
     const float y = fminf(fmaxf(255.f * (value - lo) * inv_range, 0.f), 255.f);
-    const float t = __fadd_rn(y, 8388608.f);
-    unsigned q = __float_as_uint(t) & 0xffu;
-    if (__fsub_rn(y, __fsub_rn(t, 8388608.f)) == 0.5f)
-        ++q;
-    return q;
+    return (__float_as_uint(__fadd_rz(y, 4194304.5f)) >> 1) & 0xffu;
 }
 
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
@@ -409,6 +408,36 @@ __device__ __forceinline__ void for_row_elements(int total, int stride, F&& f) {
             c -= stride;
             ++r;
         }
+    }
+}
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
+// Starts `bytes` (a multiple of 16) at p, 16-byte aligned, on their way to L2.
+__device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+// Staging of up to kRowsBlock degree-3 rows (16-byte aligned) for the
+// thread-per-row path: thread t copies the 16-byte segments e = t + kRowsBlock
+// k of the contiguous block; k -> k + 3 moves on by whole rows, so every copy
+// is at a fixed offset from three per-thread bases.
+constexpr int kRowsBlock = 128;
+constexpr int kRowStride = 52; // floats per staged row: 16-byte reads of eight rows hit every bank
+__device__ __forceinline__ void stage_rows48(float* s_coef, const float* src, int rows) {
+#pragma unroll
+    for (int k0 = 0; k0 < 3; ++k0) {
+        constexpr int kStep = kRowsBlock / 4; // rows per three k
+        const int e = int(threadIdx.x) + kRowsBlock * k0;
+        const int r = e / 12, c = e - 12 * r;
+        float* sd = s_coef + r * kRowStride + 4 * c;
+        const float* gs = src + 4 * e;
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+            if (r + kStep * g < rows)
+                cp_async16(sd + kStep * kRowStride * g, gs + 48 * kStep * g);
     }
 }
 
@@ -550,81 +579,32 @@ __device__ __forceinline__ void sh_adam_row_half(bool ok, size_t i, int stride, 
 }
 
 // Fused SH Adam, phase 2 for degree-3 rows (48 columns, all active), one
-// thread per row: the instruction path with the fewest instructions per
-// coefficient (launch constants folded once, groups of four independent
-// coefficient chains, no cross-lane reductions). The coefficient gradients
-// come from the row's basis values and clamped colour gradient (4 shared
-// loads per 12 columns); the new parameters go straight to HBM as 16-byte row
-// segments, and the log-second values take the parameters' shared-memory
-// slots for the encode pass; the new fp16 first moments and codes are written
-// in place and leave with one coalesced write-back per CTA.
-template <bool kFirstBlock>
-__device__ __forceinline__ void sh_adam_block48(int q, float* prow, __half* frow,
-                                                const uint8_t* crow, const float* wdl,
-                                                float3 dl, float* pout, float dlo, float drange,
-                                                float rlo, float rrange, float& dmin,
-                                                float& dmax, float& rmin, float& rmax,
-                                                const ShAdamConsts& k) {
-    const float w[4] = {wdl[4 * q], wdl[4 * q + 1], wdl[4 * q + 2], wdl[4 * q + 3]};
-    const float d[3] = {dl.x, dl.y, dl.z};
-#pragma unroll
-    for (int g = 0; g < 3; ++g) {
-        const int c0 = 12 * q + 4 * g;
-        float pv[4], gv[4], fv[4], cf[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            pv[j] = prow[c0 + j];
-            gv[j] = w[(4 * g + j) / 3] * d[(4 * g + j) % 3];
-        }
-        const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(frow + c0));
-        const float2 f23 = __half22float2(*reinterpret_cast<const __half2*>(frow + c0 + 2));
-        fv[0] = f01.x;
-        fv[1] = f01.y;
-        fv[2] = f23.x;
-        fv[3] = f23.y;
-        const unsigned cw = *reinterpret_cast<const unsigned*>(crow + c0);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            cf[j] = code_to_float((cw >> (8 * j)) & 0xffu);
-        float pn[4], fn[4], ln[4], chk = 0.f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const bool rest = !(kFirstBlock && g == 0 && j < 3);
-            ln[j] = sh_adam_coef_fast(rest, pv[j], gv[j], fv[j], cf[j], rest ? rlo : dlo,
-                                      rest ? rrange : drange, k, pn[j], fn[j], chk);
-        }
-        if (isfinite(chk)) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                pv[j] = pn[j];
-                fv[j] = fn[j];
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const bool rest = !(kFirstBlock && g == 0 && j < 3);
-                ln[j] = sh_adam_coef(rest, pv[j], gv[j], fv[j], cf[j], rest ? rlo : dlo,
-                                     rest ? rrange : drange, k);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (kFirstBlock && g == 0 && j < 3) {
-                dmin = fminf(dmin, ln[j]);
-                dmax = fmaxf(dmax, ln[j]);
-            } else {
-                rmin = fminf(rmin, ln[j]);
-                rmax = fmaxf(rmax, ln[j]);
-            }
-            prow[c0 + j] = ln[j];
-        }
-        *reinterpret_cast<float4*>(pout + c0) = make_float4(pv[0], pv[1], pv[2], pv[3]);
-        *reinterpret_cast<__half2*>(frow + c0) = __floats2half2_rn(fv[0], fv[1]);
-        *reinterpret_cast<__half2*>(frow + c0 + 2) = __floats2half2_rn(fv[2], fv[3]);
-    }
+// thread per row. Only the parameters pass through shared memory (the SH
+// adjoint reads them too): the row's fp16 first moments and codes are the
+// thread's own, read and written as 16- and 8-byte segments of its row, which
+// leaves 284 bytes of shared memory per Gaussian and five CTAs per SM (440
+// bytes and four CTAs with every row staged). Columns go in pairs on f32x2
+// instructions, element by element the arithmetic of sh_adam_coef, in two
+// halves of 24 columns; the coefficient gradients come from the row's basis
+// values and clamped colour gradient; the log-second values take the
+// parameters' shared slots for the encode pass.
+
+struct CheckedCoef {
+    float param, first, ls;
+};
+
+__device__ __noinline__ CheckedCoef sh_adam_coef_checked(bool rest, float param, float grad,
+                                                         float first, float code, float lo,
+                                                         float range, const ShAdamConsts& k) {
+    CheckedCoef o{param, first, 0.f};
+    o.ls = sh_adam_coef(rest, o.param, grad, o.first, code, lo, range, k);
+    return o;
 }
 
-__device__ __forceinline__ void sh_adam_row48(float* prow, __half* frow, uint8_t* crow,
+// Finiteness of a group is read off chk: a NaN or infinity in m or v reaches
+// the new parameter or the log value, whose sum it makes non-finite; the group
+// is then redone by sh_adam_coef.
+__device__ __forceinline__ void sh_adam_row48(float* prow, uint4* frow, uint2* crow,
                                               const float* wdl, float4 bnd, float* pout,
                                               float4* bout, const ShAdamConsts& k) {
     float b0 = bnd.x, b1 = bnd.y, b2 = bnd.z, b3 = bnd.w;
@@ -632,34 +612,153 @@ __device__ __forceinline__ void sh_adam_row48(float* prow, __half* frow, uint8_t
     if (!isfinite(b2) || !isfinite(b3)) b2 = b3 = 0.f;
     const float drange = b1 - b0, rrange = b3 - b2;
     float dmin = 1e30f, dmax = -1e30f, rmin = 1e30f, rmax = -1e30f;
-    const float3 dl = make_float3(wdl[16], wdl[17], wdl[18]);
-    sh_adam_block48<true>(0, prow, frow, crow, wdl, dl, pout, b0, drange, b2, rrange, dmin, dmax,
-                          rmin, rmax, k);
+    const float d[3] = {wdl[16], wdl[17], wdl[18]};
 #pragma unroll 1
-    for (int q = 1; q < 4; ++q)
-        sh_adam_block48<false>(q, prow, frow, crow, wdl, dl, pout, b0, drange, b2, rrange, dmin,
-                               dmax, rmin, rmax, k);
+    for (int h = 0; h < 2; ++h) { // columns 24 h ... 24 h + 23
+        uint4 fw[3];
+        uint2 cw[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            fw[j] = frow[3 * h + j];
+            cw[j] = crow[3 * h + j];
+        }
+        // the first three columns of the first half are the DC coefficient
+        const float lo0 = h ? b2 : b0, range0 = h ? rrange : drange;
+        const float lr0 = h ? k.rest_lr : k.lr, reg0 = h ? k.reg : 0.f;
+        unsigned* fws = reinterpret_cast<unsigned*>(fw);
+        const unsigned* cws = reinterpret_cast<const unsigned*>(cw);
+        float mn0 = 1e30f, mx0 = -1e30f;
+#pragma unroll
+        for (int g = 0; g < 6; ++g) { // four columns
+            const float4 p4 = *reinterpret_cast<const float4*>(prow + 24 * h + 4 * g);
+            const float pv[4] = {p4.x, p4.y, p4.z, p4.w};
+            float gv[4], cf[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int c = 4 * g + j;
+                gv[j] = wdl[8 * h + c / 3] * d[c % 3];
+                cf[j] = __uint_as_float(0x4b000000u | ((cws[g] >> (8 * j)) & 0xffu));
+            }
+            float pn[4], fn[4], ln[4];
+            float2 chk = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) { // a pair: columns j = 2 q, 2 q + 1
+                const bool dc0 = g == 0, dc1 = g == 0 && q == 0; // may be DC columns
+                const float2 lo = make_float2(dc0 ? lo0 : b2, dc1 ? lo0 : b2);
+                const float2 range = make_float2(dc0 ? range0 : rrange, dc1 ? range0 : rrange);
+                const float2 nlr = make_float2(dc0 ? -lr0 : -k.rest_lr, dc1 ? -lr0 : -k.rest_lr);
+                const float2 reg = make_float2(dc0 ? reg0 : k.reg, dc1 ? reg0 : k.reg);
+                const float2 prev = make_float2(pv[2 * q], pv[2 * q + 1]);
+                const float2 code = __fadd2_rn(make_float2(cf[2 * q], cf[2 * q + 1]),
+                                               make_float2(-8388608.f, -8388608.f));
+                const float2 log_s = __ffma2_rn(
+                    range, __fmul2_rn(code, make_float2(1.f / 255.f, 1.f / 255.f)), lo);
+                const float2 s = __fmul2_rn(
+                    make_float2(kCodecEps, kCodecEps),
+                    __fadd2_rn(make_float2(__expf(log_s.x), __expf(log_s.y)),
+                               make_float2(-1.f, -1.f)));
+                const float2 g2 = __fmul2_rn(s, s);
+                const float2 first =
+                    __half22float2(*reinterpret_cast<const __half2*>(&fws[2 * g + q]));
+                const float2 g1 = __fmul2_rn(
+                    __fmul2_rn(first, __ffma2_rn(make_float2(fabsf(s.x), fabsf(s.y)),
+                                                 make_float2(k.rs_pc2, k.rs_pc2),
+                                                 make_float2(k.eps, k.eps))),
+                    make_float2(k.pc1, k.pc1));
+                const float2 grad =
+                    __ffma2_rn(reg, prev, make_float2(gv[2 * q], gv[2 * q + 1]));
+                const float2 m = __ffma2_rn(make_float2(k.ob1, k.ob1), grad,
+                                            __fmul2_rn(make_float2(k.b1, k.b1), g1));
+                const float2 v = __ffma2_rn(__fmul2_rn(make_float2(k.ob2, k.ob2), grad), grad,
+                                            __fmul2_rn(make_float2(k.b2, k.b2), g2));
+                const float2 sv = make_float2(sqrtf(fmaxf(v.x, 0.f)), sqrtf(fmaxf(v.y, 0.f)));
+                const float2 num = __fmul2_rn(m, make_float2(k.ic1, k.ic1));
+                const float2 den = __ffma2_rn(sv, make_float2(k.rs_c2, k.rs_c2),
+                                              make_float2(k.eps, k.eps));
+                const float2 nrm =
+                    make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
+                const float2 np = __ffma2_rn(nlr, nrm, prev);
+                const float2 one_sv = __ffma2_rn(
+                    sv, make_float2(1.f / kCodecEps, 1.f / kCodecEps), make_float2(1.f, 1.f));
+                const float2 ls = make_float2(__logf(one_sv.x), __logf(one_sv.y));
+                chk = __fadd2_rn(chk, __fadd2_rn(np, ls));
+                pn[2 * q] = np.x;
+                pn[2 * q + 1] = np.y;
+                fn[2 * q] = nrm.x;
+                fn[2 * q + 1] = nrm.y;
+                ln[2 * q] = ls.x;
+                ln[2 * q + 1] = ls.y;
+            }
+            if (!k.norm_ok || !isfinite(chk.x + chk.y)) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const bool dc = g == 0 && j < 3 && h == 0;
+                    const __half2 fp = *reinterpret_cast<const __half2*>(&fws[2 * g + j / 2]);
+                    const CheckedCoef o = sh_adam_coef_checked(
+                        !dc, pv[j], gv[j], j & 1 ? __high2float(fp) : __low2float(fp),
+                        cf[j] - 8388608.f, dc ? b0 : b2, dc ? drange : rrange, k);
+                    pn[j] = o.param;
+                    fn[j] = o.first;
+                    ln[j] = o.ls;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (g == 0 && j < 3) {
+                    mn0 = fminf(mn0, ln[j]);
+                    mx0 = fmaxf(mx0, ln[j]);
+                } else {
+                    rmin = fminf(rmin, ln[j]);
+                    rmax = fmaxf(rmax, ln[j]);
+                }
+            }
+            *reinterpret_cast<float4*>(pout + 24 * h + 4 * g) =
+                make_float4(pn[0], pn[1], pn[2], pn[3]);
+            *reinterpret_cast<float4*>(prow + 24 * h + 4 * g) =
+                make_float4(ln[0], ln[1], ln[2], ln[3]);
+            const __half2 f01 = __floats2half2_rn(fn[0], fn[1]);
+            const __half2 f23 = __floats2half2_rn(fn[2], fn[3]);
+            fws[2 * g] = *reinterpret_cast<const unsigned*>(&f01);
+            fws[2 * g + 1] = *reinterpret_cast<const unsigned*>(&f23);
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            frow[3 * h + j] = fw[j];
+        if (h == 0) {
+            dmin = mn0;
+            dmax = mx0;
+        } else {
+            rmin = fminf(rmin, mn0);
+            rmax = fmaxf(rmax, mx0);
+        }
+    }
     *bout = make_float4(dmin, dmax, rmin, rmax);
     const float inv_d = 1.f / fmaxf(dmax - dmin, kCodecEps);
     const float inv_r = 1.f / fmaxf(rmax - rmin, kCodecEps);
-#pragma unroll 2
-    for (int c0 = 0; c0 < 48; c0 += 4) {
-        float lv[4];
+#pragma unroll 1
+    for (int h = 0; h < 6; ++h) { // eight columns
+        unsigned w[2];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            lv[j] = prow[c0 + j];
-        unsigned w = 0;
+        for (int g = 0; g < 2; ++g) {
+            const float4 l4 = *reinterpret_cast<const float4*>(prow + 8 * h + 4 * g);
+            const float lv[4] = {l4.x, l4.y, l4.z, l4.w};
+            w[g] = 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const bool dc = c0 + j < 3;
-            w |= codec_encode_int(lv[j], dc ? dmin : rmin, dc ? inv_d : inv_r) << (8 * j);
+            for (int j = 0; j < 4; ++j) {
+                const bool dc = g == 0 && j < 3 && h == 0;
+                w[g] |= codec_encode_int(lv[j], dc ? dmin : rmin, dc ? inv_d : inv_r) << (8 * j);
+            }
         }
-        *reinterpret_cast<unsigned*>(crow + c0) = w;
+        crow[h] = make_uint2(w[0], w[1]);
     }
 }
 
-template <bool kFusedStruct, bool kFusedSH, bool kGeo>
-__global__ void __launch_bounds__(kGBlock, 4) gaussian_backward_kernel(
+// kRows48: the fused SH Adam on degree-3 rows with all columns active and
+// 16-byte aligned state (sh_adam_row48); the other layouts and degrees take
+// the half-warp rows.
+template <bool kFusedStruct, bool kFusedSH, bool kGeo, bool kRows48>
+__global__ void __launch_bounds__(kRows48 ? kRowsBlock : kGBlock,
+                                  kRows48 && !kGeo ? 5 : 4) gaussian_backward_kernel(
     int n, const float* __restrict__ means, const float* __restrict__ log_scales,
     const float* __restrict__ quats, const float* __restrict__ logits,
     const float* __restrict__ filter_3d, const float* __restrict__ sh, int sh_degree,
@@ -671,19 +770,33 @@ __global__ void __launch_bounds__(kGBlock, 4) gaussian_backward_kernel(
     // first moments [kGBlock][kHalfStride], u8 codes [kGBlock][kCodeStride]
     // and code bounds [kGBlock] float4; without it the coefficient gradients
     // [kGBlock][kShStride].
+    // kRows48: SH rows [kGBlock][kRowStride] and basis rows [kGBlock][kWdlStride].
+    constexpr int kCoefStride = kRows48 ? kRowStride : kShStride;
     float* s_coef = smem;
-    float* s_aux = smem + kGBlock * kShStride;
+    constexpr int kRows = kRows48 ? kRowsBlock : kGBlock;
+    float* s_aux = smem + kRows * kCoefStride;
     __half* s_first = reinterpret_cast<__half*>(s_aux + kGBlock * kWdlStride);
     uint8_t* s_code = reinterpret_cast<uint8_t*>(s_first + kGBlock * kHalfStride);
     float4* s_bnd = reinterpret_cast<float4*>(s_code + kGBlock * kCodeStride);
     const int tid = threadIdx.x;
-    const int row0 = blockIdx.x * kGBlock;
-    const int rows = min(kGBlock, n - row0);
+    const int row0 = blockIdx.x * kRows;
+    const int rows = min(kRows, n - row0);
     const int stride = sh ? sh_bases * 3 : 0;
     // 1. Asynchronous, coalesced staging of this CTA's SH rows (contiguous),
     //    and with fused SH Adam of their fp16 first moments, u8 codes and code
     //    bounds.
-    if (stride == 48 && rows == kGBlock) {
+    if constexpr (kRows48) {
+        stage_rows48(s_coef, sh + size_t(row0) * 48, rows);
+        // the rows that the Adam reads later start their way from HBM
+        if (tid == 0) {
+            prefetch_l2(reinterpret_cast<const __half*>(sha.first) + size_t(row0) * 48,
+                        unsigned(rows) * 96u);
+            prefetch_l2(sha.packed + size_t(row0) * 48, unsigned(rows) * 48u);
+        }
+    } else if (stride == 48 && rows == kGBlock &&
+               (!kFusedSH || ((reinterpret_cast<uintptr_t>(sha.first) |
+                               reinterpret_cast<uintptr_t>(sha.packed)) & 3) == 0)) {
+        // (moments and codes that are not 4-byte aligned go element by element)
         stage_full48(s_coef, s_first, s_code, sh + size_t(row0) * 48,
                      kFusedSH ? reinterpret_cast<const uint32_t*>(
                                     reinterpret_cast<const __half*>(sha.first) + size_t(row0) * 48)
@@ -706,7 +819,7 @@ __global__ void __launch_bounds__(kGBlock, 4) gaussian_backward_kernel(
             });
         }
     }
-    if constexpr (kFusedSH)
+    if constexpr (kFusedSH && !kRows48)
         if (sh && tid < rows)
             s_bnd[tid] = reinterpret_cast<const float4*>(sha.bounds)[row0 + tid];
     // 2. Meanwhile every per-Gaussian input of this thread is loaded up front.
@@ -796,10 +909,22 @@ __global__ void __launch_bounds__(kGBlock, 4) gaussian_backward_kernel(
         }
         const float3 dcol = make_float3(g2.x, g2.y, g2.z);
         if (sh) {
-            const float3* crow = reinterpret_cast<const float3*>(s_coef + tid * kShStride);
             const float3 campos = make_float3(K.center[0], K.center[1], K.center[2]);
             float3 dm;
-            if constexpr (kFusedSH)
+            const float3* crow = reinterpret_cast<const float3*>(s_coef + tid * kCoefStride);
+            if constexpr (kRows48) {
+                float4 q[12];
+#pragma unroll
+                for (int k = 0; k < 12; ++k)
+                    q[k] = reinterpret_cast<const float4*>(crow)[k];
+                const float* f = reinterpret_cast<const float*>(q);
+                float3 c[16];
+#pragma unroll
+                for (int k = 0; k < 16; ++k)
+                    c[k] = make_float3(f[3 * k], f[3 * k + 1], f[3 * k + 2]);
+                dm = sh_color_backward<true>(c, 3, 16, mean, campos, clamp_bits, dcol, nullptr,
+                                             wdl);
+            } else if constexpr (kFusedSH)
                 dm = sh_color_backward<true>(crow, sh_degree, sh_bases, mean, campos, clamp_bits,
                                              dcol, nullptr, wdl);
             else
@@ -925,35 +1050,21 @@ __global__ void __launch_bounds__(kGBlock, 4) gaussian_backward_kernel(
 
     // 5. SH: the fused quantized Adam (phase 2, one half-warp per row) or the
     //    coalesced accumulation of the coefficient gradients.
-    if constexpr (kFusedSH) {
+    if constexpr (kRows48) {
+        if (valid)
+            sh_adam_row48(s_coef + tid * kRowStride,
+                          reinterpret_cast<uint4*>(reinterpret_cast<__half*>(sha.first) +
+                                                   size_t(i) * 48),
+                          reinterpret_cast<uint2*>(sha.packed + size_t(i) * 48), wdl,
+                          reinterpret_cast<const float4*>(sha.bounds)[i],
+                          sha.parameter + size_t(i) * 48,
+                          reinterpret_cast<float4*>(sha.bounds) + i, sh_adam_consts(sha));
+    } else if constexpr (kFusedSH) {
         if (!sh)
             return;
         __syncthreads();
         const int active = (sh_degree + 1) * (sh_degree + 1) * 3;
         const ShAdamConsts kc = sh_adam_consts(sha);
-        const bool aligned = ((reinterpret_cast<uintptr_t>(sha.parameter) & 15) |
-                              (reinterpret_cast<uintptr_t>(sha.first) & 7) |
-                              (reinterpret_cast<uintptr_t>(sha.packed) & 3)) == 0;
-        if (stride == 48 && active == 48 && aligned) {
-            // one thread per row, then the coalesced write-back of the new
-            // fp16 first moments and codes (four columns per thread and step)
-            if (valid)
-                sh_adam_row48(s_coef + tid * kShStride, s_first + tid * kHalfStride,
-                              s_code + tid * kCodeStride, s_aux + tid * kWdlStride, s_bnd[tid],
-                              sha.parameter + size_t(i) * 48,
-                              reinterpret_cast<float4*>(sha.bounds) + i, kc);
-            __syncthreads();
-            uint2* fdst = reinterpret_cast<uint2*>(reinterpret_cast<__half*>(sha.first) +
-                                                   size_t(row0) * 48);
-            unsigned* cdst = reinterpret_cast<unsigned*>(sha.packed + size_t(row0) * 48);
-            for_row_elements(rows * 12, 12, [&](int e, int r, int cq) {
-                const unsigned* f =
-                    reinterpret_cast<const unsigned*>(s_first + r * kHalfStride + 4 * cq);
-                fdst[e] = make_uint2(f[0], f[1]);
-                cdst[e] = *reinterpret_cast<const unsigned*>(s_code + r * kCodeStride + 4 * cq);
-            });
-            return;
-        }
         // other strides and degrees: one half-warp per row
         const int l = tid & 15, hw = tid >> 4;
         constexpr int kHalves = kGBlock / 16;       // half-warps per CTA
@@ -984,7 +1095,9 @@ __global__ void __launch_bounds__(kGBlock, 4) gaussian_backward_kernel(
     }
 }
 
-size_t gaussian_backward_smem(bool fused_sh) {
+size_t gaussian_backward_smem(bool fused_sh, bool rows48) {
+    if (rows48)
+        return size_t(kRowsBlock) * (kRowStride + kWdlStride) * sizeof(float);
     if (!fused_sh)
         return size_t(kGBlock) * 2 * kShStride * sizeof(float);
     return size_t(kGBlock) * ((kShStride + kWdlStride) * sizeof(float) +
@@ -996,33 +1109,42 @@ void launch_gaussian_backward(cudaStream_t s, int n, const float* means, const f
                               const float* sh, int sh_degree, int sh_bases, const Camera& K,
                               const GaussianState& st, const int* radii, const GradOutArgs& out,
                               const StructureAdamArgs* sa, const ShAdamArgs* sha, bool geometry) {
-    const int blocks = (n + kGBlock - 1) / kGBlock;
     StructureAdamArgs sa0{};
     ShAdamArgs sha0{};
     const bool fs = sa != nullptr, fh = sha != nullptr && sh != nullptr;
-    const size_t smem = gaussian_backward_smem(fh);
-#define GSB_LAUNCH(FS, FH, GEO)                                                                  \
+    const bool rows48 = fh && sh_bases == 16 && sh_degree == 3 &&
+                        ((reinterpret_cast<uintptr_t>(sh) | reinterpret_cast<uintptr_t>(sha->parameter) |
+                          reinterpret_cast<uintptr_t>(sha->first) |
+                          reinterpret_cast<uintptr_t>(sha->packed)) & 15) == 0;
+    const size_t smem = gaussian_backward_smem(fh, rows48);
+    const int threads = rows48 ? kRowsBlock : kGBlock;
+    const int blocks = (n + threads - 1) / threads;
+#define GSB_LAUNCH(FS, FH, GEO, R48)                                                             \
     do {                                                                                         \
-        auto kfn = gaussian_backward_kernel<FS, FH, GEO>;                                        \
+        auto kfn = gaussian_backward_kernel<FS, FH, GEO, R48>;                                        \
         static bool attr_set = false;                                                            \
         if (!attr_set) {                                                                         \
             cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));   \
             attr_set = true;                                                                     \
         }                                                                                        \
-        kfn<<<blocks, kGBlock, smem, s>>>(n, means, log_scales, quats, logits, filter_3d, sh,    \
+        kfn<<<blocks, threads, smem, s>>>(n, means, log_scales, quats, logits, filter_3d, sh,    \
                                           sh_degree, sh_bases, K, st, radii, out,                \
                                           sa ? *sa : sa0, sha ? *sha : sha0);                    \
     } while (0)
     if (geometry) {
-        if (fs && fh) GSB_LAUNCH(true, true, true);
-        else if (fs) GSB_LAUNCH(true, false, true);
-        else if (fh) GSB_LAUNCH(false, true, true);
-        else GSB_LAUNCH(false, false, true);
+        if (fs && rows48) GSB_LAUNCH(true, true, true, true);
+        else if (rows48) GSB_LAUNCH(false, true, true, true);
+        else if (fs && fh) GSB_LAUNCH(true, true, true, false);
+        else if (fs) GSB_LAUNCH(true, false, true, false);
+        else if (fh) GSB_LAUNCH(false, true, true, false);
+        else GSB_LAUNCH(false, false, true, false);
     } else {
-        if (fs && fh) GSB_LAUNCH(true, true, false);
-        else if (fs) GSB_LAUNCH(true, false, false);
-        else if (fh) GSB_LAUNCH(false, true, false);
-        else GSB_LAUNCH(false, false, false);
+        if (fs && rows48) GSB_LAUNCH(true, true, false, true);
+        else if (rows48) GSB_LAUNCH(false, true, false, true);
+        else if (fs && fh) GSB_LAUNCH(true, true, false, false);
+        else if (fs) GSB_LAUNCH(true, false, false, false);
+        else if (fh) GSB_LAUNCH(false, true, false, false);
+        else GSB_LAUNCH(false, false, false, false);
     }
 #undef GSB_LAUNCH
 }
