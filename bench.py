@@ -493,8 +493,8 @@ def main():
                                       world), world)
     clk = clocks.stop()
     counts = {"instances": step.last.rendered_instances, "visible": step.last.visible_count,
-              "depth_passes": (step.last.depth_bits + 7) // 8,
-              "tile_passes": (step.last.tile_bits + 7) // 8}
+              "depth_passes": -(-step.last.depth_bits // 9),
+              "tile_passes": -(-step.last.tile_bits // 9)}
     peaks = {}
     pk = ROOT / "MEASURED_PEAKS.json"
     peak_src = "fallback"
@@ -531,7 +531,7 @@ def main():
                 "per_stage": roof},
             "e2e": {"value": round(e2e_ms, 4), "unit": "ms/iter",
                     "h2d_bytes_per_step": int(target.numel() * 4), "d2h_bytes_per_step": 4},
-            "gpu_launches": args.steps * (12 + counts["depth_passes"] + counts["tile_passes"]),
+            "gpu_launches": args.steps * (10 + counts["depth_passes"] + counts["tile_passes"]),
             "clocks": clk,
             "cpu_baseline": cpu,
         }

@@ -808,7 +808,7 @@ void plan(gs_batch* b, const gs_gaussians* g, const gs_camera* cams, int views,
         b->cvals[k] = reinterpret_cast<unsigned*>(cst + align_up(tiles * 4) * (2 + k));
     }
     b->counters = reinterpret_cast<unsigned*>(b->counters_buf.exact(kBcWords * 4, st, true));
-    b->hist_buf.exact(8 * 256 * sizeof(unsigned), st);
+    b->hist_buf.exact(8 * kMaxRadix * sizeof(unsigned), st);
     b->tile_ctr_buf.exact(64 * sizeof(unsigned), st);
     b->scan_status_buf.exact(std::max<size_t>(scan_status_bytes(int(pairs)), 256), st);
     // the schedule's kernels: grid sizes and attributes
@@ -858,9 +858,9 @@ void plan(gs_batch* b, const gs_gaussians* g, const gs_camera* cams, int views,
         b->ikeys[k] = reinterpret_cast<unsigned*>(ik + align_up(cap * 4) * k);
         b->ivals[k] = reinterpret_cast<unsigned*>(ik + align_up(cap * 4) * (2 + k));
     }
-    const size_t status = std::max({sort_status_bytes(pairs, 4),
-                                    sort_status_bytes(cap, radix_passes(b->tile_bits)),
-                                    sort_status_bytes(tiles, radix_passes(b->cost_bits)),
+    const size_t status = std::max({sort_status_bytes(pairs, radix_plan(32)),
+                                    sort_status_bytes(cap, radix_plan(b->tile_bits)),
+                                    sort_status_bytes(tiles, radix_plan(b->cost_bits)),
                                     size_t(256)});
     b->status_buf.exact(status, st);
     b->cost_result = 0;

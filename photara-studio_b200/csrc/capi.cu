@@ -315,7 +315,7 @@ gs_status gs_create(gs_context** out, int device, void* stream) {
         ck(cudaMallocHost(&c->host_counts, 16 * sizeof(unsigned)), "pinned counters");
         std::memset(c->host_counts, 0, 16 * sizeof(unsigned));
         c->counters.ensure(64, c->stream, true);
-        c->sort_hist.ensure(8 * 256 * sizeof(unsigned), c->stream);
+        c->sort_hist.ensure(8 * kMaxRadix * sizeof(unsigned), c->stream);
         c->sort_counters.ensure(64, c->stream);
         for (auto& set : c->ev)
             for (auto& e : set)
@@ -445,11 +445,11 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
             frame += align_up(std::max<size_t>(bytes, 1));
             return at;
         };
-        const size_t o_hist_d = (carve(size_t(tiles) * sizeof(uint2)), carve(4 * 256 * 4));
-        const size_t o_hist_t = carve(4 * 256 * 4);
+        const size_t o_hist_d = (carve(size_t(tiles) * sizeof(uint2)), carve(4 * kMaxRadix * 4));
+        const size_t o_hist_t = carve(4 * kMaxRadix * 4);
         const size_t o_compact = carve(scan_status_bytes(n));
         const size_t o_scan = carve(scan_status_bytes(n));
-        const size_t o_dsort = carve(sort_status_bytes(size_t(n), 4));
+        const size_t o_dsort = carve(sort_status_bytes_max(size_t(n), 32));
         const size_t o_ctr = carve(16 * sizeof(unsigned));
         const int ppt = compositing_px(c, tiles);
         // the strips by adjoint work, listed by the compositing; only the
@@ -483,8 +483,7 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
         const int depth_bits = msb_bits(visible ? dmax - dmin + 1u : 1u);
         ensure_instances(c, std::max<size_t>(instances, 1), 2);
         // The tile sort's status and counters, sized by the instance count.
-        const int tpasses = radix_passes(tile_bits);
-        const size_t tstat = align_up(sort_status_bytes(instances, tpasses));
+        const size_t tstat = align_up(sort_status_bytes(instances, radix_plan(tile_bits)));
         char* ts = c->sort_status.ensure(tstat + 256, st);
         ck(cudaMemsetAsync(ts, 0, tstat + 256, st), "tile sort reset");
         int cur = 0;
@@ -854,7 +853,7 @@ gs_status gs_sort_pairs_u64(gs_context* c, const unsigned long long* keys_in,
             return;
         cudaStream_t st = c->stream;
         ensure_instances(c, count, 8);
-        c->sort_status.ensure(std::max<size_t>(sort_status_bytes(c->inst_cap, 8), 256), st);
+        c->sort_status.ensure(std::max<size_t>(sort_status_bytes(c->inst_cap, sort_plan<unsigned long long>(64)), 256), st);
         c->have_forward = false; // the instance buffers are reused here
         ck(cudaMemcpyAsync(c->keys[0], keys_in, count * 8, cudaMemcpyDeviceToDevice, st), "sort in");
         ck(cudaMemcpyAsync(c->vals[0], vals_in, count * 4, cudaMemcpyDeviceToDevice, st), "sort in");

@@ -180,8 +180,33 @@ void launch_scan(cudaStream_t s, int n, const unsigned* in, const unsigned* inde
                  unsigned long long* status, unsigned* tile_counter, unsigned* total,
                  unsigned* err, bool zeroed = false, unsigned* groups = nullptr,
                  int group_shift = 0, unsigned group_cap = 0);
-int radix_passes(int bits);
-size_t sort_status_bytes(size_t count, int passes);
+// The digits of a radix sort of `bits` key bits: the fewest passes of at most
+// `most` bits each, the bits spread evenly (the first passes take the odd
+// ones), so a 25-bit depth sort takes 9 + 8 + 8 bits and 13 tile bits 7 + 6.
+// Digit histograms are [passes][kMaxRadix] words.
+constexpr int kMaxDigitBits = 9;
+constexpr int kMaxRadix = 1 << kMaxDigitBits;
+struct RadixPlan {
+    int bits = 0, passes = 0;
+    __host__ __device__ int width(int p) const {
+        return bits / passes + (p < bits % passes ? 1 : 0);
+    }
+    __host__ __device__ int shift(int p) const {
+        const int odd = bits % passes;
+        return p * (bits / passes) + (p < odd ? p : odd);
+    }
+};
+__host__ __device__ inline RadixPlan radix_plan(int bits, int most = kMaxDigitBits) {
+    return RadixPlan{bits, (bits + most - 1) / most};
+}
+// 64-bit keys keep 8-bit digits: their staged tile fills the shared memory.
+template <typename Key> RadixPlan sort_plan(int bits) {
+    return radix_plan(bits, sizeof(Key) == 8 ? 8 : kMaxDigitBits);
+}
+// Look-back status bytes of a sort of `count` keys; _max: of any 32-bit-key
+// plan of at most `bits` bits.
+size_t sort_status_bytes(size_t count, const RadixPlan& plan);
+size_t sort_status_bytes_max(size_t count, int bits);
 template <typename Key>
 int launch_radix_sort(cudaStream_t s, Key* keys[2], unsigned* vals[2], size_t count,
                       const unsigned* count_dev, int begin_bit, int end_bit, unsigned* hist,

@@ -69,27 +69,54 @@ __global__ void __launch_bounds__(kBlock) preprocess_kernel(
 }
 
 // The radix sort's digit histograms of the keys a kernel writes, counted as
-// they are written (8-bit digits over key bits [0, bits), up to 4 passes):
-// the sort then skips its own read of the keys. Per-block shared histograms,
-// flushed with one global atomic per non-empty bin.
+// they are written (the digits of radix_plan over key bits [0, bits), up to 4
+// passes): the sort then skips its own read of the keys. Per-block shared
+// histograms, flushed with one global atomic per non-empty bin. A digit of w
+// bits has 2^(9 - w) counters per bin in neighbouring banks, taken by lane:
+// neighbouring instances mostly share their high tile digit, and 32 lanes on
+// one counter are served one by one (emit at 1M / 1080p 68 us on single
+// counters of 7 + 6 bits).
 struct DigitCounter {
-    unsigned (*h)[256];
+    unsigned (*h)[kMaxRadix];
+    RadixPlan plan;
+    int w0, c0, w1, c1; // widths and counter bits of the first two digits
+    unsigned l0, l1;    // the lane's counter among a bin's
+    __device__ __forceinline__ DigitCounter(unsigned (*hist)[kMaxRadix], int bits)
+        : h(hist), plan(radix_plan(bits)) {
+        w0 = plan.width(0);
+        c0 = kMaxDigitBits - w0;
+        l0 = lane_id() & ((1u << c0) - 1u);
+        w1 = plan.passes > 1 ? plan.width(1) : 0;
+        c1 = kMaxDigitBits - w1;
+        l1 = lane_id() & ((1u << c1) - 1u);
+    }
     __device__ __forceinline__ void zero() {
-        for (int k = threadIdx.x; k < 4 * 256; k += blockDim.x)
+        for (int k = threadIdx.x; k < plan.passes * kMaxRadix; k += blockDim.x)
             (&h[0][0])[k] = 0;
     }
-    __device__ __forceinline__ void count(unsigned key, int bits) {
-        for (int p = 0, shift = 0; shift < bits; ++p, shift += 8) {
-            const int b = min(8, bits - shift);
-            atomicAdd(&h[p][(key >> shift) & ((1u << b) - 1u)], 1u);
+    __device__ __forceinline__ void count(unsigned key) {
+        atomicAdd(&h[0][((key << c0) & (kMaxRadix - 1)) | l0], 1u);
+        if (plan.passes > 1) {
+            key >>= w0;
+            atomicAdd(&h[1][((key << c1) & (kMaxRadix - 1)) | l1], 1u);
+            for (int p = 2, at = w1; p < plan.passes; at += plan.width(p), ++p) {
+                const int c = kMaxDigitBits - plan.width(p);
+                atomicAdd(&h[p][(((key >> at) << c) & (kMaxRadix - 1)) |
+                                (lane_id() & ((1u << c) - 1u))],
+                          1u);
+            }
         }
     }
-    __device__ __forceinline__ void flush(unsigned* __restrict__ hist, int bits) {
-        const int passes = (bits + 7) / 8;
-        for (int k = threadIdx.x; k < passes * 256; k += blockDim.x) {
-            const unsigned v = (&h[0][0])[k];
-            if (v)
-                atomicAdd(&hist[k], v);
+    __device__ __forceinline__ void flush(unsigned* __restrict__ hist) {
+        for (int p = 0; p < plan.passes; ++p) {
+            const int w = plan.width(p), c = kMaxDigitBits - w;
+            for (int d = threadIdx.x; d < 1 << w; d += blockDim.x) {
+                unsigned v = 0;
+                for (int k = 0; k < 1 << c; ++k)
+                    v += h[p][(d << c) | k];
+                if (v)
+                    atomicAdd(&hist[p * kMaxRadix + d], v);
+            }
         }
     }
 };
@@ -115,10 +142,10 @@ __global__ void __launch_bounds__(kBlock) depth_compact_kernel(
     // host is still reading the draw counts back.
     const unsigned dmin = counters[4];
     const int bits = 32 - __clz(int(counters[5] - dmin + 1u));
-    __shared__ unsigned s_hist[4][256];
+    __shared__ unsigned s_hist[4][kMaxRadix];
     __shared__ unsigned s_warp[8];
     __shared__ unsigned s_tile, s_prefix;
-    DigitCounter dc{s_hist};
+    DigitCounter dc(s_hist, bits);
     dc.zero();
     if (threadIdx.x == 0)
         s_tile = atomicAdd(tile_counter, 1u);
@@ -150,12 +177,12 @@ __global__ void __launch_bounds__(kBlock) depth_compact_kernel(
             const unsigned key = st.depth[base + k] - dmin;
             keys[out] = key;
             values[out] = unsigned(base + k);
-            dc.count(key, bits);
+            dc.count(key);
             ++out;
         }
     }
     __syncthreads();
-    dc.flush(hist, bits);
+    dc.flush(hist);
 }
 
 // Duplicate-with-keys. Warps take the visible Gaussians in depth order in
@@ -174,8 +201,8 @@ __global__ void __launch_bounds__(kEmitBlock) emit_keys_kernel(
     unsigned* __restrict__ hist) {
     // column: (first instance in the 32 Gaussians' range, first tile, tile step, Gaussian)
     __shared__ uint4 s_col[kEmitBlock / 32][32 * kSpanCols];
-    __shared__ unsigned s_hist[4][256];
-    DigitCounter dc{s_hist};
+    __shared__ unsigned s_hist[3][kMaxRadix]; // tile ids stay below 2^27
+    DigitCounter dc(s_hist, bits);
     dc.zero();
     __syncthreads();
     const int warp = int(threadIdx.x >> 5);
@@ -185,9 +212,9 @@ __global__ void __launch_bounds__(kEmitBlock) emit_keys_kernel(
     emit_warp_range<kTileW, kTileH>(
         r_begin, r_end, order, st, [&](unsigned i) { return __ldg(&st.rec[i].spans); },
         [&](unsigned) { return EmitView{grid_x, grid_y, 0u}; }, keys, values, capacity,
-        s_col[warp], [&](unsigned key) { dc.count(key, bits); });
+        s_col[warp], [&](unsigned key) { dc.count(key); });
     __syncthreads();
-    dc.flush(hist, bits);
+    dc.flush(hist);
 }
 
 // Per-tile [start, end) from the sorted keys. ranges[] is zeroed beforehand.
