@@ -16,11 +16,12 @@
 //   4 duplicate-with-keys in depth order with global tile ids as keys;
 //   5 onesweep sort of the instances on the tile-id bits (stable), instance
 //     count read on the device (capacity-sized grids);
-//   6 tile ranges; optional tile ordering by cost (heaviest first);
-//   7 persistent compositing kernel: each CTA pulls tiles of any view
-//     (static stride, a dynamic queue, or the cost order) and runs the shared
-//     per-tile body of composite.cuh for the planned tile shape;
-//   8 persistent compositing adjoint, same schedule;
+//   6 tile ranges; optional tile ordering by instance count (heaviest first);
+//   7 persistent compositing kernel: one-warp CTAs pull strips of tiles of any
+//     view (static stride, a dynamic queue, or the tile order) and run the
+//     shared strip body of strip.cuh for the planned tile shape;
+//   8 persistent compositing adjoint, same schedule (heaviest first: by the
+//     work each strip's forward recorded);
 //   9 per-Gaussian adjoint looping over the views in registers (one write of
 //     each summed gradient, no atomics).
 // The tile shape (8x8, 16x16, 16x32), pixels per thread and schedule are plan
@@ -36,11 +37,11 @@
 
 #include "../../include/gsplat_b200.h"
 #include "adjoint.cuh"
-#include "composite.cuh"
 #include "emit.cuh"
 #include "host.h"
 #include "kernels.h"
 #include "preprocess.cuh"
+#include "strip.cuh"
 
 using namespace gsb;
 using namespace gsb::host;
@@ -62,7 +63,7 @@ enum BatchCounter : int {
     kBcPairs = 5,     // V * N (count for the depth sort)
     kBcTotal = 6,     // scan total
     kBcSorted = 7,    // min(instances, capacity): count for the tile sort
-    kBcTiles = 8,     // total tiles (count for the cost sort)
+    kBcTiles = 8,     // total tiles
     kBcInstances64 = 10, // words 10-11: instances requested by the preprocess (u64)
     kBcWords = 16
 };
@@ -143,65 +144,42 @@ __global__ void __launch_bounds__(kBatchEmitBlock) batch_emit_kernel(
     int n, const unsigned* __restrict__ counters, const unsigned* __restrict__ groups,
     int group_shift, unsigned group_cap, const unsigned* __restrict__ order, GaussianState st,
     const BatchView* __restrict__ views, unsigned* __restrict__ keys, unsigned* __restrict__ vals,
-    unsigned capacity) {
+    unsigned capacity, int bits, unsigned* __restrict__ hist) {
     __shared__ uint4 s_col[kBatchEmitBlock / 32][32 * kSpanCols];
+    __shared__ unsigned s_hist[3][kMaxRadix]; // tile ids stay below 2^27
+    DigitCounter dc(s_hist, bits);
+    dc.zero();
+    __syncthreads();
     const int warp = int(threadIdx.x >> 5);
     const unsigned total = counters[kBcTotal];
     const int visible = int(counters[kBcVisible]);
     const unsigned group_count =
         min(unsigned((size_t(total) + (size_t(1) << group_shift) - 1) >> group_shift), group_cap);
     const unsigned g = blockIdx.x * (kBatchEmitBlock / 32) + unsigned(warp);
-    if (g >= group_count)
-        return; // warp-uniform; the kernel has no block-wide barrier
-    const int r_begin = int(groups[g]);
+    const int r_begin = g < group_count ? int(groups[g]) : visible;
     const int r_end = g + 1 < group_count ? int(groups[g + 1]) : visible;
     emit_warp_range<TW, TH>(
-        r_begin, r_end, order, st, [&](unsigned p) { return __ldg(&st.spans[p]); },
+        r_begin, r_end, order, st,
         [&](unsigned p) {
             const BatchView& v = views[p / unsigned(n)];
             return EmitView{v.K.grid_x, v.K.grid_y, v.tile_base};
         },
-        keys, vals, capacity, s_col[warp], [](unsigned) {});
+        keys, vals, capacity, s_col[warp], [&](unsigned key) { dc.count(key); });
+    __syncthreads();
+    dc.flush(hist);
 }
 
 // ------------------------------------------------------------- stage 6 --
-__global__ void __launch_bounds__(kBlock) batch_ranges_kernel(const unsigned* __restrict__ counters,
-                                                              const unsigned* __restrict__ keys,
-                                                              uint2* __restrict__ ranges,
-                                                              unsigned tiles) {
-    const unsigned count = counters[kBcSorted];
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count)
-        return;
-    const unsigned tile = keys[i];
-    if (i == 0) {
-        if (tile < tiles)
-            ranges[tile].x = 0;
-    } else {
-        const unsigned prev = keys[i - 1];
-        if (tile != prev) {
-            if (prev < tiles)
-                ranges[prev].y = i;
-            if (tile < tiles)
-                ranges[tile].x = i;
-        }
-    }
-    if (i == count - 1 && tile < tiles)
-        ranges[tile].y = count;
-}
-
-// Heaviest-first order: 16-bit inverted instance counts, sorted stably.
+// Heaviest-first order of the forward: the tiles by instance count (empty ones
+// last, they still write the background), listed by work class.
 __global__ void __launch_bounds__(kBlock) batch_tile_cost_kernel(unsigned tiles,
                                                                  const uint2* __restrict__ ranges,
-                                                                 unsigned* __restrict__ keys,
-                                                                 unsigned* __restrict__ vals) {
+                                                                 StripOrder heavy) {
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= tiles)
         return;
     const uint2 r = ranges[t];
-    const unsigned len = r.y > r.x ? r.y - r.x : 0u;
-    keys[t] = 0xffffu - (len < 0xffffu ? len : 0xffffu);
-    vals[t] = t;
+    strip_order_add(heavy, t, r.y > r.x ? r.y - r.x + 1u : 1u);
 }
 
 // --------------------------------------------------------- stages 7 / 8 --
@@ -210,96 +188,139 @@ enum BatchSchedule : int { kSchedStatic = 0, kSchedDynamic = 1, kSchedHeavyFirst
 struct TileLookup {
     const BatchView* views;
     const unsigned short* tile_view;
-    const unsigned* tile_order; // heaviest-first permutation (schedule 2)
+    StripOrder heavy; // tiles by instance count (heaviest-first forward)
+    StripOrder work;  // strips by adjoint work (heaviest-first adjoint)
 };
 
-// Next tile of this CTA (uniform across the CTA), or >= tiles when done.
+// Place of the CTA's next item in the schedule's order.
 template <int SCHED>
-__device__ __forceinline__ unsigned next_tile(unsigned& k, unsigned tiles, unsigned* queue,
-                                              unsigned* s_item, const TileLookup& L) {
-    unsigned item;
+__device__ __forceinline__ unsigned next_item(unsigned& k, unsigned* queue) {
     if constexpr (SCHED == kSchedStatic) {
-        __syncthreads();
-        item = blockIdx.x + k * gridDim.x;
-        ++k;
+        return blockIdx.x + k++ * gridDim.x;
     } else {
-        if (threadIdx.x == 0)
-            *s_item = atomicAdd(queue, 1u);
-        __syncthreads();
-        item = *s_item;
-        __syncthreads();
+        unsigned item = 0;
+        if (lane_id() == 0)
+            item = atomicAdd(queue, 1u);
+        return __shfl_sync(0xffffffffu, item, 0);
     }
-    if (item >= tiles)
-        return item;
-    return SCHED == kSchedHeavyFirst ? L.tile_order[item] : item;
 }
 
+// Resident warps per SM, as the single-view strip kernels.
+template <int PX> constexpr int kBatchForwardCtas = PX == 8 ? 20 : PX == 4 ? 28 : 32;
+template <int PX> constexpr int kBatchBackwardCtas = PX == 8 ? 16 : PX == 4 ? 20 : 24;
+
 template <int TW, int TH, int PX, int SCHED>
-__global__ void __launch_bounds__(TileGeom<TW, TH, PX>::kThreads) batch_forward_kernel(
-    unsigned tiles, const uint2* __restrict__ ranges, const unsigned* __restrict__ order,
-    GaussianState st, TileLookup L, unsigned* __restrict__ queue, float3 bg,
-    float* __restrict__ color, float* __restrict__ alpha, float* __restrict__ pix_T,
-    unsigned* __restrict__ pix_last) {
-    using G = TileGeom<TW, TH, PX>;
-    __shared__ TileStage<G::kBatch> s;
-    __shared__ unsigned char s_vis[G::kBatch];
-    __shared__ unsigned s_item;
-    for (int k = threadIdx.x; k < G::kBatch; k += G::kThreads)
-        s_vis[k] = 0;
+__global__ void __launch_bounds__(32, kBatchForwardCtas<PX>) batch_forward_kernel(
+    const __grid_constant__ CUtensorMap map, unsigned* __restrict__ err, unsigned tiles,
+    const uint2* __restrict__ ranges, const unsigned* __restrict__ order, TileLookup L,
+    unsigned* __restrict__ queue, float3 bg, float* __restrict__ color, float* __restrict__ alpha,
+    float* __restrict__ pix_T, unsigned* __restrict__ pix_last) {
+    constexpr unsigned kStrips = TH / StripGeom<TW, PX>::kRows;
+    __shared__ StripStage s;
+    StripFeed feed{s, &map, err};
+    feed.init();
     unsigned k = 0;
     for (;;) {
-        const unsigned tile = next_tile<SCHED>(k, tiles, queue, &s_item, L);
-        if (tile >= tiles)
+        const unsigned item = next_item<SCHED>(k, queue);
+        if (item >= tiles * kStrips)
             break;
+        const unsigned at = item / kStrips, strip = item % kStrips;
+        const unsigned tile = SCHED == kSchedHeavyFirst ? strip_order_get(L.heavy, at) : at;
         const unsigned v = L.tile_view[tile];
         const BatchView& bv = L.views[v];
-        const int gx = bv.K.grid_x;
-        const unsigned local = tile - bv.tile_base;
+        const unsigned gx = unsigned(bv.K.grid_x), local = tile - bv.tile_base;
         const size_t pb = bv.pix_base;
         const ViewTarget o{bv.K.width, bv.K.height, bv.K.alpha_clip, bg, color + 3 * pb,
                            alpha + pb, pix_T + pb, pix_last + pb};
-        composite_forward_tile<TW, TH, PX>(s, s_vis, int(local % unsigned(gx)),
-                                           int(local / unsigned(gx)), ranges[tile], order, st, o,
-                                           nullptr);
+        if (!composite_forward_strip<TW, PX>(
+                feed, int(local % gx) * TW,
+                int(local / gx) * TH + int(strip) * StripGeom<TW, PX>::kRows, ranges[tile], order,
+                o, nullptr, L.work, tile * kStrips + strip))
+            break;
+        __syncwarp();
     }
 }
 
 template <int TW, int TH, int PX, int SCHED>
-__global__ void __launch_bounds__(TileGeom<TW, TH, PX>::kThreads) batch_backward_kernel(
-    unsigned tiles, const uint2* __restrict__ ranges, const unsigned* __restrict__ order,
-    GaussianState st, TileLookup L, unsigned* __restrict__ queue, float3 bg,
-    const float* __restrict__ pix_T, const unsigned* __restrict__ pix_last,
-    const float* __restrict__ dL_color, const float* __restrict__ dL_alpha) {
-    using G = TileGeom<TW, TH, PX>;
-    __shared__ BackStage<G::kBatch> sb;
-    __shared__ unsigned s_wmax[G::kWarps];
-    __shared__ unsigned s_item;
-    for (int k = threadIdx.x; k < G::kBatch * 12; k += G::kThreads)
-        (&sb.acc[0][0])[k] = 0.f;
+__global__ void __launch_bounds__(32, kBatchBackwardCtas<PX>) batch_backward_kernel(
+    const __grid_constant__ CUtensorMap map, unsigned* __restrict__ err, unsigned tiles,
+    const uint2* __restrict__ ranges, const unsigned* __restrict__ order, float4* __restrict__ grad,
+    TileLookup L, unsigned* __restrict__ queue, float3 bg, const float* __restrict__ pix_T,
+    const unsigned* __restrict__ pix_last, const float* __restrict__ dL_color,
+    const float* __restrict__ dL_alpha) {
+    constexpr unsigned kStrips = TH / StripGeom<TW, PX>::kRows;
+    __shared__ StripStage s;
+    StripFeed feed{s, &map, err};
+    feed.init();
     unsigned k = 0;
     for (;;) {
-        const unsigned tile = next_tile<SCHED>(k, tiles, queue, &s_item, L);
-        if (tile >= tiles)
+        const unsigned item = next_item<SCHED>(k, queue);
+        if (item >= tiles * kStrips)
             break;
+        const unsigned at = SCHED == kSchedHeavyFirst ? strip_order_get(L.work, item) : item;
+        if (at == 0xffffffffu) // past the strips that have work
+            break;
+        const unsigned tile = at / kStrips, strip = at % kStrips;
         const unsigned v = L.tile_view[tile];
         const BatchView& bv = L.views[v];
-        const int gx = bv.K.grid_x;
-        const unsigned local = tile - bv.tile_base;
+        const unsigned gx = unsigned(bv.K.grid_x), local = tile - bv.tile_base;
         const size_t pb = bv.pix_base;
         const ViewGrads o{bv.K.width,  bv.K.height,
                           bv.K.alpha_clip, bg,
                           pix_T + pb,  pix_last + pb,
                           dL_color + 3 * pb, dL_alpha ? dL_alpha + pb : nullptr,
                           nullptr};
-        composite_backward_tile<TW, TH, PX, true, false>(sb, s_wmax, int(local % unsigned(gx)),
-                                                         int(local / unsigned(gx)), ranges[tile],
-                                                         order, st, o);
+        if (!composite_backward_strip<TW, PX, true, false>(
+                feed, int(local % gx) * TW,
+                int(local / gx) * TH + int(strip) * StripGeom<TW, PX>::kRows, ranges[tile], order,
+                o, grad))
+            break;
+        __syncwarp();
     }
 }
 
 // ------------------------------------------------------------- stage 9 --
 constexpr int kBGBlock = 128;
 constexpr int kBShStride = 49;
+
+// Adds the view-summed structure gradients of Gaussian i to the outputs.
+__device__ __forceinline__ void store_view_sums(int i, const ProjGrad& sum, float refine,
+                                                const Activated& act,
+                                                const float* __restrict__ quats,
+                                                const float* __restrict__ logits,
+                                                const float* __restrict__ filter_3d,
+                                                const GradOutArgs& out) {
+    if (out.refine_weight)
+        out.refine_weight[i] += refine;
+    if (out.means) {
+        out.means[3 * i + 0] += sum.d_mean.x;
+        out.means[3 * i + 1] += sum.d_mean.y;
+        out.means[3 * i + 2] += sum.d_mean.z;
+    }
+    if (out.activated) {
+        if (out.scales) {
+            out.scales[3 * i + 0] += sum.d_scale.x;
+            out.scales[3 * i + 1] += sum.d_scale.y;
+            out.scales[3 * i + 2] += sum.d_scale.z;
+        }
+        if (out.rotations) {
+            out.rotations[4 * i + 0] += sum.d_rot.x;
+            out.rotations[4 * i + 1] += sum.d_rot.y;
+            out.rotations[4 * i + 2] += sum.d_rot.z;
+            out.rotations[4 * i + 3] += sum.d_rot.w;
+        }
+        if (out.opacities)
+            out.opacities[i] += sum.d_opac;
+    } else {
+        const RawGrad rg = chain_to_raw(sum, act, quats, logits, filter_3d, i);
+        if (out.scales)
+            for (int k = 0; k < 3; ++k) out.scales[3 * i + k] += rg.log_s[k];
+        if (out.rotations)
+            for (int k = 0; k < 4; ++k) out.rotations[4 * i + k] += rg.quat[k];
+        if (out.opacities)
+            out.opacities[i] += rg.logit;
+    }
+}
 
 // One thread per Gaussian; loops over the views that saw it, summing the
 // projection and SH adjoints in registers / its shared SH row, then writes
@@ -366,7 +387,7 @@ __global__ void __launch_bounds__(kBGBlock) batch_gaussian_backward_kernel(
         refine += g1.z;
         const float3 dcol = make_float3(g2.x, g2.y, g2.z);
         if (sh) {
-            const unsigned clamp_bits = __float_as_uint(st.rgb[slot].w);
+            const unsigned clamp_bits = __float_as_uint(st.rec[slot].rgb.w);
             const float3 dm = sh_color_backward(
                 reinterpret_cast<const float3*>(sh) + size_t(i) * sh_bases, sh_degree, sh_bases,
                 mean, make_float3(K.center[0], K.center[1], K.center[2]), clamp_bits, dcol,
@@ -392,40 +413,154 @@ __global__ void __launch_bounds__(kBGBlock) batch_gaussian_backward_kernel(
         out.colors[3 * i + 1] += dcol_sum.y;
         out.colors[3 * i + 2] += dcol_sum.z;
     }
-    if (out.refine_weight)
-        out.refine_weight[i] += refine;
-    if (out.means) {
-        out.means[3 * i + 0] += sum.d_mean.x;
-        out.means[3 * i + 1] += sum.d_mean.y;
-        out.means[3 * i + 2] += sum.d_mean.z;
+    store_view_sums(i, sum, refine, act, quats, logits, filter_3d, out);
+}
+
+// The same for 16-byte aligned degree-3 rows: the CTA's rows are staged once by
+// 16-byte copies (one view's adjoint reads a row 48 values at a time, and a
+// row read from HBM per view had each lane on its own line), the coefficient
+// gradients accumulate in shared memory in groups of four, and a view's
+// gradient slot is loaded while the view before it is worked on. Bound: the
+// latency of those loads at 12 to 16 warps per SM. Eight views of 500,000
+// Gaussians 757 -> 266 us.
+constexpr int kBRowStride = 52; // floats: 16-byte accesses of eight rows hit every bank
+
+__global__ void __launch_bounds__(kBGBlock, 4) batch_gaussian_backward48_kernel(
+    int n, int views, const float* __restrict__ means, const float* __restrict__ log_scales,
+    const float* __restrict__ quats, const float* __restrict__ logits,
+    const float* __restrict__ filter_3d, const float* __restrict__ sh, int sh_degree,
+    const BatchView* __restrict__ bviews, GaussianState st, const int* __restrict__ radii,
+    GradOutArgs out) {
+    extern __shared__ float4 smem48[];
+    float* s_coef = reinterpret_cast<float*>(smem48);  // [kBGBlock][kBRowStride]
+    float* s_acc = s_coef + kBGBlock * kBRowStride;    // [kBGBlock][kBRowStride]
+    Camera* sK = reinterpret_cast<Camera*>(s_acc + kBGBlock * kBRowStride);
+    const int tid = threadIdx.x;
+    const int row0 = blockIdx.x * kBGBlock;
+    const int rows = min(kBGBlock, n - row0);
+    for (int e = tid; e < rows * 12; e += kBGBlock) {
+        const int r = e / 12, c = e - 12 * r;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         smem_u32(s_coef + r * kBRowStride + 4 * c)),
+                     "l"(sh + size_t(row0) * 48 + 4 * size_t(e))
+                     : "memory");
     }
-    if (out.activated) {
-        if (out.scales) {
-            out.scales[3 * i + 0] += sum.d_scale.x;
-            out.scales[3 * i + 1] += sum.d_scale.y;
-            out.scales[3 * i + 2] += sum.d_scale.z;
-        }
-        if (out.rotations) {
-            out.rotations[4 * i + 0] += sum.d_rot.x;
-            out.rotations[4 * i + 1] += sum.d_rot.y;
-            out.rotations[4 * i + 2] += sum.d_rot.z;
-            out.rotations[4 * i + 3] += sum.d_rot.w;
-        }
-        if (out.opacities)
-            out.opacities[i] += sum.d_opac;
-    } else {
-        const RawGrad rg = chain_to_raw(sum, act, quats, logits, filter_3d, i);
-        if (out.scales)
-            for (int k = 0; k < 3; ++k) out.scales[3 * i + k] += rg.log_s[k];
-        if (out.rotations)
-            for (int k = 0; k < 4; ++k) out.rotations[4 * i + k] += rg.quat[k];
-        if (out.opacities)
-            out.opacities[i] += rg.logit;
+    constexpr int kWords = int(sizeof(Camera) / 4);
+    for (int k = tid; k < views * kWords; k += kBGBlock) {
+        const int v = k / kWords, w = k - v * kWords;
+        reinterpret_cast<unsigned*>(sK)[k] = reinterpret_cast<const unsigned*>(&bviews[v].K)[w];
     }
+    float4* acc = reinterpret_cast<float4*>(s_acc + tid * kBRowStride);
+#pragma unroll
+    for (int c = 0; c < 12; ++c)
+        acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const int i = row0 + tid;
+    if (i >= n)
+        return;
+    const float3 mean = make_float3(means[3 * i], means[3 * i + 1], means[3 * i + 2]);
+    const Activated act = activate(log_scales, quats, logits, filter_3d, i);
+    ProjGrad sum;
+    sum.d_mean = make_float3(0.f, 0.f, 0.f);
+    sum.d_scale = make_float3(0.f, 0.f, 0.f);
+    sum.d_rot = make_float4(0.f, 0.f, 0.f, 0.f);
+    sum.d_opac = 0.f;
+    float refine = 0.f;
+    bool any = false;
+    struct Slot {
+        float4 g0, g1, g2;
+        unsigned clamp;
+    };
+    auto load = [&](int v, Slot& o) {
+        const size_t slot = size_t(v) * size_t(n) + size_t(i);
+        if (radii[slot] <= 0)
+            return false;
+        const float4* g = st.grad + slot * kGradSlots;
+        o.g0 = g[0];
+        o.g1 = g[1];
+        o.g2 = g[2];
+        o.clamp = __float_as_uint(st.rec[slot].rgb.w);
+        return true;
+    };
+    Slot next;
+    bool seen_next = load(0, next);
+#pragma unroll 1
+    for (int v = 0; v < views; ++v) {
+        const Slot cur = next;
+        const bool seen = seen_next;
+        if (v + 1 < views)
+            seen_next = load(v + 1, next);
+        if (!seen)
+            continue;
+        any = true;
+        float4* g = st.grad + (size_t(v) * size_t(n) + size_t(i)) * kGradSlots;
+        g[0] = g[1] = g[2] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const Camera& K = sK[v];
+        const ProjGrad pg = projection_backward(mean, K, act.scale, act.rot, cur.g0,
+                                                make_float2(cur.g1.x, cur.g1.y));
+        sum.d_mean.x += pg.d_mean.x;
+        sum.d_mean.y += pg.d_mean.y;
+        sum.d_mean.z += pg.d_mean.z;
+        sum.d_scale.x += pg.d_scale.x;
+        sum.d_scale.y += pg.d_scale.y;
+        sum.d_scale.z += pg.d_scale.z;
+        sum.d_rot.x += pg.d_rot.x;
+        sum.d_rot.y += pg.d_rot.y;
+        sum.d_rot.z += pg.d_rot.z;
+        sum.d_rot.w += pg.d_rot.w;
+        sum.d_opac += pg.d_opac;
+        refine += cur.g1.z;
+        float4 q[12];
+#pragma unroll
+        for (int c = 0; c < 12; ++c)
+            q[c] = reinterpret_cast<const float4*>(s_coef + tid * kBRowStride)[c];
+        const float* f = reinterpret_cast<const float*>(q);
+        float3 c[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            c[k] = make_float3(f[3 * k], f[3 * k + 1], f[3 * k + 2]);
+        const float3 dcol = make_float3(cur.g2.x, cur.g2.y, cur.g2.z);
+        float w[19]; // basis values, clamped colour gradient
+        const float3 dm = sh_color_backward<true>(
+            c, sh_degree, 16, mean, make_float3(K.center[0], K.center[1], K.center[2]), cur.clamp,
+            dcol, nullptr, w);
+        sum.d_mean.x += dm.x;
+        sum.d_mean.y += dm.y;
+        sum.d_mean.z += dm.z;
+#pragma unroll
+        for (int e = 0; e < 12; ++e) {
+            float4 a = acc[e];
+            a.x += w[(4 * e) / 3] * w[16 + (4 * e) % 3];
+            a.y += w[(4 * e + 1) / 3] * w[16 + (4 * e + 1) % 3];
+            a.z += w[(4 * e + 2) / 3] * w[16 + (4 * e + 2) % 3];
+            a.w += w[(4 * e + 3) / 3] * w[16 + (4 * e + 3) % 3];
+            acc[e] = a;
+        }
+    }
+    if (!any)
+        return;
+    if (out.sh) {
+        float4* dst = reinterpret_cast<float4*>(out.sh + size_t(i) * 48);
+#pragma unroll
+        for (int e = 0; e < 12; ++e) {
+            float4 a = dst[e];
+            const float4 b = acc[e];
+            a.x += b.x;
+            a.y += b.y;
+            a.z += b.z;
+            a.w += b.w;
+            dst[e] = a;
+        }
+    }
+    store_view_sums(i, sum, refine, act, quats, logits, filter_3d, out);
 }
 
 size_t batch_gaussian_backward_smem(int views) {
     return size_t(views) * sizeof(Camera) + size_t(2) * kBGBlock * kBShStride * sizeof(float);
+}
+size_t batch_gaussian_backward48_smem(int views) {
+    return size_t(views) * sizeof(Camera) + size_t(2) * kBGBlock * kBRowStride * sizeof(float);
 }
 
 } // namespace gsb
@@ -444,6 +579,14 @@ bool valid_shape(int tw, int th, int ppt) {
     return false;
 }
 
+// Pixels per thread of the strips: the schedule's, but eight for four once the
+// views give as many 16x16 tiles as the single-view rule asks for eight
+// (kAutoPx4Tiles in capi.cu; both sides measured there).
+int strip_px(const gs_batch_schedule& s, size_t tiles) {
+    const size_t tiles16 = tiles * size_t(s.tile_w) * size_t(s.tile_h) / 256;
+    return s.pixels_per_thread == 4 && tiles16 > 4800 ? 8 : s.pixels_per_thread;
+}
+
 // Dispatch a lambda templated on <TW, TH> / <TW, TH, PX> to the compiled variants.
 template <typename F> void with_tile(int tw, int th, F&& f) {
     if (tw == 8 && th == 8) f.template operator()<8, 8>();
@@ -457,8 +600,10 @@ template <typename F> void with_shape(int tw, int th, int ppt, F&& f) {
     else if (tw == 8 && th == 8 && ppt == 2) f.template operator()<8, 8, 2>();
     else if (tw == 16 && th == 16 && ppt == 2) f.template operator()<16, 16, 2>();
     else if (tw == 16 && th == 16 && ppt == 4) f.template operator()<16, 16, 4>();
+    else if (tw == 16 && th == 16 && ppt == 8) f.template operator()<16, 16, 8>();
     else if (tw == 16 && th == 32 && ppt == 2) f.template operator()<16, 32, 2>();
     else if (tw == 16 && th == 32 && ppt == 4) f.template operator()<16, 32, 4>();
+    else if (tw == 16 && th == 32 && ppt == 8) f.template operator()<16, 32, 8>();
     else throw InvalidArg("gsplat_b200: unsupported batch tile shape / pixels per thread");
 }
 
@@ -477,13 +622,15 @@ struct gs_batch {
     int views = 0;
     size_t pairs = 0, capacity = 0, total_pixels = 0;
     unsigned total_tiles = 0;
-    int tile_bits = 0, cost_bits = 16;
+    int tile_bits = 0;
+    int px = 4; // pixels per thread of the strips
+    bool rows48_fits = false;
     int grid_fwd = 0, grid_bwd = 0;
-    int depth_result = 0, inst_result = 0, cost_result = 0;
+    int depth_result = 0, inst_result = 0;
     std::vector<BatchView> host_views;
     // device buffers
     DevBuf views_buf, tile_view_buf, state_buf, grad_buf, radii_buf, dsort_buf, isort_buf,
-        ranges_buf, cost_buf, pixel_buf, hist_buf, status_buf, scan_status_buf, tile_ctr_buf,
+        ranges_buf, order_buf, pixel_buf, hist_buf, status_buf, scan_status_buf, tile_ctr_buf,
         counters_buf, groups_buf;
     unsigned* emit_groups = nullptr; // the emit's instance groups, cut by the offset scan
     int group_shift = 9;
@@ -496,8 +643,8 @@ struct gs_batch {
     unsigned* dvals[2] = {nullptr, nullptr};
     unsigned* ikeys[2] = {nullptr, nullptr};
     unsigned* ivals[2] = {nullptr, nullptr};
-    unsigned* ckeys[2] = {nullptr, nullptr};
-    unsigned* cvals[2] = {nullptr, nullptr};
+    StripOrder heavy{}, work{}; // heaviest-first orders (counts NULL: not kept)
+    RecStaging staging{};
     uint2* ranges = nullptr;
     float* pix_T = nullptr;
     unsigned* pix_last = nullptr;
@@ -548,28 +695,17 @@ void drop_graph(gs_batch* b) {
 
 GaussianState carve_state(char* p, size_t cap) {
     GaussianState st{};
-    st.mean2d = reinterpret_cast<float2*>(p);
-    p += align_up(cap * 8);
-    st.conic = reinterpret_cast<float4*>(p);
-    p += align_up(cap * 16);
-    st.rgb = reinterpret_cast<float4*>(p);
-    p += align_up(cap * 16);
+    st.rec = reinterpret_cast<SplatRec*>(p);
+    p += align_up(cap * sizeof(SplatRec));
     st.depth = reinterpret_cast<unsigned*>(p);
     p += align_up(cap * 4);
     st.touched = reinterpret_cast<unsigned*>(p);
     p += align_up(cap * 4);
     st.offset = reinterpret_cast<unsigned*>(p);
-    p += align_up(cap * 4);
-    st.bounds = reinterpret_cast<ushort4*>(p);
-    p += align_up(cap * 8);
-    st.spans = reinterpret_cast<uint4*>(p);
     return st;
 }
 
-size_t state_bytes(size_t cap) {
-    return align_up(cap * 8) + align_up(cap * 16) * 2 + align_up(cap * 4) * 3 + align_up(cap * 8) +
-           align_up(cap * 16);
-}
+size_t state_bytes(size_t cap) { return align_up(cap * sizeof(SplatRec)) + align_up(cap * 4) * 3; }
 
 void launch_preprocess_stage(gs_batch* b) {
     const gs_gaussians& g = b->g;
@@ -615,34 +751,33 @@ void enqueue_forward(gs_batch* b, float* color, float* alpha) {
                 b->counters + kBcTotal, b->counters + kBcErr, /*zeroed=*/false, b->emit_groups,
                 b->group_shift, b->group_cap);
     const unsigned emit_blocks = (b->group_cap + kBatchEmitBlock / 32 - 1) / (kBatchEmitBlock / 32);
-    with_shape(b->sched.tile_w, b->sched.tile_h, b->sched.pixels_per_thread,
-               [&]<int TW, int TH, int PX>() {
-                   batch_emit_kernel<TW, TH><<<emit_blocks, kBatchEmitBlock, 0, s>>>(
-                       n, b->counters, b->emit_groups, b->group_shift, b->group_cap, order, b->st,
-                       b->d_views, b->ikeys[0], b->ivals[0], unsigned(b->capacity));
-               });
-    b->inst_result = launch_radix_sort<unsigned>(s, b->ikeys, b->ivals, b->capacity,
-                                                 b->counters + kBcSorted, 0, b->tile_bits, hist,
-                                                 status, tctr, b->counters + kBcErr);
+    // the emit counts the tile sort's digits (the depth sort's counts are done with)
+    ck(cudaMemsetAsync(hist, 0, 3 * kMaxRadix * sizeof(unsigned), s), "digit counts");
+    with_tile(b->sched.tile_w, b->sched.tile_h, [&]<int TW, int TH>() {
+        batch_emit_kernel<TW, TH><<<emit_blocks, kBatchEmitBlock, 0, s>>>(
+            n, b->counters, b->emit_groups, b->group_shift, b->group_cap, order, b->st, b->d_views,
+            b->ikeys[0], b->ivals[0], unsigned(b->capacity), b->tile_bits, hist);
+    });
+    b->inst_result = launch_radix_sort<unsigned>(
+        s, b->ikeys, b->ivals, b->capacity, b->counters + kBcSorted, 0, b->tile_bits, hist, status,
+        tctr, b->counters + kBcErr, /*hist_ready=*/true);
     ck(cudaMemsetAsync(b->ranges, 0, size_t(b->total_tiles) * sizeof(uint2), s), "ranges");
-    batch_ranges_kernel<<<int((b->capacity + kBlock - 1) / kBlock), kBlock, 0, s>>>(
-        b->counters, b->ikeys[b->inst_result], b->ranges, b->total_tiles);
+    launch_tile_ranges(s, b->capacity, b->counters + kBcSorted, b->ikeys[b->inst_result],
+                       b->ranges, int(b->total_tiles));
     if (b->sched.schedule == kSchedHeavyFirst) {
+        ck(cudaMemsetAsync(b->heavy.count, 0, 2 * kWorkClasses * sizeof(unsigned), s), "orders");
         batch_tile_cost_kernel<<<int((b->total_tiles + kBlock - 1) / kBlock), kBlock, 0, s>>>(
-            b->total_tiles, b->ranges, b->ckeys[0], b->cvals[0]);
-        b->cost_result = launch_radix_sort<unsigned>(s, b->ckeys, b->cvals, b->total_tiles,
-                                                     b->counters + kBcTiles, 0, b->cost_bits,
-                                                     hist, status, tctr, b->counters + kBcErr);
+            b->total_tiles, b->ranges, b->heavy);
     }
-    const TileLookup L{b->d_views, b->d_tile_view, b->cvals[b->cost_result]};
+    const TileLookup L{b->d_views, b->d_tile_view, b->heavy, b->work};
     const float3 bg = make_float3(b->s.background[0], b->s.background[1], b->s.background[2]);
-    with_shape(b->sched.tile_w, b->sched.tile_h, b->sched.pixels_per_thread,
+    with_shape(b->sched.tile_w, b->sched.tile_h, b->px,
                [&]<int TW, int TH, int PX>() {
-                   using G = TileGeom<TW, TH, PX>;
                    auto go = [&](auto kernel) {
-                       kernel<<<b->grid_fwd, G::kThreads, 0, s>>>(
-                           b->total_tiles, b->ranges, b->ivals[b->inst_result], b->st, L,
-                           b->counters + kBcWork, bg, color, alpha, b->pix_T, b->pix_last);
+                       kernel<<<b->grid_fwd, 32, 0, s>>>(
+                           b->staging.map, b->staging.err, b->total_tiles, b->ranges,
+                           b->ivals[b->inst_result], L, b->counters + kBcWork, bg, color, alpha,
+                           b->pix_T, b->pix_last);
                    };
                    if (b->sched.schedule == kSchedStatic)
                        go(batch_forward_kernel<TW, TH, PX, kSchedStatic>);
@@ -654,20 +789,25 @@ void enqueue_forward(gs_batch* b, float* color, float* alpha) {
     ck(cudaGetLastError(), "batch forward launch");
 }
 
+// 16 SH bases with 16-byte aligned rows, in and out.
+bool rows48(const gs_gaussians& g, const float* sh_grad) {
+    return g.sh && g.sh_bases == 16 &&
+           ((reinterpret_cast<uintptr_t>(g.sh) | reinterpret_cast<uintptr_t>(sh_grad)) & 15) == 0;
+}
+
 void enqueue_backward(gs_batch* b, const float* dL_color, const float* dL_alpha,
                       const gs_model_grads* grads) {
     cudaStream_t s = b->stream;
     ck(cudaMemsetAsync(b->counters + kBcWorkBack, 0, sizeof(unsigned), s), "queue reset");
-    const TileLookup L{b->d_views, b->d_tile_view, b->cvals[b->cost_result]};
+    const TileLookup L{b->d_views, b->d_tile_view, b->heavy, b->work};
     const float3 bg = make_float3(b->s.background[0], b->s.background[1], b->s.background[2]);
-    with_shape(b->sched.tile_w, b->sched.tile_h, b->sched.pixels_per_thread,
+    with_shape(b->sched.tile_w, b->sched.tile_h, b->px,
                [&]<int TW, int TH, int PX>() {
-                   using G = TileGeom<TW, TH, PX>;
                    auto go = [&](auto kernel) {
-                       kernel<<<b->grid_bwd, G::kThreads, 0, s>>>(
-                           b->total_tiles, b->ranges, b->ivals[b->inst_result], b->st, L,
-                           b->counters + kBcWorkBack, bg, b->pix_T, b->pix_last, dL_color,
-                           dL_alpha);
+                       kernel<<<b->grid_bwd, 32, 0, s>>>(
+                           b->staging.map, b->staging.err, b->total_tiles, b->ranges,
+                           b->ivals[b->inst_result], b->st.grad, L, b->counters + kBcWorkBack, bg,
+                           b->pix_T, b->pix_last, dL_color, dL_alpha);
                    };
                    if (b->sched.schedule == kSchedStatic)
                        go(batch_backward_kernel<TW, TH, PX, kSchedStatic>);
@@ -688,10 +828,17 @@ void enqueue_backward(gs_batch* b, const float* dL_color, const float* dL_alpha,
         out.activated = grads->activated;
     }
     const gs_gaussians& g = b->g;
-    batch_gaussian_backward_kernel<<<(g.count + kBGBlock - 1) / kBGBlock, kBGBlock,
-                                     batch_gaussian_backward_smem(b->views), s>>>(
-        g.count, b->views, g.means, g.log_scales, g.quaternions, g.opacity_logits, g.filter_3d,
-        g.sh, g.sh_degree, g.sh_bases, b->d_views, b->st, b->radii, out);
+    const int blocks = (g.count + kBGBlock - 1) / kBGBlock;
+    if (b->rows48_fits && rows48(g, out.sh))
+        batch_gaussian_backward48_kernel<<<blocks, kBGBlock,
+                                           batch_gaussian_backward48_smem(b->views), s>>>(
+            g.count, b->views, g.means, g.log_scales, g.quaternions, g.opacity_logits, g.filter_3d,
+            g.sh, g.sh_degree, b->d_views, b->st, b->radii, out);
+    else
+        batch_gaussian_backward_kernel<<<blocks, kBGBlock, batch_gaussian_backward_smem(b->views),
+                                         s>>>(
+            g.count, b->views, g.means, g.log_scales, g.quaternions, g.opacity_logits, g.filter_3d,
+            g.sh, g.sh_degree, g.sh_bases, b->d_views, b->st, b->radii, out);
     ck(cudaGetLastError(), "batch backward launch");
 }
 
@@ -802,23 +949,26 @@ void plan(gs_batch* b, const gs_gaussians* g, const gs_camera* cams, int views,
     b->pix_T = reinterpret_cast<float*>(px);
     b->pix_last = reinterpret_cast<unsigned*>(px + align_up(pixels * 4));
     b->ranges = reinterpret_cast<uint2*>(b->ranges_buf.exact(tiles * sizeof(uint2), st));
-    char* cst = b->cost_buf.exact(align_up(tiles * 4) * 4, st);
-    for (int k = 0; k < 2; ++k) {
-        b->ckeys[k] = reinterpret_cast<unsigned*>(cst + align_up(tiles * 4) * k);
-        b->cvals[k] = reinterpret_cast<unsigned*>(cst + align_up(tiles * 4) * (2 + k));
-    }
+    b->px = strip_px(sc, tiles);
     b->counters = reinterpret_cast<unsigned*>(b->counters_buf.exact(kBcWords * 4, st, true));
+    encode_record_map(&b->staging.map, b->st.rec, pairs);
+    b->staging.err = b->counters + kBcErr;
     b->hist_buf.exact(8 * kMaxRadix * sizeof(unsigned), st);
     b->tile_ctr_buf.exact(64 * sizeof(unsigned), st);
     b->scan_status_buf.exact(std::max<size_t>(scan_status_bytes(int(pairs)), 256), st);
     // the schedule's kernels: grid sizes and attributes
     const size_t gsmem = batch_gaussian_backward_smem(views);
     req(gsmem <= 227 * 1024, "too many views for the per-Gaussian backward");
+    const size_t gsmem48 = batch_gaussian_backward48_smem(views);
+    b->rows48_fits = gsmem48 <= 227 * 1024;
+    if (b->rows48_fits)
+        ck(cudaFuncSetAttribute(batch_gaussian_backward48_kernel,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, int(gsmem48)),
+           "smem attribute");
     ck(cudaFuncSetAttribute(batch_gaussian_backward_kernel,
                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(gsmem)),
        "smem attribute");
-    with_shape(sc.tile_w, sc.tile_h, sc.pixels_per_thread, [&]<int TW, int TH, int PX>() {
-        using G = TileGeom<TW, TH, PX>;
+    with_shape(sc.tile_w, sc.tile_h, b->px, [&]<int TW, int TH, int PX>() {
         const void* fk;
         const void* bk;
         if (sc.schedule == kSchedStatic) {
@@ -832,10 +982,23 @@ void plan(gs_batch* b, const gs_gaussians* g, const gs_camera* cams, int views,
             bk = reinterpret_cast<const void*>(
                 batch_backward_kernel<TW, TH, PX, kSchedHeavyFirst>);
         }
-        const int of = sc.ctas_per_sm > 0 ? sc.ctas_per_sm : occupancy(fk, G::kThreads, 0);
-        const int ob = sc.ctas_per_sm > 0 ? sc.ctas_per_sm : occupancy(bk, G::kThreads, 0);
-        b->grid_fwd = int(std::min<size_t>(size_t(b->sms) * of, tiles));
-        b->grid_bwd = int(std::min<size_t>(size_t(b->sms) * ob, tiles));
+        // ctas_per_sm counts tiles in flight: a tile's strips are CTAs of their own
+        const size_t strips = TH / StripGeom<TW, PX>::kRows;
+        const size_t of = sc.ctas_per_sm > 0 ? sc.ctas_per_sm * strips : occupancy(fk, 32, 0);
+        const size_t ob = sc.ctas_per_sm > 0 ? sc.ctas_per_sm * strips : occupancy(bk, 32, 0);
+        const size_t items = tiles * strips;
+        req(items < (size_t(1) << 31), "too many tiles");
+        b->grid_fwd = int(std::min<size_t>(size_t(b->sms) * of, items));
+        b->grid_bwd = int(std::min<size_t>(size_t(b->sms) * ob, items));
+        b->heavy = b->work = StripOrder{};
+        if (sc.schedule == kSchedHeavyFirst) {
+            // counts of both orders side by side (one memset), then the lists
+            unsigned* w = reinterpret_cast<unsigned*>(b->order_buf.exact(
+                sizeof(unsigned) * kWorkClasses * (2 + tiles + items), st));
+            b->heavy = {w, w + 2 * kWorkClasses, unsigned(tiles)};
+            b->work = {w + kWorkClasses, w + 2 * kWorkClasses + kWorkClasses * tiles,
+                       unsigned(items)};
+        }
     });
     // instance capacity
     size_t cap = instance_capacity;
@@ -860,10 +1023,8 @@ void plan(gs_batch* b, const gs_gaussians* g, const gs_camera* cams, int views,
     }
     const size_t status = std::max({sort_status_bytes(pairs, radix_plan(32)),
                                     sort_status_bytes(cap, radix_plan(b->tile_bits)),
-                                    sort_status_bytes(tiles, radix_plan(b->cost_bits)),
                                     size_t(256)});
     b->status_buf.exact(status, st);
-    b->cost_result = 0;
     ck(cudaStreamSynchronize(st), "plan sync");
     b->planned = true;
 }
@@ -905,9 +1066,9 @@ void gs_batch_destroy(gs_batch* b) {
         cudaDeviceSynchronize();
     drop_graph(b);
     for (DevBuf* d : {&b->views_buf, &b->tile_view_buf, &b->state_buf, &b->grad_buf,
-                      &b->radii_buf, &b->dsort_buf, &b->isort_buf, &b->ranges_buf, &b->cost_buf,
+                      &b->radii_buf, &b->dsort_buf, &b->isort_buf, &b->ranges_buf, &b->order_buf,
                       &b->pixel_buf, &b->hist_buf, &b->status_buf, &b->scan_status_buf,
-                      &b->tile_ctr_buf, &b->counters_buf})
+                      &b->tile_ctr_buf, &b->counters_buf, &b->groups_buf})
         d->release();
     if (b->host_counters)
         cudaFreeHost(b->host_counters);

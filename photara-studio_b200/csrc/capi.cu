@@ -201,35 +201,6 @@ void check_forward_sorts(gs_context* c) {
         raise_timeout(c, c->host_counts[8], "in the forward's sorts");
 }
 
-// The record array as a [rows][16] float32 tensor with a box of one row (the
-// shape tile::gather4 copies), encoded through the driver's
-// cuTensorMapEncodeTiled (reached through the runtime, so the library links
-// no driver stub). The driver checks the base (16-byte aligned) and the row
-// stride (64 bytes).
-void encode_record_map(gs_context* c, size_t rows) {
-    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-    if (!encode) {
-        cudaDriverEntryPointQueryResult q{};
-        ck(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled",
-                                            reinterpret_cast<void**>(&encode), 12000,
-                                            cudaEnableDefault, &q),
-           "driver entry point cuTensorMapEncodeTiled");
-        if (q != cudaDriverEntryPointSuccess || !encode)
-            throw std::runtime_error("gsplat_b200: cuTensorMapEncodeTiled is not available");
-    }
-    const cuuint64_t dims[2] = {16, cuuint64_t(rows)};
-    const cuuint64_t strides[1] = {sizeof(SplatRec)};
-    const cuuint32_t box[2] = {16, 1};
-    const cuuint32_t elem[2] = {1, 1};
-    const CUresult r = encode(&c->staging.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, c->st.rec,
-                              dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS)
-        throw std::runtime_error("gsplat_b200: cuTensorMapEncodeTiled failed (" +
-                                 std::to_string(int(r)) + ")");
-}
-
 const RecStaging& record_staging(gs_context* c) {
     c->staging.err = device_error_word(c);
     return c->staging;
@@ -239,28 +210,19 @@ void carve_gaussians(gs_context* c, int n) {
     const size_t N = size_t(n);
     if (N > c->gauss_cap) {
         const size_t cap = N + N / 4 + 1024;
-        const size_t bytes = align_up(cap * 8) + align_up(cap * 16) * 4 + align_up(cap * 4) * 3 +
-                             align_up(cap * 8);
+        const size_t bytes = align_up(cap * 4) * 3 + align_up(cap * 16) * 2;
         char* p = c->gauss.ensure(bytes, c->stream);
-        c->st.mean2d = reinterpret_cast<float2*>(p);
-        p += align_up(cap * 8);
-        c->st.conic = reinterpret_cast<float4*>(p);
-        p += align_up(cap * 16);
-        c->st.rgb = reinterpret_cast<float4*>(p);
-        p += align_up(cap * 16);
         c->st.depth = reinterpret_cast<unsigned*>(p);
         p += align_up(cap * 4);
         c->st.touched = reinterpret_cast<unsigned*>(p);
         p += align_up(cap * 4);
         c->st.offset = reinterpret_cast<unsigned*>(p);
         p += align_up(cap * 4);
-        c->st.bounds = reinterpret_cast<ushort4*>(p);
-        p += align_up(cap * 8);
         c->plane = reinterpret_cast<float4*>(p);
         p += align_up(cap * 16);
         c->normal = reinterpret_cast<float4*>(p);
         c->st.rec = reinterpret_cast<SplatRec*>(c->rec.ensure(cap * sizeof(SplatRec), c->stream));
-        encode_record_map(c, cap);
+        encode_record_map(&c->staging.map, c->st.rec, cap);
         c->gauss_cap = cap;
     }
     if (N > c->grad_cap) {
@@ -342,7 +304,7 @@ void gs_destroy(gs_context* c) {
     for (DevBuf* b : {&c->gauss, &c->grad, &c->scan_status, &c->counters, &c->inst_keys,
                       &c->inst_vals, &c->sort_hist, &c->sort_status, &c->sort_counters,
                       &c->ranges, &c->pixel, &c->depth_sort, &c->loss, &c->probe,
-                      &c->geo_grad})
+                      &c->geo_grad, &c->rec, &c->emit_groups})
         b->release();
     if (c->host_counts)
         cudaFreeHost(c->host_counts);
@@ -370,7 +332,7 @@ size_t gs_workspace_bytes(const gs_context* c) {
     for (const DevBuf* b : {&c->gauss, &c->grad, &c->scan_status, &c->counters, &c->inst_keys,
                             &c->inst_vals, &c->sort_hist, &c->sort_status, &c->sort_counters,
                             &c->ranges, &c->pixel, &c->depth_sort, &c->loss, &c->probe,
-                            &c->geo_grad})
+                            &c->geo_grad, &c->rec, &c->emit_groups})
         t += b->bytes;
     return t;
 }
@@ -523,7 +485,7 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
             ck(cudaGetLastError(), "sort launch");
             mark(c, 3, true);
             mark(c, 4, false);
-            launch_tile_ranges(st, int(instances), tkeys[cur],
+            launch_tile_ranges(st, instances, nullptr, tkeys[cur],
                                reinterpret_cast<uint2*>(c->ranges.p), tiles);
             ck(cudaGetLastError(), "ranges launch");
             mark(c, 4, true);
@@ -915,7 +877,7 @@ gs_status gs_forward_colors(gs_context* c, const float* colors, const gs_outputs
         req(colors && out && out->color && out->alpha, "invalid colour reuse arguments");
         check_forward_sorts(c);
         const int n = c->g.count;
-        ck(launch_set_colors(c->stream, n, colors, c->st.rgb, c->st.rec), "colour slots");
+        ck(launch_set_colors(c->stream, n, colors, c->st.rec), "colour slots");
         c->g.colors = colors;
         // empty tiles (ranges zeroed by the forward) composite the background
         launch_composite_forward(c->stream, c->tiles, reinterpret_cast<const uint2*>(c->ranges.p),

@@ -21,9 +21,10 @@ enum DeviceError : unsigned {
 
 // The compositing inputs of one Gaussian in one 64-byte record (four per
 // TMA gather): conic and opacity, colour and clamp bits, centre, alpha box.
-// Written by the preprocess next to the per-field arrays; the single-view
-// compositing kernels stage it into shared memory with tile::gather4 copies.
-// The last 16 bytes, which the compositing kernels do not read, hold the
+// Written by the preprocess for every visible Gaussian, the only copy of these
+// fields: the compositing kernels stage it into shared memory with
+// tile::gather4 copies, the others read what they need of its one 64-byte
+// line. The last 16 bytes, which the compositing kernels do not read, hold the
 // preprocess's tile walk in compact form (TileSpans) for the instance emit.
 struct __align__(16) SplatRec {
     float4 co;      // conic (xx, xy, yy), opacity * coefficient
@@ -36,22 +37,16 @@ static_assert(sizeof(SplatRec) == 64, "one TMA row per record");
 
 // Per-Gaussian forward state (structure of arrays, one slot per Gaussian).
 struct GaussianState {
-    float2* mean2d;     // pixel-space centre
-    float4* conic;      // inverse screen covariance (xx, xy, yy), opacity * coef
-    float4* rgb;        // SH colour; w holds the clamp bits as an int
+    SplatRec* rec;      // centre, conic, colour, box and tile walk
     unsigned* depth;    // radial depth as ordered float bits
     unsigned* touched;  // tiles overlapped
     unsigned* offset;   // exclusive scan of touched
-    ushort4* bounds;    // [x0,x1) [y0,y1) pixel box of the alpha >= 1/255 ellipse
     float4* grad;       // 3 float4 per Gaussian, see GradSlot
     float4* plane;      // ray plane (depth over screen offset, peak distance, 1/sigma);
                         // NULL unless the median-depth channel is rendered
     float4* normal;     // camera-space footprint normal (w unused); with plane
     float4* geo_grad;   // 2 float4 per Gaussian, see kGeoGradSlots; NULL unless the
                         // median-depth / normal channels are differentiated
-    SplatRec* rec;      // packed compositing inputs (NULL: not written)
-    uint4* spans;       // the tile walk's span records where no SplatRec holds them
-                        // (NULL: not written)
 };
 
 // Geometry-channel backward scratch per Gaussian, 2 x float4 (32 B), zeroed

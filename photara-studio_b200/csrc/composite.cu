@@ -172,9 +172,9 @@ __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
         if (base + tid < n) {
             const unsigned g = order[range.x + base + tid];
             s_id[tid] = g;
-            s_xy[tid] = st.mean2d[g];
-            s_co[tid] = st.conic[g];
-            s_rgb[tid] = st.rgb[g];
+            s_xy[tid] = st.rec[g].xy;
+            s_co[tid] = st.rec[g].co;
+            s_rgb[tid] = st.rec[g].rgb;
             s_plane[tid] = st.plane[g];
             s_nrm[tid] = st.normal[g];
         }
@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
                 break;
             if (base + tid < int(block_max)) {
                 const unsigned g = order[range.x + base + tid];
-                s_xy[tid] = st.mean2d[g];
-                s_co[tid] = st.conic[g];
+                s_xy[tid] = st.rec[g].xy;
+                s_co[tid] = st.rec[g].co;
                 s_plane[tid] = st.plane[g];
             }
             __syncthreads();
@@ -348,8 +348,8 @@ __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
                 break;
             if (base + tid < int(block_max)) {
                 const unsigned g = order[range.x + base + tid];
-                s_xy[tid] = st.mean2d[g];
-                s_co[tid] = st.conic[g];
+                s_xy[tid] = st.rec[g].xy;
+                s_co[tid] = st.rec[g].co;
                 s_plane[tid] = st.plane[g];
             }
             __syncthreads();
@@ -545,12 +545,12 @@ __global__ void __launch_bounds__(kGeoThreads) composite_backward_geometry_kerne
         if (tid < cnt) {
             const unsigned g = order[range.x + base + tid];
             s.id[tid] = g;
-            s.xy[tid] = st.mean2d[g];
-            s.co[tid] = st.conic[g];
-            s.rgb[tid] = st.rgb[g];
+            s.xy[tid] = st.rec[g].xy;
+            s.co[tid] = st.rec[g].co;
+            s.rgb[tid] = st.rec[g].rgb;
             s.plane[tid] = st.plane[g];
             s.nrm[tid] = st.normal[g];
-            const ushort4 bx = st.bounds[g];
+            const ushort4 bx = st.rec[g].bounds;
             unsigned m = 0;
 #pragma unroll
             for (int w = 0; w < kGeoThreads / 32; ++w)

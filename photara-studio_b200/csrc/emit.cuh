@@ -8,8 +8,62 @@
 #pragma once
 
 #include "common.cuh"
+#include "kernels.h"
 
 namespace gsb {
+
+// The radix sort's digit histograms of the keys a kernel writes, counted as
+// they are written (the digits of radix_plan over key bits [0, bits), up to 4
+// passes): the sort then skips its own read of the keys. Per-block shared
+// histograms, flushed with one global atomic per non-empty bin. A digit of w
+// bits has 2^(9 - w) counters per bin in neighbouring banks, taken by lane:
+// neighbouring instances mostly share their high tile digit, and 32 lanes on
+// one counter are served one by one (emit at 1M / 1080p 68 us on single
+// counters of 7 + 6 bits).
+struct DigitCounter {
+    unsigned (*h)[kMaxRadix];
+    RadixPlan plan;
+    int w0, c0, w1, c1; // widths and counter bits of the first two digits
+    unsigned l0, l1;    // the lane's counter among a bin's
+    __device__ __forceinline__ DigitCounter(unsigned (*hist)[kMaxRadix], int bits)
+        : h(hist), plan(radix_plan(bits)) {
+        w0 = plan.width(0);
+        c0 = kMaxDigitBits - w0;
+        l0 = lane_id() & ((1u << c0) - 1u);
+        w1 = plan.passes > 1 ? plan.width(1) : 0;
+        c1 = kMaxDigitBits - w1;
+        l1 = lane_id() & ((1u << c1) - 1u);
+    }
+    __device__ __forceinline__ void zero() {
+        for (int k = threadIdx.x; k < plan.passes * kMaxRadix; k += blockDim.x)
+            (&h[0][0])[k] = 0;
+    }
+    __device__ __forceinline__ void count(unsigned key) {
+        atomicAdd(&h[0][((key << c0) & (kMaxRadix - 1)) | l0], 1u);
+        if (plan.passes > 1) {
+            key >>= w0;
+            atomicAdd(&h[1][((key << c1) & (kMaxRadix - 1)) | l1], 1u);
+            for (int p = 2, at = w1; p < plan.passes; at += plan.width(p), ++p) {
+                const int c = kMaxDigitBits - plan.width(p);
+                atomicAdd(&h[p][(((key >> at) << c) & (kMaxRadix - 1)) |
+                                (lane_id() & ((1u << c) - 1u))],
+                          1u);
+            }
+        }
+    }
+    __device__ __forceinline__ void flush(unsigned* __restrict__ hist) {
+        for (int p = 0; p < plan.passes; ++p) {
+            const int w = plan.width(p), c = kMaxDigitBits - w;
+            for (int d = threadIdx.x; d < 1 << w; d += blockDim.x) {
+                unsigned v = 0;
+                for (int k = 0; k < 1 << c; ++k)
+                    v += h[p][(d << c) | k];
+                if (v)
+                    atomicAdd(&hist[p * kMaxRadix + d], v);
+            }
+        }
+    }
+};
 
 constexpr unsigned kColSkip = 0xffffffffu; // column step of a Gaussian walked again
 
@@ -22,8 +76,7 @@ struct EmitView {
 // Writes the instances of the Gaussians order[r], r in [r_begin, r_end),
 // which are consecutive in depth order, so their instances fill one
 // contiguous output range starting at st.offset[r_begin]. The warp takes
-// them 32 at a time: their span records (span_of(slot), the preprocess's
-// walk) become a list of columns in `cols` (32 * kSpanCols entries of this
+// them 32 at a time: their span records (the preprocess's walk) become a list of columns in `cols` (32 * kSpanCols entries of this
 // warp's shared memory), each a run of instances with tile ids start,
 // start + step, ... (step 1 or the tile grid width), and the warp writes the
 // range 32 consecutive instances at a time, coalesced: a lane finds its
@@ -32,11 +85,11 @@ struct EmitView {
 // walked again by the whole warp afterwards (a column per lane). Keys are
 // view_of(slot).tile_base + tile id; count(key) sees every key written.
 // Called by whole warps with warp-uniform r_begin / r_end.
-template <int TW, int TH, typename SpanOf, typename ViewOf, typename Count>
+template <int TW, int TH, typename ViewOf, typename Count>
 __device__ __forceinline__ void emit_warp_range(int r_begin, int r_end,
                                                 const unsigned* __restrict__ order,
-                                                const GaussianState& st, SpanOf span_of,
-                                                ViewOf view_of, unsigned* __restrict__ keys,
+                                                const GaussianState& st, ViewOf view_of,
+                                                unsigned* __restrict__ keys,
                                                 unsigned* __restrict__ values,
                                                 unsigned capacity, uint4* cols, Count count) {
     const unsigned full = 0xffffffffu;
@@ -48,7 +101,7 @@ __device__ __forceinline__ void emit_warp_range(int r_begin, int r_end,
         if (r < r_end) {
             i = order[r];
             cnt = st.touched[i];
-            sp = span_of(i);
+            sp = __ldg(&st.rec[i].spans);
         }
         const unsigned incl = warp_incl_scan(cnt);
         const unsigned e = incl - cnt; // lane's first instance in the 32 Gaussians' range
@@ -133,7 +186,7 @@ __device__ __forceinline__ void emit_warp_range(int r_begin, int r_end,
             const EmitView gv = view_of(gi);
             TileWalk w;
             unsigned k0 = 0;
-            if (walk_setup<TW, TH>(st.mean2d[gi], st.conic[gi], gv.grid_x, gv.grid_y, w)) {
+            if (walk_setup<TW, TH>(st.rec[gi].xy, st.rec[gi].co, gv.grid_x, gv.grid_y, w)) {
                 for (int u0 = w.u_min; u0 < w.u_max && k0 < gcnt; u0 += 32) {
                     const int tu = u0 + int(lane);
                     int v_min = 0, v_max = 0;

@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(kRows48 ? kRowsBlock : kGBlock,
         g0 = gslot[0];
         g1 = gslot[1];
         g2 = gslot[2];
-        clamp_bits = __float_as_uint(st.rgb[i].w);
+        clamp_bits = __float_as_uint(st.rec[i].rgb.w);
         if constexpr (kGeo) {
             gplane = st.geo_grad[size_t(i) * kGeoGradSlots];
             gnorm = st.geo_grad[size_t(i) * kGeoGradSlots + 1];

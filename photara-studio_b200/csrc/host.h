@@ -3,10 +3,14 @@
 // device buffer.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
+#include <cudaTypedefs.h>
 
 #include <stdexcept>
 #include <string>
+
+#include "common.cuh"
 
 namespace gsb {
 namespace host {
@@ -84,6 +88,35 @@ struct DevBuf {
         bytes = 0;
     }
 };
+
+// The record array as a [rows][16] float32 tensor with a box of one row (the
+// shape tile::gather4 copies), encoded through the driver's
+// cuTensorMapEncodeTiled (reached through the runtime, so the library links
+// no driver stub). The driver checks the base (16-byte aligned) and the row
+// stride (64 bytes).
+inline void encode_record_map(CUtensorMap* map, SplatRec* rec, size_t rows) {
+    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+    if (!encode) {
+        cudaDriverEntryPointQueryResult q{};
+        ck(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled",
+                                            reinterpret_cast<void**>(&encode), 12000,
+                                            cudaEnableDefault, &q),
+           "driver entry point cuTensorMapEncodeTiled");
+        if (q != cudaDriverEntryPointSuccess || !encode)
+            throw std::runtime_error("gsplat_b200: cuTensorMapEncodeTiled is not available");
+    }
+    const cuuint64_t dims[2] = {16, cuuint64_t(rows)};
+    const cuuint64_t strides[1] = {sizeof(SplatRec)};
+    const cuuint32_t box[2] = {16, 1};
+    const cuuint32_t elem[2] = {1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, rec, dims, strides, box,
+                              elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS)
+        throw std::runtime_error("gsplat_b200: cuTensorMapEncodeTiled failed (" +
+                                 std::to_string(int(r)) + ")");
+}
 
 inline int msb_bits(unsigned v) {
     int b = 0;

@@ -157,8 +157,9 @@ void launch_emit_keys(cudaStream_t s, int visible, unsigned instances, const uns
                       int group_shift, const unsigned* order, const GaussianState& st,
                       int grid_x, int grid_y, unsigned* keys, unsigned* values,
                       unsigned capacity, int bits, unsigned* hist);
-void launch_tile_ranges(cudaStream_t s, int count, const unsigned* keys, uint2* ranges,
-                        int tiles);
+// count_ptr (may be NULL): the key count on the device, `count` then its bound.
+void launch_tile_ranges(cudaStream_t s, size_t count, const unsigned* count_ptr,
+                        const unsigned* keys, uint2* ranges, int tiles);
 void launch_compose_keys(cudaStream_t s, int count, const unsigned* tiles,
                          const unsigned* values, const unsigned* depth,
                          unsigned long long* out);
@@ -360,8 +361,7 @@ cudaError_t launch_pruning_scores(cudaStream_t s, int tiles, const uint2* ranges
                                   const unsigned* pix_last, const float* image, int gaussian_pop,
                                   float* scores);
 
-cudaError_t launch_set_colors(cudaStream_t s, int n, const float* colors, float4* rgb,
-                              SplatRec* rec);
+cudaError_t launch_set_colors(cudaStream_t s, int n, const float* colors, SplatRec* rec);
 
 size_t gaussian_backward_smem(bool fused_sh);
 void launch_gaussian_backward(cudaStream_t s, int n, const float* means, const float* log_scales,

@@ -68,59 +68,6 @@ __global__ void __launch_bounds__(kBlock) preprocess_kernel(
         counters[6] = unsigned(n);
 }
 
-// The radix sort's digit histograms of the keys a kernel writes, counted as
-// they are written (the digits of radix_plan over key bits [0, bits), up to 4
-// passes): the sort then skips its own read of the keys. Per-block shared
-// histograms, flushed with one global atomic per non-empty bin. A digit of w
-// bits has 2^(9 - w) counters per bin in neighbouring banks, taken by lane:
-// neighbouring instances mostly share their high tile digit, and 32 lanes on
-// one counter are served one by one (emit at 1M / 1080p 68 us on single
-// counters of 7 + 6 bits).
-struct DigitCounter {
-    unsigned (*h)[kMaxRadix];
-    RadixPlan plan;
-    int w0, c0, w1, c1; // widths and counter bits of the first two digits
-    unsigned l0, l1;    // the lane's counter among a bin's
-    __device__ __forceinline__ DigitCounter(unsigned (*hist)[kMaxRadix], int bits)
-        : h(hist), plan(radix_plan(bits)) {
-        w0 = plan.width(0);
-        c0 = kMaxDigitBits - w0;
-        l0 = lane_id() & ((1u << c0) - 1u);
-        w1 = plan.passes > 1 ? plan.width(1) : 0;
-        c1 = kMaxDigitBits - w1;
-        l1 = lane_id() & ((1u << c1) - 1u);
-    }
-    __device__ __forceinline__ void zero() {
-        for (int k = threadIdx.x; k < plan.passes * kMaxRadix; k += blockDim.x)
-            (&h[0][0])[k] = 0;
-    }
-    __device__ __forceinline__ void count(unsigned key) {
-        atomicAdd(&h[0][((key << c0) & (kMaxRadix - 1)) | l0], 1u);
-        if (plan.passes > 1) {
-            key >>= w0;
-            atomicAdd(&h[1][((key << c1) & (kMaxRadix - 1)) | l1], 1u);
-            for (int p = 2, at = w1; p < plan.passes; at += plan.width(p), ++p) {
-                const int c = kMaxDigitBits - plan.width(p);
-                atomicAdd(&h[p][(((key >> at) << c) & (kMaxRadix - 1)) |
-                                (lane_id() & ((1u << c) - 1u))],
-                          1u);
-            }
-        }
-    }
-    __device__ __forceinline__ void flush(unsigned* __restrict__ hist) {
-        for (int p = 0; p < plan.passes; ++p) {
-            const int w = plan.width(p), c = kMaxDigitBits - w;
-            for (int d = threadIdx.x; d < 1 << w; d += blockDim.x) {
-                unsigned v = 0;
-                for (int k = 0; k < 1 << c; ++k)
-                    v += h[p][(d << c) | k];
-                if (v)
-                    atomicAdd(&hist[p * kMaxRadix + d], v);
-            }
-        }
-    }
-};
-
 // Depth sort input, compacted: the visible Gaussians (touched > 0) in index
 // order, keyed by their depth bits rebased on the frame minimum, with their
 // indices as values; the sort then orders only them. The compaction is an
@@ -210,25 +157,28 @@ __global__ void __launch_bounds__(kEmitBlock) emit_keys_kernel(
     const int r_begin = g < group_count ? int(groups[g]) : visible;
     const int r_end = g + 1 < group_count ? int(groups[g + 1]) : visible;
     emit_warp_range<kTileW, kTileH>(
-        r_begin, r_end, order, st, [&](unsigned i) { return __ldg(&st.rec[i].spans); },
-        [&](unsigned) { return EmitView{grid_x, grid_y, 0u}; }, keys, values, capacity,
+        r_begin, r_end, order, st, [&](unsigned) { return EmitView{grid_x, grid_y, 0u}; }, keys, values, capacity,
         s_col[warp], [&](unsigned key) { dc.count(key); });
     __syncthreads();
     dc.flush(hist);
 }
 
 // Per-tile [start, end) from the sorted keys. ranges[] is zeroed beforehand.
+// count_ptr (may be NULL): the number of keys, at most `count`, on the device.
 __global__ void __launch_bounds__(kBlock) tile_ranges_kernel(
-    int count, const unsigned* __restrict__ keys, uint2* __restrict__ ranges, unsigned tiles) {
+    unsigned count, const unsigned* __restrict__ count_ptr, const unsigned* __restrict__ keys,
+    uint2* __restrict__ ranges, unsigned tiles) {
+    if (count_ptr)
+        count = min(count, *count_ptr);
     // Four consecutive keys per thread (one 16-byte load when whole) and the
     // key before them; a boundary between positions i-1 and i ends the range
     // of the key at i-1 and starts the range of the key at i.
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i0 = 4 * t;
-    if (i0 >= count)
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned i0 = 4 * t;
+    if (t >= (count + 3) / 4)
         return;
     unsigned k[4];
-    if (i0 + 4 <= count) {
+    if (count - i0 >= 4) {
         const uint4 v = reinterpret_cast<const uint4*>(keys)[t];
         k[0] = v.x;
         k[1] = v.y;
@@ -237,13 +187,13 @@ __global__ void __launch_bounds__(kBlock) tile_ranges_kernel(
     } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            k[j] = i0 + j < count ? keys[i0 + j] : 0u;
+            k[j] = j < int(count - i0) ? keys[i0 + j] : 0u;
     }
     unsigned prev = i0 > 0 ? keys[i0 - 1] : 0u;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const int i = i0 + j;
-        if (i >= count)
+        const unsigned i = i0 + j;
+        if (j >= int(min(count - i0, 4u)))
             break;
         const unsigned tile = k[j];
         if (i == 0) {
@@ -251,12 +201,12 @@ __global__ void __launch_bounds__(kBlock) tile_ranges_kernel(
                 ranges[tile].x = 0;
         } else if (tile != prev) {
             if (prev < tiles)
-                ranges[prev].y = unsigned(i);
+                ranges[prev].y = i;
             if (tile < tiles)
-                ranges[tile].x = unsigned(i);
+                ranges[tile].x = i;
         }
         if (i == count - 1 && tile < tiles)
-            ranges[tile].y = unsigned(count);
+            ranges[tile].y = count;
         prev = tile;
     }
 }
@@ -337,14 +287,14 @@ void launch_emit_keys(cudaStream_t s, int visible, unsigned instances, const uns
                                                    grid_y, keys, values, capacity, bits, hist);
 }
 
-void launch_tile_ranges(cudaStream_t s, int count, const unsigned* keys, uint2* ranges,
-                        int tiles) {
-    if (count <= 0)
+void launch_tile_ranges(cudaStream_t s, size_t count, const unsigned* count_ptr,
+                        const unsigned* keys, uint2* ranges, int tiles) {
+    if (count == 0)
         return;
     // keys must be 16-byte aligned (the sort's buffers are)
-    const int threads = (count + 3) / 4;
-    tile_ranges_kernel<<<(threads + kBlock - 1) / kBlock, kBlock, 0, s>>>(count, keys, ranges,
-                                                                          unsigned(tiles));
+    const size_t threads = (count + 3) / 4;
+    tile_ranges_kernel<<<unsigned((threads + kBlock - 1) / kBlock), kBlock, 0, s>>>(
+        unsigned(count), count_ptr, keys, ranges, unsigned(tiles));
 }
 
 } // namespace gsb

@@ -81,8 +81,6 @@ __device__ __forceinline__ PreResult preprocess_one(
                 } else {
                     rgb = make_float3(colors[3 * i], colors[3 * i + 1], colors[3 * i + 2]);
                 }
-                st.mean2d[slot] = m2;
-                st.conic[slot] = co;
                 if constexpr (kGeometry) {
                     float4 pl;
                     float3 nm;
@@ -90,7 +88,6 @@ __device__ __forceinline__ PreResult preprocess_one(
                     st.plane[slot] = pl;
                     st.normal[slot] = make_float4(nm.x, nm.y, nm.z, 0.f);
                 }
-                st.rgb[slot] = make_float4(rgb.x, rgb.y, rgb.z, __uint_as_float(clamp_bits));
                 depth_bits = __float_as_uint(norm3df(t.x, t.y, t.z));
                 st.depth[slot] = depth_bits;
                 radius_out = int(radius);
@@ -102,18 +99,13 @@ __device__ __forceinline__ PreResult preprocess_one(
                     static_cast<unsigned short>(fmaxf(0.f, fminf(65535.f, floorf(px + ex) + 1.f))),
                     static_cast<unsigned short>(fmaxf(0.f, fminf(65535.f, floorf(py - ey)))),
                     static_cast<unsigned short>(fmaxf(0.f, fminf(65535.f, floorf(py + ey) + 1.f))));
-                st.bounds[slot] = box;
-                if (st.rec) {
-                    SplatRec r;
-                    r.co = co;
-                    r.rgb = make_float4(rgb.x, rgb.y, rgb.z, __uint_as_float(clamp_bits));
-                    r.xy = m2;
-                    r.bounds = box;
-                    r.spans = spans;
-                    st.rec[slot] = r;
-                } else if (st.spans) {
-                    st.spans[slot] = spans;
-                }
+                SplatRec r;
+                r.co = co;
+                r.rgb = make_float4(rgb.x, rgb.y, rgb.z, __uint_as_float(clamp_bits));
+                r.xy = m2;
+                r.bounds = box;
+                r.spans = spans;
+                st.rec[slot] = r;
             }
         }
     }

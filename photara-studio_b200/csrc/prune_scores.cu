@@ -29,8 +29,7 @@ constexpr int kWarps = kThreads / 32;
 
 __global__ void __launch_bounds__(kThreads) pruning_scores_kernel(
     const uint2* __restrict__ ranges, const unsigned* __restrict__ order,
-    const float2* __restrict__ mean2d, const float4* __restrict__ conic,
-    const float4* __restrict__ rgb, const unsigned* __restrict__ pix_last,
+    const SplatRec* __restrict__ rec, const unsigned* __restrict__ pix_last,
     const float* __restrict__ image, int width, int height, int grid_x, float alpha_clip,
     int gaussian_pop, float* __restrict__ scores) {
     __shared__ float2 s_xy[kThreads];
@@ -75,9 +74,9 @@ __global__ void __launch_bounds__(kThreads) pruning_scores_kernel(
         if (tid < n) {
             const unsigned g = order[range.x + base + tid];
             s_id[tid] = g;
-            s_xy[tid] = mean2d[g];
-            s_co[tid] = conic[g];
-            s_rgb[tid] = rgb[g];
+            s_xy[tid] = rec[g].xy;
+            s_co[tid] = rec[g].co;
+            s_rgb[tid] = rec[g].rgb;
         }
         __syncthreads();
         // warp-uniform walk; lanes past their last entry contribute zero
@@ -145,7 +144,7 @@ cudaError_t launch_pruning_scores(cudaStream_t s, int tiles, const uint2* ranges
                                   float* scores) {
     if (tiles > 0)
         pruning_scores_kernel<<<tiles, kThreads, 0, s>>>(
-            ranges, order, st.mean2d, st.conic, st.rgb, pix_last, image, K.width, K.height,
+            ranges, order, st.rec, pix_last, image, K.width, K.height,
             K.grid_x, K.alpha_clip, gaussian_pop, scores);
     return cudaGetLastError();
 }

@@ -260,9 +260,9 @@ __device__ __forceinline__ int pair_blend(float2 a, float4 c, unsigned pos, floa
 // of `order`. kCount: also adds to *pairs the (Gaussian, pixel) pairs whose
 // alpha test runs on a pixel that has not ended, for the roofline figures.
 // sched (count may be NULL): receives the strip (index `strip`) with its
-// adjoint work.
+// adjoint work. False: the staging gave up (the strip was not written).
 template <int TW, int PX, bool kCount = false>
-__device__ __forceinline__ void composite_forward_strip(
+__device__ __forceinline__ bool composite_forward_strip(
     StripFeed& feed, int x0, int y0, uint2 range, const unsigned* __restrict__ order,
     const ViewTarget& o, float* __restrict__ visibility, const StripOrder& sched, unsigned strip,
     unsigned long long* __restrict__ pairs = nullptr) {
@@ -312,7 +312,7 @@ __device__ __forceinline__ void composite_forward_strip(
         if (!feed.wait(buf)) {
             if (left > 0)
                 feed.wait(buf ^ 1);
-            return;
+            return false;
         }
         const SplatRec* rec = feed.s.rec[buf];
         unsigned mask[NP], all;
@@ -444,6 +444,7 @@ __device__ __forceinline__ void composite_forward_strip(
             }
         }
     }
+    return true;
 }
 
 // ---------------------------------------------------------------- adjoint --
@@ -603,9 +604,9 @@ __device__ __forceinline__ int strip_slot10() {
 // Adjoint of the strip with origin (x0, y0): per-Gaussian gradients are added
 // to rows of kGradSlots float4 at `grad`. kCount: counts into *pairs the
 // (Gaussian, pixel) pairs evaluated (the pixel's last contributor lies at or
-// behind the Gaussian) and does nothing else.
+// behind the Gaussian) and does nothing else. False as the forward.
 template <int TW, int PX, bool kRefine, bool kDensify, bool kCount = false>
-__device__ __forceinline__ void composite_backward_strip(
+__device__ __forceinline__ bool composite_backward_strip(
     StripFeed& feed, int x0, int y0, uint2 range, const unsigned* __restrict__ order,
     const ViewGrads& o, float4* __restrict__ grad,
     unsigned long long* __restrict__ pairs = nullptr) {
@@ -647,7 +648,7 @@ __device__ __forceinline__ void composite_backward_strip(
     }
     const int total = int(min(__reduce_max_sync(full, wl), range.y - range.x));
     if (total == 0)
-        return;
+        return true;
     const int slot = kDensify ? strip_slot12() : strip_slot10();
     const float scale = slot_scale(slot);
     float* const row = reinterpret_cast<float*>(grad) + max(slot, 0);
@@ -664,7 +665,7 @@ __device__ __forceinline__ void composite_backward_strip(
         if (!feed.wait(buf)) {
             if (base > 0)
                 feed.wait(buf ^ 1);
-            return;
+            return false;
         }
         const SplatRec* rec = feed.s.rec[buf];
         unsigned mask[NP], all;
@@ -786,6 +787,7 @@ __device__ __forceinline__ void composite_backward_strip(
     }
     if constexpr (kCount)
         warp_count_add(evaluated, pairs);
+    return true;
 }
 
 } // namespace gsb
