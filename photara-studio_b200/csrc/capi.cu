@@ -40,6 +40,12 @@ using namespace gsb::host;
 constexpr int kAutoPx1Tiles = 600;
 constexpr int kAutoPx2Tiles = 1000;
 constexpr int kAutoPx4Tiles = 4800;
+// Up to this many tiles the adjoint walks the list segments in parallel, from
+// checkpoints of the forward. Forward + adjoint, us, without / with: 256 tiles
+// 157 / 100, 300 tiles 132 / 99, 690 tiles 150 / 133, 1,200 tiles 293 / 303,
+// 1,900 tiles 250 / 268 (enough strips to fill the GPU already).
+constexpr int kSegmentTiles = 800;
+constexpr int kSegmentLevels = 16;
 
 struct gs_context {
     int device = 0;
@@ -47,7 +53,7 @@ struct gs_context {
     std::string error;
     // workspace
     DevBuf gauss, grad, scan_status, counters, inst_keys, inst_vals, sort_hist, sort_status,
-        sort_counters, ranges, pixel, depth_sort, loss, probe, geo_grad, rec, emit_groups;
+        sort_counters, ranges, pixel, depth_sort, loss, probe, geo_grad, rec, emit_groups, segment;
     unsigned* host_counts = nullptr; // pinned [16]: [0, 8) draw counts, [8] error word after the sorts
     size_t gauss_cap = 0, grad_cap = 0, inst_cap = 0, pixel_cap = 0, geo_grad_cap = 0;
     GaussianState st{};
@@ -75,6 +81,7 @@ struct gs_context {
     float* pix_dtdt = nullptr; // dT/dt at the median depth (geometry training forwards)
     unsigned* work_lists = nullptr; // the last colour training forward's strips by adjoint work
     int work_px = 0;                // its pixels per thread (the strips' shape)
+    SegmentStore segments{};        // its checkpoints (levels 0: none kept)
     bool geometry = false;     // the last forward rendered the median-depth / normal channels
     const float* fwd_depth = nullptr;  // its median-depth and normal outputs (caller memory)
     const float* fwd_normal = nullptr;
@@ -134,6 +141,11 @@ int compositing_px(const gs_context* c, int tiles) {
     if (c->pixels_per_thread > 0)
         return c->pixels_per_thread;
     return tiles <= kAutoPx1Tiles ? 1 : tiles <= kAutoPx2Tiles ? 2 : tiles <= kAutoPx4Tiles ? 4 : 8;
+}
+
+// Checkpoint levels of a training forward on the automatic schedule.
+int segment_levels(const gs_context* c, int tiles) {
+    return c->pixels_per_thread > 0 || tiles > kSegmentTiles ? 0 : kSegmentLevels;
 }
 
 void mark(gs_context* c, int stage, bool end) {
@@ -304,7 +316,7 @@ void gs_destroy(gs_context* c) {
     for (DevBuf* b : {&c->gauss, &c->grad, &c->scan_status, &c->counters, &c->inst_keys,
                       &c->inst_vals, &c->sort_hist, &c->sort_status, &c->sort_counters,
                       &c->ranges, &c->pixel, &c->depth_sort, &c->loss, &c->probe,
-                      &c->geo_grad, &c->rec, &c->emit_groups})
+                      &c->geo_grad, &c->rec, &c->emit_groups, &c->segment})
         b->release();
     if (c->host_counts)
         cudaFreeHost(c->host_counts);
@@ -332,7 +344,7 @@ size_t gs_workspace_bytes(const gs_context* c) {
     for (const DevBuf* b : {&c->gauss, &c->grad, &c->scan_status, &c->counters, &c->inst_keys,
                             &c->inst_vals, &c->sort_hist, &c->sort_status, &c->sort_counters,
                             &c->ranges, &c->pixel, &c->depth_sort, &c->loss, &c->probe,
-                            &c->geo_grad, &c->rec, &c->emit_groups})
+                            &c->geo_grad, &c->rec, &c->emit_groups, &c->segment})
         t += b->bytes;
     return t;
 }
@@ -416,11 +428,13 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
         const int ppt = compositing_px(c, tiles);
         // the strips by adjoint work, listed by the compositing; only the
         // class counts at its start are zeroed
+        const size_t o_last = carve(size_t(tiles) * sizeof(unsigned)); // SegmentStore::tile_last
         const size_t o_work = carve(kWorkListZeroed * sizeof(unsigned));
         const size_t zeroed = frame;
         frame = o_work + align_up(strip_order_words(tiles, ppt) * sizeof(unsigned));
         char* fb = c->ranges.ensure(frame, st);
         c->work_lists = nullptr; // set below by a colour training forward
+        c->segments = SegmentStore{};
         unsigned* fctr = reinterpret_cast<unsigned*>(fb + o_ctr); // [0] compaction [1] scan
                                                                   // [2..6) depth sort passes
         unsigned* hist = reinterpret_cast<unsigned*>(fb + o_hist_d);
@@ -517,11 +531,16 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
             if (train) {
                 c->work_lists = reinterpret_cast<unsigned*>(fb + o_work);
                 c->work_px = ppt;
+                const int levels = segment_levels(c, tiles);
+                if (levels > 0)
+                    c->segments = {reinterpret_cast<float4*>(c->segment.ensure(
+                                       size_t(levels) * P * sizeof(float4), st)),
+                                   reinterpret_cast<unsigned*>(fb + o_last), levels};
             }
             launch_composite_forward(st, tiles, reinterpret_cast<const uint2*>(c->ranges.p),
                                      c->vals[cur], K, bg, out->color, out->alpha, c->pix_T,
                                      c->pix_last, out->visibility, ppt, record_staging(c),
-                                     c->work_lists);
+                                     c->work_lists, &c->segments);
         }
         ck(cudaGetLastError(), "composite launch");
         mark(c, 5, true);
@@ -608,7 +627,7 @@ gs_status gs_backward(gs_context* c, const float* fwd_alpha, const int* fwd_radi
                                       c->pix_last, dL->color, dL->alpha, dL->densify_map,
                                       grads && grads->refine_weight ? 1 : 0,
                                       c->work_lists ? c->work_px : compositing_px(c, c->tiles),
-                                      record_staging(c), c->work_lists);
+                                      record_staging(c), c->work_lists, &c->segments);
         ck(cudaGetLastError(), "composite backward launch");
         mark(c, 6, true);
         mark(c, 7, false);
@@ -879,11 +898,13 @@ gs_status gs_forward_colors(gs_context* c, const float* colors, const gs_outputs
         const int n = c->g.count;
         ck(launch_set_colors(c->stream, n, colors, c->st.rec), "colour slots");
         c->g.colors = colors;
-        // empty tiles (ranges zeroed by the forward) composite the background
+        // empty tiles (ranges zeroed by the forward) composite the background;
+        // the checkpoints' colours are written again
         launch_composite_forward(c->stream, c->tiles, reinterpret_cast<const uint2*>(c->ranges.p),
                                  c->vals[c->sorted_buf], c->K, c->bg, out->color, out->alpha,
                                  c->pix_T, c->pix_last, out->visibility,
-                                 compositing_px(c, c->tiles), record_staging(c));
+                                 c->work_lists ? c->work_px : compositing_px(c, c->tiles),
+                                 record_staging(c), nullptr, &c->segments);
         ck(cudaGetLastError(), "colour reuse composite launch");
     });
 }

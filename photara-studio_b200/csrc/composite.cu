@@ -2,6 +2,8 @@
 // tile running the forward / adjoint of strip.cuh (numerics and organisation
 // described there; reference: third_party/splat_drender/src/render_forward.cu
 // :341-416, :508-525 and render_backward.cu:156-519).
+#include <algorithm>
+
 #include "kernels.h"
 #include "strip.cuh"
 
@@ -13,24 +15,25 @@ template <int PX> constexpr int kForwardCtas = PX == 8 ? 20 : PX == 4 ? 28 : 32;
 template <int PX> constexpr int kBackwardCtas = PX == 8 ? 16 : PX == 4 ? 20 : 24;
 
 // One warp per strip of a reference 16x16 tile (256 / (32 PX) strips per
-// tile). kCount: the same forward that also counts its evaluated pairs.
-template <int PX, bool kCount = false>
+// tile). kCount: the same forward that also counts its evaluated pairs. kSeg:
+// it stores the adjoint's checkpoints.
+template <int PX, bool kCount = false, bool kSeg = false>
 __global__ void __launch_bounds__(32, kForwardCtas<PX>) composite_forward_kernel(
     const __grid_constant__ CUtensorMap map, unsigned* __restrict__ err,
     const uint2* __restrict__ ranges, const unsigned* __restrict__ order, const Camera K,
     float3 bg, float* __restrict__ out_color, float* __restrict__ out_alpha,
     float* __restrict__ pix_T, unsigned* __restrict__ pix_last, float* __restrict__ visibility,
-    StripOrder sched, unsigned long long* __restrict__ pairs = nullptr) {
+    StripOrder sched, Checkpoints cp, unsigned long long* __restrict__ pairs = nullptr) {
     constexpr int kStrips = kTileH / StripGeom<kTileW, PX>::kRows;
     __shared__ StripStage s;
     StripFeed feed{s, &map, err};
     feed.init();
     const int tile = int(blockIdx.x) / kStrips, strip = int(blockIdx.x) % kStrips;
     const ViewTarget o{K.width, K.height, K.alpha_clip, bg, out_color, out_alpha, pix_T, pix_last};
-    composite_forward_strip<kTileW, PX, kCount>(
+    composite_forward_strip<kTileW, PX, kCount, kSeg>(
         feed, (tile % K.grid_x) * kTileW,
         (tile / K.grid_x) * kTileH + strip * StripGeom<kTileW, PX>::kRows, ranges[tile], order, o,
-        visibility, sched, blockIdx.x, pairs);
+        visibility, sched, blockIdx.x, pairs, &cp, tile);
 }
 
 template <int PX, bool kRefine, bool kDensify, bool kCount = false>
@@ -56,6 +59,41 @@ __global__ void __launch_bounds__(32, kBackwardCtas<PX>) composite_backward_kern
         feed, (tile % K.grid_x) * kTileW,
         (tile / K.grid_x) * kTileH + strip * StripGeom<kTileW, PX>::kRows, ranges[tile], order, o,
         grad, pairs);
+}
+
+// The adjoint from the forward's checkpoints: one-warp CTAs take the (segment,
+// strip) items of the frame in turn, segments in front first. Four pixels per
+// thread whatever the forward took, since segments already give enough warps
+// (256 tiles: 52 us, at eight 78 us; the whole-list adjoint 114 us at its best).
+constexpr int kSegmentPx = 4;
+
+template <bool kRefine, bool kDensify>
+__global__ void __launch_bounds__(32, kBackwardCtas<kSegmentPx>) composite_backward_segment_kernel(
+    const __grid_constant__ CUtensorMap map, unsigned* __restrict__ err, unsigned tiles,
+    const uint2* __restrict__ ranges, const unsigned* __restrict__ order, float4* __restrict__ grad,
+    const Camera K, float3 bg, const float* __restrict__ pix_T,
+    const unsigned* __restrict__ pix_last, const float* __restrict__ dL_color,
+    const float* __restrict__ dL_alpha, const float* __restrict__ densify_map, Checkpoints cp) {
+    constexpr int PX = kSegmentPx;
+    constexpr unsigned kStrips = kTileH / StripGeom<kTileW, PX>::kRows;
+    __shared__ StripStage s;
+    StripFeed feed{s, &map, err};
+    feed.init();
+    const unsigned strips = tiles * kStrips;
+    const ViewGrads o{K.width, K.height, K.alpha_clip, bg, pix_T, pix_last, dL_color, dL_alpha,
+                      densify_map};
+    for (unsigned item = blockIdx.x; item < strips * unsigned(cp.levels); item += gridDim.x) {
+        const unsigned level = item / strips, at = item % strips;
+        const int tile = int(at / kStrips), strip = int(at % kStrips);
+        if (cp.tile_last[tile] <= level * kSegment)
+            continue;
+        if (!composite_backward_strip<kTileW, PX, kRefine, kDensify, false, true>(
+                feed, (tile % K.grid_x) * kTileW,
+                (tile / K.grid_x) * kTileH + strip * StripGeom<kTileW, PX>::kRows, ranges[tile],
+                order, o, grad, nullptr, &cp, int(level)))
+            break;
+        __syncwarp();
+    }
 }
 
 size_t strip_order_words(int tiles, int pixels_per_thread) {
@@ -102,7 +140,7 @@ void launch_composite_count_pairs(cudaStream_t s, int tiles, const uint2* ranges
     auto count = [&]<int PX>() {
         const int blocks = tiles * (8 / PX);
         composite_forward_kernel<PX, true><<<blocks, 32, 0, s>>>(
-            rs.map, rs.err, ranges, order, K, bg, color, alpha, nullptr, nullptr, nullptr, {},
+            rs.map, rs.err, ranges, order, K, bg, color, alpha, nullptr, nullptr, nullptr, {}, {},
             pairs);
         composite_backward_kernel<PX, false, false, true><<<blocks, 32, 0, s>>>(
             rs.map, rs.err, ranges, order, st.grad, K, bg, pix_T, pix_last, color, nullptr,
@@ -712,12 +750,22 @@ void launch_composite_backward_geometry(cudaStream_t s, int tiles, const uint2* 
 void launch_composite_forward(cudaStream_t s, int tiles, const uint2* ranges,
                               const unsigned* order, const Camera& K, float3 bg, float* color,
                               float* alpha, float* pix_T, unsigned* pix_last, float* visibility,
-                              int pixels_per_thread, const RecStaging& rs, unsigned* work_lists) {
-    const StripOrder sched = strip_order(work_lists, tiles, pixels_per_thread);
+                              int pixels_per_thread, const RecStaging& rs, unsigned* work_lists,
+                              const SegmentStore* segments) {
+    const bool seg = segments && segments->levels > 0;
+    const StripOrder sched = strip_order(seg ? nullptr : work_lists, tiles, pixels_per_thread);
+    const Checkpoints cp = seg ? Checkpoints{segments->data, segments->tile_last, segments->levels}
+                               : Checkpoints{};
     auto fwd = [&]<int PX>() {
-        composite_forward_kernel<PX><<<tiles * (8 / PX), 32, 0, s>>>(
-            rs.map, rs.err, ranges, order, K, bg, color, alpha, pix_T, pix_last, visibility,
-            sched);
+        auto go = [&](auto kernel) {
+            kernel<<<tiles * (8 / PX), 32, 0, s>>>(rs.map, rs.err, ranges, order, K, bg, color,
+                                                   alpha, pix_T, pix_last, visibility, sched, cp,
+                                                   nullptr);
+        };
+        if constexpr (PX <= 2)
+            if (seg)
+                return go(composite_forward_kernel<PX, false, true>);
+        go(composite_forward_kernel<PX, false, false>);
     };
     if (pixels_per_thread == 1)
         fwd.template operator()<1>();
@@ -734,7 +782,28 @@ void launch_composite_backward(cudaStream_t s, int tiles, const uint2* ranges,
                                float3 bg, const float* pix_T, const unsigned* pix_last,
                                const float* dL_color, const float* dL_alpha,
                                const float* densify_map, int want_refine, int pixels_per_thread,
-                               const RecStaging& rs, unsigned* work_lists) {
+                               const RecStaging& rs, unsigned* work_lists,
+                               const SegmentStore* segments) {
+    if (segments && segments->levels > 0) {
+        const Checkpoints cp{segments->data, segments->tile_last, segments->levels};
+        constexpr int PX = kSegmentPx;
+        const unsigned items = unsigned(tiles) * (8 / PX) * unsigned(cp.levels);
+        const unsigned blocks = std::min(items, 148u * kBackwardCtas<PX>);
+        auto go = [&](auto kernel) {
+            kernel<<<blocks, 32, 0, s>>>(rs.map, rs.err, unsigned(tiles), ranges, order, st.grad,
+                                         K, bg, pix_T, pix_last, dL_color, dL_alpha, densify_map,
+                                         cp);
+        };
+        if (want_refine && densify_map)
+            go(composite_backward_segment_kernel<true, true>);
+        else if (want_refine)
+            go(composite_backward_segment_kernel<true, false>);
+        else if (densify_map)
+            go(composite_backward_segment_kernel<false, true>);
+        else
+            go(composite_backward_segment_kernel<false, false>);
+        return;
+    }
     const StripOrder sched = strip_order(work_lists, tiles, pixels_per_thread);
     auto bwd = [&]<int PX>() {
         auto go = [&](auto kernel) {

@@ -232,13 +232,22 @@ void launch_stage_probe(cudaStream_t s, unsigned limit, unsigned* err);
 // strip_order_words() words that receive the strips by adjoint work, the first
 // kWorkListZeroed of them zeroed before the call; launch_composite_backward
 // takes them with the same pixels_per_thread.
+// segments (may be NULL; one or two pixels per thread): the forward stores
+// checkpoints there instead and the adjoint walks the list segments in
+// parallel (strip.cuh).
+struct SegmentStore {
+    float4* data = nullptr;        // [levels][pixels]
+    unsigned* tile_last = nullptr; // [tiles], zeroed before the forward
+    int levels = 0;                // 0: not used
+};
 constexpr int kWorkListZeroed = 64;
 size_t strip_order_words(int tiles, int pixels_per_thread);
 void launch_composite_forward(cudaStream_t s, int tiles, const uint2* ranges,
                               const unsigned* order, const Camera& K, float3 bg, float* color,
                               float* alpha, float* pix_T, unsigned* pix_last, float* visibility,
                               int pixels_per_thread, const RecStaging& rs,
-                              unsigned* work_lists = nullptr);
+                              unsigned* work_lists = nullptr,
+                              const SegmentStore* segments = nullptr);
 // Fused L1 + SSIM loss: grad += dL/dpred, *loss_out (may be NULL) = L;
 // Training-loss terms of one view (image_loss.cu); field meanings as the
 // C ABI's gs_loss_images / gs_loss_options / gs_loss_outputs.
@@ -354,7 +363,8 @@ void launch_composite_backward(cudaStream_t s, int tiles, const uint2* ranges,
                                const float* dL_color, const float* dL_alpha,
                                const float* densify_map, int want_refine,
                                int pixels_per_thread, const RecStaging& rs,
-                               unsigned* work_lists = nullptr);
+                               unsigned* work_lists = nullptr,
+                               const SegmentStore* segments = nullptr);
 
 cudaError_t launch_pruning_scores(cudaStream_t s, int tiles, const uint2* ranges,
                                   const unsigned* order, const GaussianState& st, const Camera& K,

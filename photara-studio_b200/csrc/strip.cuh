@@ -211,6 +211,22 @@ __device__ __forceinline__ unsigned strip_order_get(const StripOrder& o, unsigne
     return o.list[size_t(cls) * o.strips + at];
 }
 
+// Checkpoints of a training forward, for frames with so few tiles that the
+// adjoint's time is the longest strip's serial walk: the list positions are cut
+// into segments of kSegment (the last level takes the rest), and at the end of
+// each one the forward stores, per pixel, the colour blended inside it and the
+// transmittance left. The adjoint then walks every segment of a strip in its own
+// warp: it starts from the stored transmittance, and the colour behind is the
+// sum over the later segments (no differences of large sums are taken).
+constexpr int kSegment = 64;
+static_assert(kSegment % kStripBatch == 0, "segments end with a batch");
+
+struct Checkpoints {
+    float4* data = nullptr;      // [levels][H * W] colour in the segment, T at its end
+    unsigned* tile_last = nullptr; // [tiles], zero before the forward: largest pix_last
+    int levels = 0;
+};
+
 // ---------------------------------------------------------------- forward --
 // A Gaussian's exponent at a vertical pixel pair, in gaussian_power's rounding
 // (element by element on f32x2 instructions).
@@ -240,8 +256,15 @@ __device__ __forceinline__ float2 pair_alpha(float4 co, float dx, float xx, floa
 // Selects on values instead of flags kept across the pairs: eight pixels'
 // flags exceed the predicate registers and were moved through general ones
 // (179 ALU instructions per visit of a whole tile).
+// kSeg: also adds the blend to the segment's colour sums.
+struct SegSums {
+    float2 r, g, b;
+};
+
+template <bool kSeg>
 __device__ __forceinline__ int pair_blend(float2 a, float4 c, unsigned pos, float2& T, float2& r,
-                                          float2& g, float2& b, unsigned& la, unsigned& lb) {
+                                          float2& g, float2& b, unsigned& la, unsigned& lb,
+                                          SegSums& seg) {
     const float2 tt = __fmul2_rn(T, __ffma2_rn(a, f2s(-1.f), f2s(1.f)));
     const bool ba = !(tt.x < kTransmittanceFloor);
     const bool bb = !(tt.y < kTransmittanceFloor);
@@ -249,6 +272,11 @@ __device__ __forceinline__ int pair_blend(float2 a, float4 c, unsigned pos, floa
     r = __ffma2_rn(f2s(c.x), w, r);
     g = __ffma2_rn(f2s(c.y), w, g);
     b = __ffma2_rn(f2s(c.z), w, b);
+    if constexpr (kSeg) {
+        seg.r = __ffma2_rn(f2s(c.x), w, seg.r);
+        seg.g = __ffma2_rn(f2s(c.y), w, seg.g);
+        seg.b = __ffma2_rn(f2s(c.z), w, seg.b);
+    }
     T.x = ba ? tt.x : -fabsf(T.x);
     T.y = bb ? tt.y : -fabsf(T.y);
     la = ba ? pos : la;
@@ -261,11 +289,13 @@ __device__ __forceinline__ int pair_blend(float2 a, float4 c, unsigned pos, floa
 // alpha test runs on a pixel that has not ended, for the roofline figures.
 // sched (count may be NULL): receives the strip (index `strip`) with its
 // adjoint work. False: the staging gave up (the strip was not written).
-template <int TW, int PX, bool kCount = false>
+// kSeg: stores the checkpoints and adds the strip to tile_last[tile].
+template <int TW, int PX, bool kCount = false, bool kSeg = false>
 __device__ __forceinline__ bool composite_forward_strip(
     StripFeed& feed, int x0, int y0, uint2 range, const unsigned* __restrict__ order,
     const ViewTarget& o, float* __restrict__ visibility, const StripOrder& sched, unsigned strip,
-    unsigned long long* __restrict__ pairs = nullptr) {
+    unsigned long long* __restrict__ pairs = nullptr, const Checkpoints* cp = nullptr,
+    int tile = 0) {
     using G = StripGeom<TW, PX>;
     constexpr int NP = G::kBands;
     constexpr unsigned full = 0xffffffffu;
@@ -296,6 +326,27 @@ __device__ __forceinline__ bool composite_forward_strip(
         return s < 0;
     };
     unsigned long long evaluated = 0;
+    SegSums seg[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+        seg[p].r = seg[p].g = seg[p].b = f2s(0.f);
+    // Stores segment `level`'s sums and the transmittance, and starts the next.
+    auto checkpoint = [&](int level) {
+        float4* dst = cp->data + size_t(level) * o.width * o.height;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+#pragma unroll
+            for (int q = 0; q < (PX > 1 ? 2 : 1); ++q) {
+                const int y = py + p * G::kBandRows + q;
+                if (px < o.width && y < o.height)
+                    dst[size_t(y) * o.width + px] =
+                        make_float4(q ? seg[p].r.y : seg[p].r.x, q ? seg[p].g.y : seg[p].g.x,
+                                    q ? seg[p].b.y : seg[p].b.x, fabsf(q ? T[p].y : T[p].x));
+            }
+            seg[p].r = seg[p].g = seg[p].b = f2s(0.f);
+        }
+    };
+    int level = 0;
 
     bool more = n > 0 && !__all_sync(full, ended());
     unsigned id_next = 0;
@@ -354,6 +405,11 @@ __device__ __forceinline__ bool composite_forward_strip(
                     r[0].x += c.x * w;
                     g[0].x += c.y * w;
                     b[0].x += c.z * w;
+                    if constexpr (kSeg) {
+                        seg[0].r.x += c.x * w;
+                        seg[0].g.x += c.y * w;
+                        seg[0].b.x += c.z * w;
+                    }
                     T[0].x = bl ? tt : -fabsf(T[0].x);
                     la[0] = bl ? unsigned(base + j[u] + 1) : la[0];
                     seen |= w > 0.f ? 1u << j[u] : 0u;
@@ -387,14 +443,15 @@ __device__ __forceinline__ bool composite_forward_strip(
                         e[p] = pair_alpha(co, dx, xx, nxy, __fadd2_rn(f2s(xy.y), nfy[p]), clip);
 #pragma unroll
                     for (int p = 0; p < NP; ++p)
-                        bl |= pair_blend(e[p], c, pos, T[p], r[p], g[p], b[p], la[p], lb[p]);
+                        bl |= pair_blend<kSeg>(e[p], c, pos, T[p], r[p], g[p], b[p], la[p], lb[p],
+                                               seg[p]);
                 } else {
 #pragma unroll
                     for (int p = 0; p < NP; ++p)
                         if ((mask[p] >> j) & 1u)
-                            bl |= pair_blend(
+                            bl |= pair_blend<kSeg>(
                                 pair_alpha(co, dx, xx, nxy, __fadd2_rn(f2s(xy.y), nfy[p]), clip),
-                                c, pos, T[p], r[p], g[p], b[p], la[p], lb[p]);
+                                c, pos, T[p], r[p], g[p], b[p], la[p], lb[p], seg[p]);
                 }
                 seen |= (bl << 1) != 0 ? 1u << j : 0u;
                 if ((++visit & 3) == 0 && __all_sync(full, ended()))
@@ -411,10 +468,25 @@ __device__ __forceinline__ bool composite_forward_strip(
             feed.wait(buf ^ 1); // the copy in flight lands before the CTA leaves
             more = false;
         }
+        if constexpr (kSeg) {
+            if (!more)
+                checkpoint(level);
+            else if ((base + kStripBatch) % kSegment == 0 && level + 1 < cp->levels)
+                checkpoint(level++);
+        }
         buf ^= 1;
     }
     if constexpr (kCount)
         warp_count_add(evaluated, pairs);
+    if constexpr (kSeg) {
+        unsigned wl = 0;
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+            wl = max(wl, max(la[p], lb[p]));
+        wl = __reduce_max_sync(full, wl);
+        if (lane == 0 && wl)
+            atomicMax(cp->tile_last + tile, wl);
+    }
     if (sched.count) {
         unsigned wl = 0;
 #pragma unroll
@@ -604,12 +676,14 @@ __device__ __forceinline__ int strip_slot10() {
 // Adjoint of the strip with origin (x0, y0): per-Gaussian gradients are added
 // to rows of kGradSlots float4 at `grad`. kCount: counts into *pairs the
 // (Gaussian, pixel) pairs evaluated (the pixel's last contributor lies at or
-// behind the Gaussian) and does nothing else. False as the forward.
-template <int TW, int PX, bool kRefine, bool kDensify, bool kCount = false>
+// behind the Gaussian) and does nothing else. kSeg: only segment `level` of
+// the list, from the forward's checkpoints. False as the forward.
+template <int TW, int PX, bool kRefine, bool kDensify, bool kCount = false, bool kSeg = false>
 __device__ __forceinline__ bool composite_backward_strip(
     StripFeed& feed, int x0, int y0, uint2 range, const unsigned* __restrict__ order,
     const ViewGrads& o, float4* __restrict__ grad,
-    unsigned long long* __restrict__ pairs = nullptr) {
+    unsigned long long* __restrict__ pairs = nullptr, const Checkpoints* cp = nullptr,
+    int level = 0) {
     using G = StripGeom<TW, PX>;
     constexpr int NP = G::kBands;
     constexpr unsigned full = 0xffffffffu;
@@ -646,9 +720,38 @@ __device__ __forceinline__ bool composite_backward_strip(
         nfy[p] = f2(-float(y), -float(y + 1));
         wl = max(wl, max(a.last, c.last));
     }
-    const int total = int(min(__reduce_max_sync(full, wl), range.y - range.x));
-    if (total == 0)
+    int total = int(min(__reduce_max_sync(full, wl), range.y - range.x));
+    const int start = kSeg ? level * kSegment : 0; // first list position walked
+    if (total <= start)
         return true;
+    if constexpr (kSeg) {
+        if (level + 1 < cp->levels) {
+            const unsigned end = unsigned(start + kSegment);
+            total = min(total, int(end));
+            // a pixel blended past the segment starts from its checkpoint; the
+            // colour behind it is that of the later segments
+            auto resume = [&](int y, unsigned last, float& T, float& sdot, float gx, float gy,
+                              float gz) {
+                if (last <= end)
+                    return;
+                const float4* c = cp->data + size_t(level) * P + size_t(y) * o.width + px;
+                T = c->w;
+                for (unsigned l = unsigned(level) + 1;
+                     l < unsigned(cp->levels) && l * kSegment < last; ++l) {
+                    c += P;
+                    sdot += c->x * gx + c->y * gy + c->z * gz;
+                }
+            };
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                const int y = py + p * G::kBandRows;
+                resume(y, st[p].la, st[p].T.x, st[p].sdot.x, st[p].gx.x, st[p].gy.x, st[p].gz.x);
+                if constexpr (PX > 1)
+                    resume(y + 1, st[p].lb, st[p].T.y, st[p].sdot.y, st[p].gx.y, st[p].gy.y,
+                           st[p].gz.y);
+            }
+        }
+    }
     const int slot = kDensify ? strip_slot12() : strip_slot10();
     const float scale = slot_scale(slot);
     float* const row = reinterpret_cast<float*>(grad) + max(slot, 0);
@@ -656,14 +759,14 @@ __device__ __forceinline__ bool composite_backward_strip(
     int base = (total - 1) / kStripBatch * kStripBatch;
     unsigned id_next = feed.issue(0, order, range.x + unsigned(base), total - base);
     int buf = 0;
-    for (; base >= 0; base -= kStripBatch) {
+    for (; base >= start; base -= kStripBatch) {
         const int cnt = min(kStripBatch, total - base);
         const unsigned id = id_next;
-        if (base > 0)
+        if (base > start)
             id_next = feed.issue(buf ^ 1, order, range.x + unsigned(base - kStripBatch),
                                  kStripBatch);
         if (!feed.wait(buf)) {
-            if (base > 0)
+            if (base > start)
                 feed.wait(buf ^ 1);
             return false;
         }

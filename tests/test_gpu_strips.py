@@ -24,10 +24,12 @@ def rel_l2(a, b):
     return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30))
 
 
-@pytest.mark.parametrize("ppt", [1, 2, 4, 8])
+@pytest.mark.parametrize("ppt", [1, 2, 4, 8, None])
 @pytest.mark.parametrize("w,h,n", [(5, 3, 1), (16, 16, 33), (17, 31, 300), (33, 18, 5),
                                    (47, 65, 700)])
 def test_uneven_strips_match_oracle(ppt, w, h, n):
+    """ppt None: the automatic schedule, whose adjoint of so few tiles walks
+    the list segments in parallel."""
     scene = dataclasses.replace(gsb.make_scene("tiny", seed=n + w, count=n), width=w, height=h,
                                 cx=w / 2.0, cy=h / 2.0, fx=40.0, fy=40.0)
     model, cam = device_model(scene), camera_of(scene)
@@ -54,3 +56,43 @@ def test_uneven_strips_match_oracle(ppt, w, h, n):
     assert torch.equal(weighted.densify_weight, weighted.densify_weight_den)
     assert abs(float(weighted.densify_weight_den.sum()) - float(r.alpha.sum())) <= \
         1e-4 * max(float(r.alpha.sum()), 1.0)
+
+
+@pytest.mark.parametrize("count,logit", [(64, 0.0), (65, -3.0), (1024, -5.0), (1500, -5.2)])
+def test_long_lists_in_segments_match_whole_lists(count, logit):
+    """Every Gaussian over the whole of a small image, lists of one segment to
+    more than the sixteen checkpoint levels hold: the segment-parallel adjoint
+    against the whole-list one and, for one more colour set, after
+    forward_colors. Tolerance (relative L2): the whole-list walk recovers the
+    transmittance by one rounded multiplication per entry (an ulp, 2^-23, each),
+    the segments restart it from the forward's, so the two may part by
+    count * 2^-23 of a term; 1e-5 for the other sums, 1e-4 for the opacities,
+    whose terms cancel."""
+    drift = count * 2.0 ** -23
+    scene = dataclasses.replace(gsb.make_scene("tiny", seed=count, count=count), width=20,
+                                height=18, cx=10.0, cy=9.0, fx=20.0, fy=20.0)
+    model, cam = device_model(scene), camera_of(scene)
+    model.means = (model.means * torch.tensor([0.1, 0.1, 1.0], device="cuda")).contiguous()
+    # unequal axes: an isotropic Gaussian's quaternion gradient is zero, and the
+    # relative difference of two roundings of zero has no bound
+    model.log_scales = (1.0 + 0.5 * (model.log_scales + 3.5)).contiguous()
+    model.opacity_logits = torch.full_like(model.opacity_logits, logit)
+    g = torch.Generator("cuda").manual_seed(count)
+    colors = [torch.rand((count, 3), device="cuda", generator=g) for _ in range(2)]
+    gc = torch.randn((3, 18, 20), device="cuda", generator=g)
+    ga = torch.randn((18, 20), device="cuda", generator=g)
+    out = []
+    for ppt in (1, None):
+        rast = gsb.Rasterizer(pixels_per_thread=ppt)
+        r = rast.forward(model, cam, gsb.RasterizeOptions(colors_precomp=colors[0],
+                                                          background=(0.1, 0.2, 0.3)))
+        first = rast.backward(model, r, gc, ga)
+        again = rast.forward_colors(r, colors[1])
+        second = rast.backward(model, again, gc, ga)
+        out.append((r.color, again.color, first, second))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    for a, b in zip(out[0][2:], out[1][2:]):
+        for name in ("means", "log_scales", "quaternions", "opacity_logits", "colors_precomp",
+                     "refine_weight"):
+            x, y = getattr(a, name).cpu().numpy(), getattr(b, name).cpu().numpy()
+            assert rel_l2(y, x) <= drift + (1e-4 if name == "opacity_logits" else 1e-5), name
