@@ -91,19 +91,24 @@ __global__ void __launch_bounds__(kBlock) batch_preprocess_kernel(
         s_vis = 0;
     }
     __syncthreads();
+    __shared__ uint4 s_rec[kBlock][4];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned touched = 0;
+    SplatRec rec;
     if (i < n) {
         const size_t slot = size_t(v) * size_t(n) + size_t(i);
         const PreResult r = preprocess_one<TW, TH>(i, slot, means, log_scales, quats, logits,
                                                    filter_3d, sh, colors, sh_degree, sh_bases, sK,
-                                                   st);
+                                                   st, rec);
         touched = r.touched;
         st.touched[slot] = r.touched;
         radii[slot] = r.radius;
         dkeys[slot] = r.touched > 0 ? r.depth_bits : 0xffffffffu;
         dvals[slot] = unsigned(slot);
     }
+    const int warp0 = int(threadIdx.x) & ~31;
+    store_records(s_rec + warp0, touched > 0, rec,
+                  st.rec + size_t(v) * size_t(n) + blockIdx.x * blockDim.x + warp0);
     const unsigned w_inst = __reduce_add_sync(0xffffffffu, touched);
     const unsigned w_vis = __popc(__ballot_sync(0xffffffffu, touched > 0));
     if (lane_id() == 0 && w_vis) {

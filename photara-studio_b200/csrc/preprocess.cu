@@ -35,17 +35,21 @@ __global__ void __launch_bounds__(kBlock) preprocess_kernel(
     if (threadIdx.x < 4)
         s_tot[threadIdx.x] = threadIdx.x == 2 ? 0xffffffffu : 0u;
     __syncthreads();
+    __shared__ uint4 s_rec[kBlock][4];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned touched = 0, depth_bits = 0;
+    SplatRec rec;
     if (i < n) {
         const PreResult r = preprocess_one<kTileW, kTileH, kGeometry>(
             i, size_t(i), means, log_scales, quats, logits, filter_3d, sh, colors, sh_degree,
-            sh_bases, K, st);
+            sh_bases, K, st, rec);
         touched = r.touched;
         depth_bits = r.depth_bits;
         st.touched[i] = touched;
         radii[i] = r.radius;
     }
+    const int warp0 = int(threadIdx.x) & ~31;
+    store_records(s_rec + warp0, touched > 0, rec, st.rec + blockIdx.x * blockDim.x + warp0);
     const unsigned full = 0xffffffffu;
     const unsigned w_inst = __reduce_add_sync(full, touched);
     const unsigned w_vis = __popc(__ballot_sync(full, touched > 0));

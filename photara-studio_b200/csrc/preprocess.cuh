@@ -18,8 +18,35 @@ struct PreResult {
     int radius;          // conservative pixel radius (0: culled)
 };
 
+// Stores the records of a warp's 32 consecutive slots (dst: lane 0's; the lanes
+// with `visible`) through the warp's shared memory, so that each store covers
+// whole 64-byte records: stored by their own lanes, a 16-byte part of 32
+// records at a time, they were four times the write requests. With the records
+// the only copy of their fields the preprocess went from 72 to 66 us at 1M /
+// 1080p and from 525 to 470 us at 8.4M / 2160p. Parts are swizzled by record,
+// so both sides use every bank. Whole warps call this.
+__device__ __forceinline__ void store_records(uint4 (*s)[4], bool visible, const SplatRec& r,
+                                              SplatRec* dst) {
+    const int lane = int(lane_id());
+    if (visible) {
+        const uint4* part = reinterpret_cast<const uint4*>(&r);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            s[lane][q ^ ((lane >> 1) & 3)] = part[q];
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, visible);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int k = 8 * q + (lane >> 2), part = lane & 3;
+        if ((mask >> k) & 1u)
+            reinterpret_cast<uint4*>(dst + k)[part] = s[k][part ^ ((k >> 1) & 3)];
+    }
+}
+
 // Writes the forward state of Gaussian i into slot `slot` of st when it is
-// visible (touched > 0); st.touched / radii are left to the caller. kGeometry
+// visible (touched > 0), but its record, which goes to `r`; st.touched / radii
+// are left to the caller. kGeometry
 // also writes the ray plane and normal of the median-depth channel.
 template <int TW, int TH, bool kGeometry = false>
 __device__ __forceinline__ PreResult preprocess_one(
@@ -27,7 +54,7 @@ __device__ __forceinline__ PreResult preprocess_one(
     const float* __restrict__ quats, const float* __restrict__ logits,
     const float* __restrict__ filter_3d, const float* __restrict__ sh,
     const float* __restrict__ colors, int sh_degree, int sh_bases, const Camera& K,
-    const GaussianState& st) {
+    const GaussianState& st, SplatRec& r) {
     unsigned touched = 0;
     unsigned depth_bits = 0;
     int radius_out = 0;
@@ -99,13 +126,11 @@ __device__ __forceinline__ PreResult preprocess_one(
                     static_cast<unsigned short>(fmaxf(0.f, fminf(65535.f, floorf(px + ex) + 1.f))),
                     static_cast<unsigned short>(fmaxf(0.f, fminf(65535.f, floorf(py - ey)))),
                     static_cast<unsigned short>(fmaxf(0.f, fminf(65535.f, floorf(py + ey) + 1.f))));
-                SplatRec r;
                 r.co = co;
                 r.rgb = make_float4(rgb.x, rgb.y, rgb.z, __uint_as_float(clamp_bits));
                 r.xy = m2;
                 r.bounds = box;
                 r.spans = spans;
-                st.rec[slot] = r;
             }
         }
     }
