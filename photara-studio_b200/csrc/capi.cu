@@ -620,7 +620,7 @@ gs_status gs_backward(gs_context* c, const float* fwd_alpha, const int* fwd_radi
                 st, c->tiles, reinterpret_cast<const uint2*>(c->ranges.p), c->vals[c->sorted_buf],
                 gst, c->K, c->bg, c->pix_T, c->pix_last, c->pix_dtdt, dL->color, dL->alpha,
                 dL->densify_map, grads && grads->refine_weight ? 1 : 0, dL->median_depth,
-                dL->normal, c->fwd_depth, c->fwd_normal);
+                dL->normal, c->fwd_depth, c->fwd_normal, record_staging(c));
         else if (c->instances > 0)
             launch_composite_backward(st, c->tiles, reinterpret_cast<const uint2*>(c->ranges.p),
                                       c->vals[c->sorted_buf], c->st, c->K, c->bg, c->pix_T,
@@ -922,8 +922,8 @@ gs_status gs_pruning_scores(gs_context* c, const float* image, int gaussian_pop,
         if (c->instances <= 0)
             return; // nothing drawn: no score
         ck(launch_pruning_scores(c->stream, c->tiles, reinterpret_cast<const uint2*>(c->ranges.p),
-                                 c->vals[c->sorted_buf], c->st, c->K, c->pix_last, image,
-                                 gaussian_pop ? 1 : 0, scores),
+                                 c->vals[c->sorted_buf], c->K, c->pix_last, image,
+                                 gaussian_pop ? 1 : 0, scores, record_staging(c)),
            "pruning score launch");
     });
 }

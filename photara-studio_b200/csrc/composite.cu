@@ -167,14 +167,21 @@ void launch_composite_count_pairs(cudaStream_t s, int tiles, const uint2* ranges
 // transmittance along the ray crosses 0.5: each Gaussian is a 1D Gaussian
 // along the ray around its plane depth, and the pixel's transmittance at a
 // probe depth is the product of the Gaussians' partial opacities there; 8
-// probes over a +-0.4 window around the seed, refined 5 times (every
-// refinement walks the tile's list up to the pixel's last contributor again),
-// then linear interpolation inside the final bracket.
+// probes over a +-0.4 window around the seed, refined 5 times (the first two
+// refinements walk the tile's list up to the pixel's last contributor again,
+// the later ones the few Gaussians kept around the bracket), then linear
+// interpolation inside the final bracket.
 constexpr int kDepthSplit = 8;
 constexpr int kDepthRefinements = 5;
 constexpr float kDepthSeedWindow = 0.4f;
 constexpr float kDepthMinTransmittance = 0.45f;
 constexpr int kGeoThreads = kTileW * kTileH;
+// Gaussians kept per pixel around the second refinement's bracket (0.1 wide),
+// in thread-local memory. Forward with depth, us, before / keeping 24, 48, 64:
+// 500,000 at 1280x720 1,760 / 1,343, 1,134, 1,172; 50,000 dense at 1280x960
+// 2,295 / 2,334, 2,047, 2,004; 20,000 at 320x243 584 / 621, 320, 335 (with too
+// few, most blocks hold a pixel that has to walk its list again).
+constexpr int kNear = 64;
 
 __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
     const uint2* __restrict__ ranges, const unsigned* __restrict__ order, GaussianState st,
@@ -264,20 +271,9 @@ __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
         block_max = max(block_max, s_warp[w]);
 
     // ---- pass 2: median-depth bisection ----
-    constexpr int S = kDepthSplit;
-    float depth_min = fmaxf(seed - kDepthSeedWindow, 0.f);
-    float depth_max = fmaxf(seed + kDepthSeedWindow, 0.f);
-    bool in_range = T <= kDepthMinTransmittance;
-    float Tp[S + 1];
-#pragma unroll
-    for (int r = 0; r < kDepthRefinements; ++r) {
-        const bool first = r == 0;
-#pragma unroll
-        for (int k = 0; k <= S; ++k)
-            if (first || (k > 0 && k < S))
-                Tp[k] = 1.f;
-        const float interval = (depth_max - depth_min) * (1.f / float(S));
-        bool ldone = !in_range;
+    // Walks the pixel's blended Gaussians (alpha, peak distance, 1/sigma).
+    auto walk = [&](bool run, auto&& f) {
+        bool ldone = !run;
         unsigned seen = 0;
         for (int base = 0; base < int(block_max); base += kGeoThreads) {
             if (__syncthreads_and(ldone))
@@ -302,48 +298,56 @@ __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
                 if (alpha < kAlphaFloor)
                     continue;
                 const float4 rp = s_plane[j];
-                const float t_peak = rp.x * dx + rp.y * dy + rp.z;
-                const float rsigma = rp.w;
-                const bool ball = rsigma > 0.f;
-                // Beyond 8 sigma of the peak a probe's Gaussian factor is
-                // exactly 0 in the product (alpha g < 2^-25, so 1 - alpha g
-                // rounds to 1 and its inverse square root is 1): the probe
-                // takes (1 - alpha) behind the peak and 1 in front of it. A
-                // Gaussian whose peak is over 8 sigma behind every probe
-                // changes nothing; one over 8 sigma in front scales all.
-                const int k0 = first ? 0 : 1, k1 = first ? S : S - 1;
-                const float d_lo = (depth_min + interval * float(k0) - t_peak) * rsigma;
-                const float d_hi = (depth_min + interval * float(k1) - t_peak) * rsigma;
-                if (ball && d_hi < -8.f)
-                    continue;
-                const float oma = 1.f - alpha;
-                if (!ball || d_lo > 8.f) {
-#pragma unroll
-                    for (int k = 0; k <= S; ++k) {
-                        if (!(first || (k > 0 && k < S)))
-                            continue;
-                        const float ts = depth_min + interval * float(k);
-                        Tp[k] *= ts > t_peak ? oma : 1.f;
-                    }
-                    continue;
-                }
-#pragma unroll
-                for (int k = 0; k <= S; ++k) {
-                    if (!(first || (k > 0 && k < S)))
-                        continue;
-                    const float ts = depth_min + interval * float(k);
-                    const float delta = (ts - t_peak) * rsigma;
-                    if (delta * delta > 64.f) {
-                        Tp[k] *= ts > t_peak ? oma : 1.f;
-                        continue;
-                    }
-                    const float gk = expf(-0.5f * delta * delta);
-                    const float omg = 1.f - alpha * gk;
-                    const float rv = rsqrtf(omg);
-                    Tp[k] *= (ts > t_peak ? oma : omg) * rv;
-                }
+                f(alpha, rp.x * dx + rp.y * dy + rp.z, rp.w);
             }
         }
+    };
+    constexpr int S = kDepthSplit;
+    float depth_min = fmaxf(seed - kDepthSeedWindow, 0.f);
+    float depth_max = fmaxf(seed + kDepthSeedWindow, 0.f);
+    bool in_range = T <= kDepthMinTransmittance;
+    float Tp[S + 1];
+    float interval = 0.f;
+    // One Gaussian's factors on the probes (first: the window's ends too).
+    // Beyond 6 sigma of the peak a probe's Gaussian factor is exactly 0 in the
+    // product (alpha g < 2^-25, so 1 - alpha g rounds to 1 and its inverse
+    // square root is 1): the probe takes (1 - alpha) behind the peak and 1 in
+    // front of it. A Gaussian whose peak is that far behind every probe
+    // changes nothing; one that far in front scales all.
+    auto probe = [&](bool first, float alpha, float t_peak, float rsigma) {
+        const bool ball = rsigma > 0.f;
+        const int k0 = first ? 0 : 1, k1 = first ? S : S - 1;
+        const float d_lo = (depth_min + interval * float(k0) - t_peak) * rsigma;
+        const float d_hi = (depth_min + interval * float(k1) - t_peak) * rsigma;
+        if (ball && d_hi < -6.f)
+            return;
+        const float oma = 1.f - alpha;
+        const bool step = !ball || d_lo > 6.f;
+#pragma unroll
+        for (int k = 0; k <= S; ++k) {
+            if (!(first || (k > 0 && k < S)))
+                continue;
+            const float ts = depth_min + interval * float(k);
+            const float delta = (ts - t_peak) * rsigma;
+            if (step || delta * delta > 36.f) {
+                Tp[k] *= ts > t_peak ? oma : 1.f;
+                continue;
+            }
+            const float gk = expf(-0.5f * delta * delta);
+            const float omg = 1.f - alpha * gk;
+            const float rv = rsqrtf(omg);
+            Tp[k] *= (ts > t_peak ? oma : omg) * rv;
+        }
+    };
+    auto begin = [&](bool first, float t) {
+#pragma unroll
+        for (int k = 0; k <= S; ++k)
+            if (first || (k > 0 && k < S))
+                Tp[k] = t;
+        interval = (depth_max - depth_min) * (1.f / float(S));
+    };
+    // Keeps the bracket of the probes around transmittance 0.5.
+    auto narrow = [&](bool first) {
         if (first)
             in_range = Tp[0] >= 0.5f && Tp[S] <= 0.5f && in_range;
         int start = 0;
@@ -362,6 +366,49 @@ __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
         depth_min = depth_min + float(start + 0) * interval;
         Tp[0] = lo_T;
         Tp[S] = hi_T;
+    };
+    begin(true, 1.f);
+    walk(in_range, [&](float alpha, float t, float rs) { probe(true, alpha, t, rs); });
+    narrow(true);
+    // The second refinement's walk also sorts the Gaussians by its bracket,
+    // which holds all later probes: those 8 sigma or more behind it change
+    // nothing any more, those as far in front scale every probe, and the few
+    // left are kept. The later refinements and dT/dt then need no walk (five
+    // walks of the list before, and a sixth for dT/dt).
+    float near_alpha[kNear], near_peak[kNear], near_rs[kNear];
+    int near_n = 0;
+    float front = 1.f;
+    begin(false, 1.f);
+    walk(in_range, [&](float alpha, float t, float rs) {
+        probe(false, alpha, t, rs);
+        const bool ball = rs > 0.f;
+        if (ball && (depth_max - t) * rs < -8.f)
+            return;
+        if (ball && (depth_min - t) * rs > 8.f) {
+            front *= 1.f - alpha;
+            return;
+        }
+        if (near_n < kNear) {
+            near_alpha[near_n] = alpha;
+            near_peak[near_n] = t;
+            near_rs[near_n] = rs;
+        }
+        ++near_n;
+    });
+    narrow(false);
+    // a pixel with more of them than are kept walks its list again
+    const bool kept = near_n <= kNear;
+    const bool any_over = __syncthreads_or(in_range && !kept);
+#pragma unroll 1
+    for (int r = 2; r < kDepthRefinements; ++r) {
+        begin(false, kept ? front : 1.f);
+        if (in_range && kept)
+            for (int k = 0; k < near_n; ++k)
+                probe(false, near_alpha[k], near_peak[k], near_rs[k]);
+        if (any_over)
+            walk(in_range && !kept,
+                 [&](float alpha, float t, float rs) { probe(false, alpha, t, rs); });
+        narrow(false);
     }
     const float w_max = __saturatef((Tp[0] - 0.5f) / (Tp[0] - Tp[S]));
     const float w_min = 1.f - w_max;
@@ -375,43 +422,23 @@ __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
     // -1/4 G_t / (1 - G_t) |delta| / sigma (render_backward.cu:47-151,
     // median_scale_walk, here evaluated where the median is found, at the
     // distance the backward recovers from the written depth). The backward
-    // turns it into dL/dt with the depth gradient.
+    // turns it into dL/dt with the depth gradient. Gaussians beyond 8 sigma
+    // of the bracket (G_t below 1.3e-14) add nothing.
     float dTdt = 0.f;
     if (pix_dtdt) {
         const float mD = depth_out / fmaxf(rln, 1.0e-8f);
-        bool ldone = !(inside && mD != 0.f && last != 0);
-        unsigned seen = 0;
-        for (int base = 0; base < int(block_max); base += kGeoThreads) {
-            if (__syncthreads_and(ldone))
-                break;
-            if (base + tid < int(block_max)) {
-                const unsigned g = order[range.x + base + tid];
-                s_xy[tid] = st.rec[g].xy;
-                s_co[tid] = st.rec[g].co;
-                s_plane[tid] = st.plane[g];
-            }
-            __syncthreads();
-            const int cnt = min(kGeoThreads, int(block_max) - base);
-            for (int j = 0; !ldone && j < cnt; ++j) {
-                ++seen;
-                ldone = seen >= last;
-                const float dx = s_xy[j].x - fx, dy = s_xy[j].y - fy;
-                const float4 co = s_co[j];
-                const float power = gaussian_power(co, dx, dy);
-                if (power > 0.f)
-                    continue;
-                const float alpha = fminf(clip, co.w * expf(power));
-                if (alpha < kAlphaFloor)
-                    continue;
-                const float4 rp = s_plane[j];
-                const float t_peak = rp.x * dx + rp.y * dy + rp.z;
-                const float rsigma = rp.w;
-                const float t_delta = (mD - t_peak) * rsigma;
-                const float g_exp = expf(-0.5f * t_delta * t_delta);
-                const float gt = alpha * g_exp;
-                dTdt += -0.25f * gt / (1.f - gt) * fabsf(t_delta) * rsigma;
-            }
-        }
+        const bool run = inside && mD != 0.f && last != 0;
+        auto slope = [&](float alpha, float t, float rs) {
+            const float t_delta = (mD - t) * rs;
+            const float g_exp = expf(-0.5f * t_delta * t_delta);
+            const float gt = alpha * g_exp;
+            dTdt += -0.25f * gt / (1.f - gt) * fabsf(t_delta) * rs;
+        };
+        if (run && kept)
+            for (int k = 0; k < near_n; ++k)
+                slope(near_alpha[k], near_peak[k], near_rs[k]);
+        if (any_over)
+            walk(run && !kept, slope);
     }
 
     if (inside) {
@@ -448,33 +475,21 @@ void launch_composite_geometry(cudaStream_t s, int tiles, const uint2* ranges,
 // ------------------------------------------- geometry-channel adjoint ----
 // Backward of the colour, median-depth and normal channels together
 // (render_backward.cu:156-519, blend_bucket_backward<GEOMETRY = true>): one
-// thread per pixel of a 16x16 tile walks its list back to front from its last
-// contributor, recovering T by T_i = T_{i+1} / (1 - a_i) as the colour
-// adjoint does. Per pixel it also carries the normal-output gradient divided
-// by the rendered alpha (the normal output is the alpha-normalised sum), the
-// running sum of the normals blended behind the current Gaussian projected on
-// it, the median distance and dL/dt (the depth gradient over -dT/dt from the
-// forward). Per (Gaussian, pixel) it adds, besides the colour terms: to
-// dL/d opacity the normal term and the median term, to dL/d mean2d the ray
-// plane's screen slope times dL/dt, and the gradients of the footprint normal
-// (3) and of the ray plane (4). The refine weight takes the colour part of
-// the mean2d gradient only, as the reference's. Twelve colour partials and
-// seven geometry partials per Gaussian are reduced across the warp (two
-// reduce-scatters), summed per tile in shared memory and added with five
-// float4 atomics per (Gaussian, tile).
-constexpr int kGeoBatch = kGeoThreads;
-
-struct GeoBackStage {
-    unsigned id[kGeoBatch];
-    float2 xy[kGeoBatch];
-    float4 co[kGeoBatch];
-    float4 rgb[kGeoBatch];
-    float4 plane[kGeoBatch];
-    float4 nrm[kGeoBatch];
-    unsigned char band[kGeoBatch];
-    float acc[kGeoBatch][20]; // [0, 12) colour slots, [12, 16) ray plane, [16, 19) normal
-};
-
+// warp per strip walks it back to front from its pixels' last contributors,
+// recovering T by T_i = T_{i+1} / (1 - a_i) as the colour adjoint does. Per
+// pixel it also carries the normal-output gradient divided by the rendered
+// alpha (the normal output is the alpha-normalised sum), the running sum of the
+// normals blended behind the current Gaussian projected on it, the median
+// distance and dL/dt (the depth gradient over -dT/dt from the forward). Per
+// (Gaussian, pixel) it adds, besides the colour terms: to dL/d opacity the
+// normal term and the median term, to dL/d mean2d the ray plane's screen slope
+// times dL/dt, and the gradients of the footprint normal (3) and of the ray
+// plane (4). The refine weight takes the colour part of the mean2d gradient
+// only, as the reference's. A pixel adds the moments of its gradient (strip.cuh)
+// and of dL/dt; the partials are formed per lane, reduced across the warp (two
+// reduce-scatters) and added by one atomic each. Bound: instruction issue.
+// 500,000 Gaussians at 1280x720 1,030 -> 723 us, against a thread per pixel,
+// both reductions per 32 pixels and accumulators in shared memory.
 // Reduce 8 per-lane values across the warp; returns the sum of slot `slot`
 // (slot = -1 for lanes that hold a duplicate).
 __device__ __forceinline__ float reduce_scatter8(const float (&v)[8], int& slot) {
@@ -504,8 +519,20 @@ __device__ __forceinline__ float reduce_scatter8(const float (&v)[8], int& slot)
     return x;
 }
 
-template <bool kRefine, bool kDensify>
-__global__ void __launch_bounds__(kGeoThreads) composite_backward_geometry_kernel(
+// Ray planes and normals of a strip's two batches, beside the records.
+struct GeoStage {
+    float4 plane[2][kStripBatch];
+    float4 normal[2][kStripBatch];
+};
+
+__device__ __forceinline__ void geo_copy16(float4* dst, const float4* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src)
+                 : "memory");
+}
+
+template <int PX, bool kRefine, bool kDensify>
+__global__ void __launch_bounds__(32, PX == 4 ? 16 : 20) composite_backward_geometry_kernel(
+    const __grid_constant__ CUtensorMap map, unsigned* __restrict__ err,
     const uint2* __restrict__ ranges, const unsigned* __restrict__ order, GaussianState st,
     const Camera K, float3 bg, const float* __restrict__ pix_T,
     const unsigned* __restrict__ pix_last, const float* __restrict__ pix_dtdt,
@@ -513,218 +540,207 @@ __global__ void __launch_bounds__(kGeoThreads) composite_backward_geometry_kerne
     const float* __restrict__ densify_map, const float* __restrict__ dL_depth,
     const float* __restrict__ dL_normal, const float* __restrict__ fwd_depth,
     const float* __restrict__ fwd_normal) {
-    __shared__ GeoBackStage s;
-    __shared__ unsigned s_wmax[kGeoThreads / 32];
-    for (int k = threadIdx.x; k < kGeoBatch * 20; k += kGeoThreads)
-        (&s.acc[0][0])[k] = 0.f;
-    const int tile = blockIdx.x;
-    const int tx = tile % K.grid_x, ty = tile / K.grid_x;
-    const int tid = threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
-    const int px = tx * kTileW + tid % kTileW, py = ty * kTileH + tid / kTileW;
-    const bool inside = px < K.width && py < K.height;
-    const float fx = float(px), fy = float(py);
+    using G = StripGeom<kTileW, PX>;
+    constexpr int NP = G::kBands;
+    constexpr unsigned full = 0xffffffffu;
+    constexpr int kStrips = kTileH / G::kRows;
+    __shared__ StripStage s;
+    __shared__ GeoStage geo;
+    StripFeed feed{s, &map, err};
+    feed.init();
+    const int tile = int(blockIdx.x) / kStrips, strip = int(blockIdx.x) % kStrips;
+    const int lane = int(lane_id());
+    const int x0 = (tile % K.grid_x) * kTileW;
+    const int y0 = (tile / K.grid_x) * kTileH + strip * G::kRows;
+    const int px = x0 + lane % kTileW;
+    const int py = y0 + 2 * (lane / kTileW); // pixel 2 p + q: row py + p * kBandRows + q
+    const float fx = float(px);
     const uint2 range = ranges[tile];
     const float clip = K.alpha_clip;
     const size_t P = size_t(K.width) * K.height;
-    const size_t pid = inside ? size_t(py) * K.width + px : 0;
     const bool with_depth = dL_depth != nullptr, with_normal = dL_normal != nullptr;
-
-    // ---- per-pixel state ----
-    float T_final = 1.f, gx = 0.f, gy = 0.f, gz = 0.f, gnx = 0.f, gny = 0.f, gnz = 0.f;
-    float fin_r = 0.f, fin = 0.f, dmap = 0.f, mD = 0.f, dmt = 0.f;
-    unsigned last = 0;
-    if (inside) {
-        T_final = pix_T[pid];
-        last = pix_last[pid];
-        gx = dL_color[pid];
-        gy = dL_color[P + pid];
-        gz = dL_color[2 * P + pid];
-        const float dfin_r = bg.x * gx + bg.y * gy + bg.z * gz - (dL_alpha ? dL_alpha[pid] : 0.f);
-        float dfin = dfin_r;
-        if (with_normal) {
-            // the normal output is the blended normal sum over alpha = 1 - T
-            const float wf = 1.f - T_final;
-            const float inv_w = wf > 0.f ? 1.f / wf : 0.f;
-            gnx = dL_normal[pid] * inv_w;
-            gny = dL_normal[P + pid] * inv_w;
-            gnz = dL_normal[2 * P + pid] * inv_w;
-            dfin += gnx * fwd_normal[pid] + gny * fwd_normal[P + pid] + gnz * fwd_normal[2 * P + pid];
-        }
-        if (with_depth) {
-            const float rln = pixel_ray_z(fx, fy, K);
-            mD = fwd_depth[pid] / fmaxf(rln, 1.0e-8f);
-            dmt = dL_depth[pid] * rln / fmaxf(-pix_dtdt[pid], 1.0e-7f);
-        }
-        fin_r = T_final * dfin_r;
-        fin = T_final * dfin;
-        dmap = densify_map ? densify_map[pid] : 0.f;
-    }
-    const float refine_scale = 1.f / fmaxf(1.f - T_final, 1.0e-5f);
-    float T = T_final, sdot = 0.f, ndot = 0.f;
     const float Wf = float(K.width), Hf = float(K.height);
 
-    unsigned wlast = last;
+    // ---- per-pixel state ----
+    float T[PX], sdot[PX], ndot[PX], gx[PX], gy[PX], gz[PX], gnx[PX], gny[PX], gnz[PX];
+    float fin_r[PX], fin[PX], rscale[PX], dmap[kDensify ? PX : 1], mD[PX], dmt[PX];
+    unsigned last[PX], wl = 0;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-        wlast = max(wlast, __shfl_xor_sync(0xffffffffu, wlast, off));
-    if (lane == 0)
-        s_wmax[warp] = wlast;
-    __syncthreads();
-    unsigned tile_last = 0;
-#pragma unroll
-    for (int w = 0; w < kGeoThreads / 32; ++w)
-        tile_last = max(tile_last, s_wmax[w]);
-    tile_last = min(tile_last, range.y - range.x);
-    const int batches = int((tile_last + kGeoBatch - 1) / kGeoBatch);
-    for (int b = batches - 1; b >= 0; --b) {
-        const int base = b * kGeoBatch;
-        const int cnt = min(kGeoBatch, int(tile_last) - base);
-        if (tid < cnt) {
-            const unsigned g = order[range.x + base + tid];
-            s.id[tid] = g;
-            s.xy[tid] = st.rec[g].xy;
-            s.co[tid] = st.rec[g].co;
-            s.rgb[tid] = st.rec[g].rgb;
-            s.plane[tid] = st.plane[g];
-            s.nrm[tid] = st.normal[g];
-            const ushort4 bx = st.rec[g].bounds;
-            unsigned m = 0;
-#pragma unroll
-            for (int w = 0; w < kGeoThreads / 32; ++w)
-                if (band_hit<kTileW, 2>(bx, tx * kTileW, ty * kTileH + 2 * w))
-                    m |= 1u << w;
-            s.band[tid] = static_cast<unsigned char>(m);
+    for (int k = 0; k < PX; ++k) {
+        const int y = py + (k / 2) * G::kBandRows + (k & 1);
+        T[k] = 1.f;
+        last[k] = 0;
+        sdot[k] = ndot[k] = gx[k] = gy[k] = gz[k] = gnx[k] = gny[k] = gnz[k] = 0.f;
+        fin_r[k] = fin[k] = mD[k] = dmt[k] = 0.f;
+        if constexpr (kDensify)
+            dmap[k] = 0.f;
+        if (px < K.width && y < K.height) {
+            const size_t pid = size_t(y) * K.width + px;
+            T[k] = pix_T[pid];
+            last[k] = pix_last[pid];
+            gx[k] = dL_color[pid];
+            gy[k] = dL_color[P + pid];
+            gz[k] = dL_color[2 * P + pid];
+            const float dfin_r =
+                bg.x * gx[k] + bg.y * gy[k] + bg.z * gz[k] - (dL_alpha ? dL_alpha[pid] : 0.f);
+            float dfin = dfin_r;
+            if (with_normal) {
+                // the normal output is the blended normal sum over alpha = 1 - T
+                const float wf = 1.f - T[k];
+                const float inv_w = wf > 0.f ? 1.f / wf : 0.f;
+                gnx[k] = dL_normal[pid] * inv_w;
+                gny[k] = dL_normal[P + pid] * inv_w;
+                gnz[k] = dL_normal[2 * P + pid] * inv_w;
+                dfin += gnx[k] * fwd_normal[pid] + gny[k] * fwd_normal[P + pid] +
+                        gnz[k] * fwd_normal[2 * P + pid];
+            }
+            if (with_depth) {
+                const float rln = pixel_ray_z(fx, float(y), K);
+                mD[k] = fwd_depth[pid] / fmaxf(rln, 1.0e-8f);
+                dmt[k] = dL_depth[pid] * rln / fmaxf(-pix_dtdt[pid], 1.0e-7f);
+            }
+            fin_r[k] = T[k] * dfin_r;
+            fin[k] = T[k] * dfin;
+            if constexpr (kDensify)
+                dmap[k] = densify_map ? densify_map[pid] : 0.f;
         }
-        __syncthreads();
-        const int jtop = min(cnt, int(wlast) - base) - 1;
-        for (int j = jtop; j >= 0; --j) {
-            if (!((s.band[j] >> warp) & 1u))
-                continue;
+        rscale[k] = 1.f / fmaxf(1.f - T[k], 1.0e-5f);
+        wl = max(wl, last[k]);
+    }
+    const int total = int(min(__reduce_max_sync(full, wl), range.y - range.x));
+    if (total == 0)
+        return;
+    const int slot = kDensify ? strip_slot12() : strip_slot10();
+    const float scale = slot_scale(slot);
+    float* const row = reinterpret_cast<float*>(st.grad) + max(slot, 0);
+
+    auto issue = [&](int b, unsigned first, int cnt) {
+        const unsigned id = feed.issue(b, order, first, cnt);
+        geo_copy16(&geo.plane[b][lane], st.plane + id);
+        geo_copy16(&geo.normal[b][lane], st.normal + id);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        return id;
+    };
+    int base = (total - 1) / kStripBatch * kStripBatch;
+    unsigned id_next = issue(0, range.x + unsigned(base), total - base);
+    int buf = 0;
+    for (; base >= 0; base -= kStripBatch) {
+        const int cnt = min(kStripBatch, total - base);
+        const unsigned id = id_next;
+        if (base > 0) {
+            id_next = issue(buf ^ 1, range.x + unsigned(base - kStripBatch), kStripBatch);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncwarp();
+        if (!feed.wait(buf)) {
+            if (base > 0)
+                feed.wait(buf ^ 1);
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            return;
+        }
+        const SplatRec* rec = feed.s.rec[buf];
+        unsigned mask[NP], all;
+        unsigned m = strip_masks<kTileW, PX>(rec, cnt, x0, y0, mask, all);
+        while (m) {
+            const int j = 31 - __clz(int(m));
+            m ^= 1u << j;
             const unsigned pos = unsigned(base + j);
-            float va[12], vg[8];
-#pragma unroll
-            for (int k = 0; k < 12; ++k)
-                va[k] = 0.f;
+            const float2 xy = rec[j].xy;
+            const float4 co = rec[j].co;
+            const float4 c = rec[j].rgb;
+            const float4 rp = geo.plane[buf][j];
+            const float4 n = geo.normal[buf][j];
+            const float dx = xy.x - fx;
+            PairSums<kDensify> acc; // .x: the lane's sums (.y unused, zero)
+            acc.s = acc.sy = acc.syy = acc.refine = f2s(0.f);
+            acc.cr = acc.cg = acc.cb = acc.dn = acc.dd = f2s(0.f);
+            float dts = 0.f, dty = 0.f; // sums of dL/dt, dL/dt dy
+            float vg[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k)
                 vg[k] = 0.f;
-            bool hit = false;
-            if (pos < last) {
-                const float2 m = s.xy[j];
-                const float4 co = s.co[j];
-                const float dx = m.x - fx, dy = m.y - fy;
+#pragma unroll
+            for (int k = 0; k < PX; ++k) {
+                if (!((mask[k / 2] >> j) & 1u))
+                    continue;
+                const float dy = xy.y - float(py + (k / 2) * G::kBandRows + (k & 1));
                 const float power = gaussian_power(co, dx, dy);
-                const float G = expf(power);
-                const float alpha = fminf(clip, co.w * G);
-                hit = !(power > 0.f) && !(alpha < kAlphaFloor);
-                if (hit) {
-                    const float4 c = s.rgb[j];
-                    const float inv_1ma = 1.f / (1.f - alpha);
-                    T = T * inv_1ma; // transmittance in front of this Gaussian
-                    const float w = alpha * T;
-                    const float cdot = c.x * gx + c.y * gy + c.z * gz;
-                    const float dL_da_r = T * cdot - (sdot + fin_r) * inv_1ma;
-                    float dL_da = T * cdot - (sdot + fin) * inv_1ma;
-                    sdot += w * cdot;
-                    if (with_normal) {
-                        const float4 n = s.nrm[j];
-                        const float nd = n.x * gnx + n.y * gny + n.z * gnz;
-                        dL_da += T * nd - ndot * inv_1ma;
-                        ndot += w * nd;
-                        vg[4] = w * gnx;
-                        vg[5] = w * gny;
-                        vg[6] = w * gnz;
-                    }
-                    const float4 rp = s.plane[j];
-                    float dt = 0.f;
-                    if (with_depth) {
-                        const float t_peak = rp.x * dx + rp.y * dy + rp.z;
-                        const float rsigma = rp.w;
-                        const float t_delta = (mD - t_peak) * rsigma;
-                        const float g_exp = expf(-0.5f * t_delta * t_delta);
-                        const float gt = alpha * g_exp;
-                        float dgt = dmt * 0.25f / (1.f - gt);
-                        dgt = mD > t_peak ? dgt : -dgt;
-                        dgt = rsigma > 0.f ? dgt : 0.f;
-                        dL_da += dgt * g_exp - dmt * (t_delta > 0.f ? 0.5f * inv_1ma : 0.f);
-                        const float ddelta = -dgt * gt * t_delta;
-                        vg[3] = ddelta * (mD - t_peak);
-                        dt = -ddelta * rsigma;
-                        vg[0] = dt * dx;
-                        vg[1] = dt * dy;
-                        vg[2] = dt;
-                    }
-                    const float dL_dG = co.w * dL_da;
-                    const float gdx = G * dx, gdy = G * dy;
-                    const float dgx = -gdx * co.x - gdy * co.y;
-                    const float dgy = -gdy * co.z - gdx * co.y;
-                    va[0] = -0.5f * gdx * dx * dL_dG;
-                    va[1] = -0.5f * gdx * dy * dL_dG;
-                    va[2] = -0.5f * gdy * dy * dL_dG;
-                    va[3] = G * dL_da;
-                    va[4] = dL_dG * dgx + dt * rp.x;
-                    va[5] = dL_dG * dgy + dt * rp.y;
-                    if constexpr (kRefine) {
-                        const float dL_dG_r = co.w * dL_da_r;
-                        const float rx = dL_dG_r * dgx * Wf, ry = dL_dG_r * dgy * Hf;
-                        va[6] = sqrtf(rx * rx + ry * ry) * refine_scale;
-                    }
-                    if constexpr (kDensify) {
-                        va[7] = dmap * w;
-                        va[11] = w;
-                    }
-                    va[8] = w * gx;
-                    va[9] = w * gy;
-                    va[10] = w * gz;
+                const float og = co.w * expf(power);
+                const float alpha = fminf(clip, og);
+                if (pos >= last[k] || power > 0.f || alpha < kAlphaFloor)
+                    continue;
+                const float inv_1ma = 1.f / (1.f - alpha);
+                T[k] *= inv_1ma; // transmittance in front of this Gaussian
+                const float w = alpha * T[k];
+                const float cdot = c.x * gx[k] + c.y * gy[k] + c.z * gz[k];
+                const float dL_da_r = T[k] * cdot - (sdot[k] + fin_r[k]) * inv_1ma;
+                float dL_da = T[k] * cdot - (sdot[k] + fin[k]) * inv_1ma;
+                sdot[k] += w * cdot;
+                if (with_normal) {
+                    const float nd = n.x * gnx[k] + n.y * gny[k] + n.z * gnz[k];
+                    dL_da += T[k] * nd - ndot[k] * inv_1ma;
+                    ndot[k] += w * nd;
+                    vg[4] += w * gnx[k];
+                    vg[5] += w * gny[k];
+                    vg[6] += w * gnz[k];
+                }
+                if (with_depth) {
+                    const float t_peak = rp.x * dx + rp.y * dy + rp.z;
+                    const float rsigma = rp.w;
+                    const float t_delta = (mD[k] - t_peak) * rsigma;
+                    const float g_exp = expf(-0.5f * t_delta * t_delta);
+                    const float gt = alpha * g_exp;
+                    float dgt = dmt[k] * 0.25f / (1.f - gt);
+                    dgt = mD[k] > t_peak ? dgt : -dgt;
+                    dgt = rsigma > 0.f ? dgt : 0.f;
+                    dL_da += dgt * g_exp - dmt[k] * (t_delta > 0.f ? 0.5f * inv_1ma : 0.f);
+                    const float ddelta = -dgt * gt * t_delta;
+                    const float dt = -ddelta * rsigma;
+                    vg[3] += ddelta * (mD[k] - t_peak);
+                    dts += dt;
+                    dty += dt * dy;
+                }
+                const float sg = og * dL_da, sgy = sg * dy;
+                acc.s.x += sg;
+                acc.sy.x += sgy;
+                acc.syy.x += sgy * dy;
+                if constexpr (kRefine) {
+                    const float sr = og * dL_da_r;
+                    const float rx = sr * (co.x * dx + co.y * dy) * Wf;
+                    const float ry = sr * (co.z * dy + co.y * dx) * Hf;
+                    acc.refine.x += sqrtf(rx * rx + ry * ry) * rscale[k];
+                }
+                // the colour and densify sums enter negated (slot_scale)
+                acc.cr.x -= w * gx[k];
+                acc.cg.x -= w * gy[k];
+                acc.cb.x -= w * gz[k];
+                if constexpr (kDensify) {
+                    acc.dn.x -= dmap[k] * w;
+                    acc.dd.x -= w;
                 }
             }
-            const unsigned hits = __ballot_sync(0xffffffffu, hit);
-            if (hits == 0)
-                continue;
-            if (__popc(hits) == 1) {
-                if (hit) {
-#pragma unroll
-                    for (int k = 0; k < 12; ++k)
-                        if (va[k] != 0.f)
-                            atomicAdd(&s.acc[j][k], va[k]);
-#pragma unroll
-                    for (int k = 0; k < 7; ++k)
-                        if (vg[k] != 0.f)
-                            atomicAdd(&s.acc[j][12 + k], vg[k]);
-                }
-                continue;
-            }
-            int slot;
-            const float ra = reduce_scatter12(va, slot);
-            if (slot >= 0 && ra != 0.f)
-                atomicAdd(&s.acc[j][slot], ra);
-            const float rg = reduce_scatter8(vg, slot);
-            if (slot >= 0 && slot < 7 && rg != 0.f)
-                atomicAdd(&s.acc[j][12 + slot], rg);
+            float v[12];
+            lane_partials<kDensify>(acc, kRefine, co, dx, v);
+            v[4] -= rp.x * dts; // scaled by -1
+            v[5] -= rp.y * dts;
+            vg[0] = dx * dts;
+            vg[1] = dty;
+            vg[2] = dts;
+            const unsigned gid = __shfl_sync(full, id, j);
+            const float sum = kDensify ? strip_reduce12(v) : strip_reduce10(v);
+            if (slot >= 0 && sum != 0.f)
+                atomicAdd(row + size_t(gid) * (4 * kGradSlots),
+                          sum * (slot == 3 ? 1.f / co.w : scale));
+            int gslot;
+            const float gsum = reduce_scatter8(vg, gslot);
+            if (gslot >= 0 && gslot < 7 && gsum != 0.f)
+                atomicAdd(reinterpret_cast<float*>(st.geo_grad) + size_t(gid) * (4 * kGeoGradSlots) +
+                              gslot,
+                          gsum);
         }
-        __syncthreads();
-        if (tid < cnt) {
-            float* a = s.acc[tid];
-            bool any = false;
-#pragma unroll
-            for (int q = 0; q < 19; ++q)
-                any |= a[q] != 0.f;
-            if (any) {
-                const size_t g = s.id[tid];
-                float4* dst = st.grad + g * kGradSlots;
-                atomicAdd(dst + 0, make_float4(a[0], a[1], a[2], a[3]));
-                atomicAdd(dst + 1, make_float4(a[4], a[5], a[6], a[7]));
-                atomicAdd(dst + 2, make_float4(a[8], a[9], a[10], a[11]));
-                float4* gdst = st.geo_grad + g * kGeoGradSlots;
-                atomicAdd(gdst + 0, make_float4(a[12], a[13], a[14], a[15]));
-                atomicAdd(gdst + 1, make_float4(a[16], a[17], a[18], 0.f));
-#pragma unroll
-                for (int q = 0; q < 19; ++q)
-                    a[q] = 0.f;
-            }
-        }
-        __syncthreads();
+        buf ^= 1;
     }
 }
 
@@ -735,16 +751,29 @@ void launch_composite_backward_geometry(cudaStream_t s, int tiles, const uint2* 
                                         const float* dL_color, const float* dL_alpha,
                                         const float* densify_map, int want_refine,
                                         const float* dL_depth, const float* dL_normal,
-                                        const float* fwd_depth, const float* fwd_normal) {
-#define GSB_GEO_BWD(R, D)                                                                        \
-    composite_backward_geometry_kernel<R, D><<<tiles, kGeoThreads, 0, s>>>(                      \
-        ranges, order, st, K, bg, pix_T, pix_last, pix_dtdt, dL_color, dL_alpha, densify_map,    \
-        dL_depth, dL_normal, fwd_depth, fwd_normal)
-    if (want_refine && densify_map) GSB_GEO_BWD(true, true);
-    else if (want_refine) GSB_GEO_BWD(true, false);
-    else if (densify_map) GSB_GEO_BWD(false, true);
-    else GSB_GEO_BWD(false, false);
-#undef GSB_GEO_BWD
+                                        const float* fwd_depth, const float* fwd_normal,
+                                        const RecStaging& rs) {
+    auto bwd = [&]<int PX>() {
+        auto go = [&](auto kernel) {
+            kernel<<<tiles * (8 / PX), 32, 0, s>>>(rs.map, rs.err, ranges, order, st, K, bg, pix_T,
+                                                   pix_last, pix_dtdt, dL_color, dL_alpha,
+                                                   densify_map, dL_depth, dL_normal, fwd_depth,
+                                                   fwd_normal);
+        };
+        if (want_refine && densify_map)
+            go(composite_backward_geometry_kernel<PX, true, true>);
+        else if (want_refine)
+            go(composite_backward_geometry_kernel<PX, true, false>);
+        else if (densify_map)
+            go(composite_backward_geometry_kernel<PX, false, true>);
+        else
+            go(composite_backward_geometry_kernel<PX, false, false>);
+    };
+    // more strips where there are too few tiles to fill the GPU
+    if (tiles <= 1000)
+        bwd.template operator()<2>();
+    else
+        bwd.template operator()<4>();
 }
 
 void launch_composite_forward(cudaStream_t s, int tiles, const uint2* ranges,

@@ -59,14 +59,6 @@ __device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* map, i
         : "memory");
 }
 
-template <int TW, int kRows>
-__device__ __forceinline__ bool band_hit(ushort4 b, int x0, int y0) {
-    // Warp pixels: x in [x0, x0+TW), y in [y0, y0+kRows); box widened by 1 px
-    // so the test can only drop Gaussians whose alpha is below 1/255 there.
-    return int(b.x) - 1 < x0 + TW && int(b.y) + 1 > x0 && int(b.z) - 1 < y0 + kRows &&
-           int(b.w) + 1 > y0;
-}
-
 // One view's image constants and buffers, already offset to that view.
 struct ViewTarget {
     int width, height;
@@ -99,43 +91,6 @@ __device__ __forceinline__ void warp_count_add(unsigned long long v, unsigned lo
         v += __shfl_xor_sync(0xffffffffu, v, off);
     if ((threadIdx.x & 31) == 0 && v)
         atomicAdd(out, v);
-}
-
-// Reduce 12 per-lane values across the warp; returns the summed value of
-// slot `slot` (or slot = -1 for lanes that hold nothing).
-__device__ __forceinline__ float reduce_scatter12(const float (&v)[12], int& slot) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
-    float u[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const float send = b4 ? v[k] : v[k + 6];
-        const float keep = b4 ? v[k + 6] : v[k];
-        u[k] = keep + __shfl_xor_sync(full, send, 16);
-    }
-    float w[4];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float send = b3 ? u[k] : u[k + 3];
-        const float keep = b3 ? u[k + 3] : u[k];
-        w[k] = keep + __shfl_xor_sync(full, send, 8);
-    }
-    w[3] = 0.f;
-    float x[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const float send = b2 ? w[k] : w[k + 2];
-        const float keep = b2 ? w[k + 2] : w[k];
-        x[k] = keep + __shfl_xor_sync(full, send, 4);
-    }
-    const float send = b1 ? x[0] : x[1];
-    const float keep = b1 ? x[1] : x[0];
-    float y = keep + __shfl_xor_sync(full, send, 2);
-    y += __shfl_xor_sync(full, y, 1);
-    const int idx = b2 ? (b1 ? -1 : 2) : (b1 ? 1 : 0);
-    slot = (idx < 0 || (lane & 1)) ? -1 : (b4 ? 6 : 0) + (b3 ? 3 : 0) + idx;
-    return y;
 }
 
 // Per-pixel backward state.

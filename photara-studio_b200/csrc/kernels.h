@@ -356,7 +356,8 @@ void launch_composite_backward_geometry(cudaStream_t s, int tiles, const uint2* 
                                         const float* dL_color, const float* dL_alpha,
                                         const float* densify_map, int want_refine,
                                         const float* dL_depth, const float* dL_normal,
-                                        const float* fwd_depth, const float* fwd_normal);
+                                        const float* fwd_depth, const float* fwd_normal,
+                                        const RecStaging& rs);
 void launch_composite_backward(cudaStream_t s, int tiles, const uint2* ranges,
                                const unsigned* order, const GaussianState& st, const Camera& K,
                                float3 bg, const float* pix_T, const unsigned* pix_last,
@@ -367,9 +368,9 @@ void launch_composite_backward(cudaStream_t s, int tiles, const uint2* ranges,
                                const SegmentStore* segments = nullptr);
 
 cudaError_t launch_pruning_scores(cudaStream_t s, int tiles, const uint2* ranges,
-                                  const unsigned* order, const GaussianState& st, const Camera& K,
+                                  const unsigned* order, const Camera& K,
                                   const unsigned* pix_last, const float* image, int gaussian_pop,
-                                  float* scores);
+                                  float* scores, const RecStaging& rs);
 
 cudaError_t launch_set_colors(cudaStream_t s, int n, const float* colors, SplatRec* rec);
 
