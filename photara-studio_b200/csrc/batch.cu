@@ -625,7 +625,7 @@ struct gs_batch {
     gs_settings s{};
     gs_batch_schedule sched{16, 16, 4, kSchedDynamic, 0};
     int views = 0;
-    size_t pairs = 0, capacity = 0, total_pixels = 0;
+    size_t pairs = 0, capacity = 0, total_pixels = 0, strips = 0;
     unsigned total_tiles = 0;
     int tile_bits = 0;
     int px = 4; // pixels per thread of the strips
@@ -959,7 +959,7 @@ void plan(gs_batch* b, const gs_gaussians* g, const gs_camera* cams, int views,
     encode_record_map(&b->staging.map, b->st.rec, pairs);
     b->staging.err = b->counters + kBcErr;
     b->hist_buf.exact(8 * kMaxRadix * sizeof(unsigned), st);
-    b->tile_ctr_buf.exact(64 * sizeof(unsigned), st);
+    b->tile_ctr_buf.exact((64 + 2 * kWorkClasses) * sizeof(unsigned), st);
     b->scan_status_buf.exact(std::max<size_t>(scan_status_bytes(int(pairs)), 256), st);
     // the schedule's kernels: grid sizes and attributes
     const size_t gsmem = batch_gaussian_backward_smem(views);
@@ -995,15 +995,7 @@ void plan(gs_batch* b, const gs_gaussians* g, const gs_camera* cams, int views,
         req(items < (size_t(1) << 31), "too many tiles");
         b->grid_fwd = int(std::min<size_t>(size_t(b->sms) * of, items));
         b->grid_bwd = int(std::min<size_t>(size_t(b->sms) * ob, items));
-        b->heavy = b->work = StripOrder{};
-        if (sc.schedule == kSchedHeavyFirst) {
-            // counts of both orders side by side (one memset), then the lists
-            unsigned* w = reinterpret_cast<unsigned*>(b->order_buf.exact(
-                sizeof(unsigned) * kWorkClasses * (2 + tiles + items), st));
-            b->heavy = {w, w + 2 * kWorkClasses, unsigned(tiles)};
-            b->work = {w + kWorkClasses, w + 2 * kWorkClasses + kWorkClasses * tiles,
-                       unsigned(items)};
-        }
+        b->strips = items;
     });
     // instance capacity
     size_t cap = instance_capacity;
@@ -1025,6 +1017,20 @@ void plan(gs_batch* b, const gs_gaussians* g, const gs_camera* cams, int views,
     for (int k = 0; k < 2; ++k) {
         b->ikeys[k] = reinterpret_cast<unsigned*>(ik + align_up(cap * 4) * k);
         b->ivals[k] = reinterpret_cast<unsigned*>(ik + align_up(cap * 4) * (2 + k));
+    }
+    // The heaviest-first orders: counts beside the tile counters; the lists in
+    // the tile sort's spare key buffer, which is free from the sort to the next
+    // forward (a buffer of their own where they do not fit).
+    b->heavy = b->work = StripOrder{};
+    if (sc.schedule == kSchedHeavyFirst) {
+        const size_t words = kWorkClasses * (tiles + b->strips);
+        const int sorted = cap > 1 ? radix_plan(b->tile_bits).passes & 1 : 0;
+        unsigned* lists = words <= cap ? b->ikeys[sorted ^ 1]
+                                       : reinterpret_cast<unsigned*>(
+                                             b->order_buf.exact(words * sizeof(unsigned), st));
+        unsigned* counts = reinterpret_cast<unsigned*>(b->tile_ctr_buf.p) + 64;
+        b->heavy = {counts, lists, unsigned(tiles)};
+        b->work = {counts + kWorkClasses, lists + kWorkClasses * tiles, unsigned(b->strips)};
     }
     const size_t status = std::max({sort_status_bytes(pairs, radix_plan(32)),
                                     sort_status_bytes(cap, radix_plan(b->tile_bits)),
