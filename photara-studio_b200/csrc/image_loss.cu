@@ -9,11 +9,14 @@
 //
 // B200 organisation: one pass over the pixels does both kernels' work. The
 // reference scatters the consistency term's depth gradient into the four
-// neighbours with atomics; here every pixel gathers what its four neighbours
-// would scatter into it (their depth normals are recomputed from depths that
-// the neighbouring threads read anyway), so the gradient images are written
-// once, without atomics, and the result is deterministic. The loss terms are
-// reduced per block and then in one fixed-order pass (double), instead of
+// neighbours with atomics; here a block works out its 32 x 8 tile's depth
+// normals and a ring of one pixel around them once, in shared memory, and every
+// pixel gathers what its four neighbours would scatter into it, so the gradient
+// images are written once, without atomics, and the result is deterministic.
+// Bound: the latency of the image loads. Full HD with every term 94 -> 89 us
+// (before, each pixel recomputed its four neighbours' normals: 1.33 instead of 5
+// evaluations a pixel now). The loss terms are reduced per block and then in one
+// fixed-order pass (double; 1,024 threads, 9.7 -> 5.7 us against 256), instead of
 // one global atomic per pixel and term. Per-pixel arithmetic is the
 // reference's, expression for expression.
 #include <cuda_runtime.h>
@@ -26,6 +29,9 @@ namespace gsb {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kTw = 32, kTh = 8; // pixels of a block
+constexpr int kRw = kTw + 2, kRh = kTh + 2; // with the ring of one
+static_assert(kTw * kTh == kThreads);
 
 struct LossArgs {
     ImageLossImages im;
@@ -99,11 +105,33 @@ __device__ __forceinline__ DepthNormal depth_normal_at(const LossArgs& a, int x,
 
 __global__ void __launch_bounds__(kThreads) image_loss_kernel(LossArgs a) {
     __shared__ float s_terms[kThreads / 32][4];
+    // per pixel of the tile and its ring: d term / d (vertical, horizontal
+    // difference), zero where the term does not apply; loss and surface normal
+    __shared__ float3 s_dy[kRh * kRw], s_dx[kRh * kRw], s_n[kRh * kRw];
+    __shared__ float s_loss[kRh * kRw];
     const size_t pixels = size_t(a.im.width) * a.im.height;
-    const size_t pixel = size_t(blockIdx.x) * kThreads + threadIdx.x;
+    const int x0 = int(blockIdx.x) * kTw, y0 = int(blockIdx.y) * kTh;
+    const int tx0 = int(threadIdx.x) % kTw, ty0 = int(threadIdx.x) / kTw;
+    const int x = x0 + tx0, y = y0 + ty0;
+    const size_t pixel = size_t(y) * a.im.width + x;
+    const ImageLossOptions& o = a.o;
+    const bool consistency =
+        o.depth_normal_weight > 0.f && a.out.grad_depth && a.out.grad_normal;
+    const float normalization = o.depth_normal_weight / float(pixels);
+    if (consistency) {
+        for (int k = threadIdx.x; k < kRh * kRw; k += kThreads) {
+            const DepthNormal r =
+                depth_normal_at(a, x0 + k % kRw - 1, y0 + k / kRw - 1, normalization);
+            const float3 zero = make_float3(0.f, 0.f, 0.f);
+            s_dy[k] = r.ok ? r.grad_dy : zero;
+            s_dx[k] = r.ok ? r.grad_dx : zero;
+            s_n[k] = r.ok ? r.normal : zero;
+            s_loss[k] = r.ok ? r.loss : 0.f;
+        }
+        __syncthreads();
+    }
     float t_rgb = 0.f, t_depth = 0.f, t_normal = 0.f, t_alpha = 0.f;
-    if (pixel < pixels) {
-        const ImageLossOptions& o = a.o;
+    if (x < a.im.width && y < a.im.height) {
         const float valid = o.mask_enabled ? a.im.mask[pixel] : 1.f;
         const float inverse_pixels = 1.f / float(pixels);
         // colour L1 (its value only when the fused SSIM kernel does not run)
@@ -172,33 +200,18 @@ __global__ void __launch_bounds__(kThreads) image_loss_kernel(LossArgs a) {
         }
         // depth-normal consistency: this pixel's own term and what its four
         // neighbours' terms send to its depth
-        const bool consistency = o.depth_normal_weight > 0.f && a.out.grad_depth &&
-                                 a.out.grad_normal;
         if (consistency) {
-            const int W = a.im.width;
-            const int x = int(pixel % W), y = int(pixel / W);
-            const float normalization = o.depth_normal_weight / float(pixels);
-            const DepthNormal self = depth_normal_at(a, x, y, normalization);
-            if (self.ok) {
-                t_normal += self.loss;
-                grad_normal.x += -normalization * self.normal.x;
-                grad_normal.y += -normalization * self.normal.y;
-                grad_normal.z += -normalization * self.normal.z;
-            }
+            const int k = (ty0 + 1) * kRw + tx0 + 1;
+            t_normal += s_loss[k];
+            grad_normal.x += -normalization * s_n[k].x;
+            grad_normal.y += -normalization * s_n[k].y;
+            grad_normal.z += -normalization * s_n[k].z;
             const float fx = a.im.fx, fy = a.im.fy, cx = a.im.cx, cy = a.im.cy;
             const float3 ray = make_float3((float(x) - cx) / fx, (float(y) - cy) / fy, 1.f);
-            const DepthNormal above = depth_normal_at(a, x, y - 1, normalization); // we are its bottom
-            if (above.ok)
-                grad_depth += dot3(above.grad_dy, ray);
-            const DepthNormal below = depth_normal_at(a, x, y + 1, normalization); // we are its top
-            if (below.ok)
-                grad_depth += -dot3(below.grad_dy, ray);
-            const DepthNormal left = depth_normal_at(a, x - 1, y, normalization); // we are its right
-            if (left.ok)
-                grad_depth += dot3(left.grad_dx, ray);
-            const DepthNormal right = depth_normal_at(a, x + 1, y, normalization); // we are its left
-            if (right.ok)
-                grad_depth += -dot3(right.grad_dx, ray);
+            grad_depth += dot3(s_dy[k - kRw], ray);  // we are the bottom of the one above
+            grad_depth += -dot3(s_dy[k + kRw], ray); // the top of the one below
+            grad_depth += dot3(s_dx[k - 1], ray);    // the right of the one to the left
+            grad_depth += -dot3(s_dx[k + 1], ray);   // the left of the one to the right
         }
         a.out.grad_alpha[pixel] = grad_alpha;
         if (a.out.grad_depth)
@@ -226,21 +239,22 @@ __global__ void __launch_bounds__(kThreads) image_loss_kernel(LossArgs a) {
         float s = 0.f;
         for (int w = 0; w < kThreads / 32; ++w)
             s += s_terms[w][threadIdx.x];
-        a.partial[size_t(blockIdx.x) * 4 + threadIdx.x] = s;
+        a.partial[(size_t(blockIdx.y) * gridDim.x + blockIdx.x) * 4 + threadIdx.x] = s;
     }
 }
 
 // terms[k] += sum over blocks of partial[block][k], in a fixed order (double).
-__global__ void reduce_terms_kernel(const float* __restrict__ partial, int blocks,
-                                    float* __restrict__ terms) {
-    __shared__ double s[4][64];
-    const int k = threadIdx.x >> 6, lane = threadIdx.x & 63;
+__global__ void __launch_bounds__(1024) reduce_terms_kernel(const float* __restrict__ partial,
+                                                            int blocks,
+                                                            float* __restrict__ terms) {
+    __shared__ double s[4][256];
+    const int k = threadIdx.x & 3, lane = threadIdx.x >> 2;
     double v = 0.0;
-    for (int b = lane; b < blocks; b += 64)
+    for (int b = lane; b < blocks; b += 256)
         v += partial[size_t(b) * 4 + k];
     s[k][lane] = v;
     __syncthreads();
-    for (int w = 32; w > 0; w >>= 1) {
+    for (int w = 128; w > 0; w >>= 1) {
         if (lane < w)
             s[k][lane] += s[k][lane + w];
         __syncthreads();
@@ -252,18 +266,17 @@ __global__ void reduce_terms_kernel(const float* __restrict__ partial, int block
 } // namespace
 
 size_t image_loss_partial_floats(int width, int height) {
-    return 4 * ((size_t(width) * height + kThreads - 1) / kThreads);
+    return 4 * size_t((width + kTw - 1) / kTw) * size_t((height + kTh - 1) / kTh);
 }
 
 cudaError_t launch_image_loss(cudaStream_t s, const ImageLossImages& im,
                               const ImageLossOptions& o, const ImageLossOutputs& out,
                               float photo_weight, float* partial) {
-    const size_t pixels = size_t(im.width) * im.height;
-    const int blocks = int((pixels + kThreads - 1) / kThreads);
+    const dim3 grid((im.width + kTw - 1) / kTw, (im.height + kTh - 1) / kTh);
     LossArgs a{im, o, out, photo_weight, out.terms ? partial : nullptr};
-    image_loss_kernel<<<blocks, kThreads, 0, s>>>(a);
+    image_loss_kernel<<<grid, kThreads, 0, s>>>(a);
     if (out.terms)
-        reduce_terms_kernel<<<1, 256, 0, s>>>(partial, blocks, out.terms);
+        reduce_terms_kernel<<<1, 1024, 0, s>>>(partial, int(grid.x * grid.y), out.terms);
     return cudaGetLastError();
 }
 
