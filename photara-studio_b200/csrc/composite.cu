@@ -169,19 +169,20 @@ void launch_composite_count_pairs(cudaStream_t s, int tiles, const uint2* ranges
 // probe depth is the product of the Gaussians' partial opacities there; 8
 // probes over a +-0.4 window around the seed, refined 5 times (the first two
 // refinements walk the tile's list up to the pixel's last contributor again,
-// the later ones the few Gaussians kept around the bracket), then linear
+// the later ones the Gaussians kept in front of and around the bracket), then linear
 // interpolation inside the final bracket.
 constexpr int kDepthSplit = 8;
 constexpr int kDepthRefinements = 5;
 constexpr float kDepthSeedWindow = 0.4f;
 constexpr float kDepthMinTransmittance = 0.45f;
 constexpr int kGeoThreads = kTileW * kTileH;
-// Gaussians kept per pixel around the second refinement's bracket (0.1 wide),
-// in thread-local memory. Forward with depth, us, before / keeping 24, 48, 64:
-// 500,000 at 1280x720 1,760 / 1,343, 1,134, 1,172; 50,000 dense at 1280x960
-// 2,295 / 2,334, 2,047, 2,004; 20,000 at 320x243 584 / 621, 320, 335 (with too
-// few, most blocks hold a pixel that has to walk its list again).
-constexpr int kNear = 64;
+// Gaussians kept per pixel in front of and around the second refinement's
+// bracket (0.1 wide), in thread-local memory. Forward with depth, us, five more
+// walks of the list / this: 500,000 at 1280x720 1,755 / 1,182; 50,000 dense at
+// 1280x960 2,285 / 1,952; 20,000 at 320x243 586 / 348; 200,000 at 700x500
+// 1,263 / 733 (with too few kept, most blocks hold a pixel that has to walk its
+// list again).
+constexpr int kNear = 96;
 
 __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
     const uint2* __restrict__ ranges, const unsigned* __restrict__ order, GaussianState st,
@@ -339,11 +340,11 @@ __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
             Tp[k] *= (ts > t_peak ? oma : omg) * rv;
         }
     };
-    auto begin = [&](bool first, float t) {
+    auto begin = [&](bool first) {
 #pragma unroll
         for (int k = 0; k <= S; ++k)
             if (first || (k > 0 && k < S))
-                Tp[k] = t;
+                Tp[k] = 1.f;
         interval = (depth_max - depth_min) * (1.f / float(S));
     };
     // Keeps the bracket of the probes around transmittance 0.5.
@@ -367,27 +368,21 @@ __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
         Tp[0] = lo_T;
         Tp[S] = hi_T;
     };
-    begin(true, 1.f);
+    begin(true);
     walk(in_range, [&](float alpha, float t, float rs) { probe(true, alpha, t, rs); });
     narrow(true);
-    // The second refinement's walk also sorts the Gaussians by its bracket,
-    // which holds all later probes: those 8 sigma or more behind it change
-    // nothing any more, those as far in front scale every probe, and the few
-    // left are kept. The later refinements and dT/dt then need no walk (five
-    // walks of the list before, and a sixth for dT/dt).
+    // The second refinement's walk also keeps the Gaussians that its bracket,
+    // which holds all later probes, does not lie 8 sigma or more in front of:
+    // those behind it change nothing any more. The later refinements and dT/dt
+    // then need no walk (five walks of the list before, and a sixth for dT/dt),
+    // and multiply the same factors in the same order.
     float near_alpha[kNear], near_peak[kNear], near_rs[kNear];
     int near_n = 0;
-    float front = 1.f;
-    begin(false, 1.f);
+    begin(false);
     walk(in_range, [&](float alpha, float t, float rs) {
         probe(false, alpha, t, rs);
-        const bool ball = rs > 0.f;
-        if (ball && (depth_max - t) * rs < -8.f)
+        if (rs > 0.f && (depth_max - t) * rs < -8.f)
             return;
-        if (ball && (depth_min - t) * rs > 8.f) {
-            front *= 1.f - alpha;
-            return;
-        }
         if (near_n < kNear) {
             near_alpha[near_n] = alpha;
             near_peak[near_n] = t;
@@ -401,7 +396,7 @@ __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
     const bool any_over = __syncthreads_or(in_range && !kept);
 #pragma unroll 1
     for (int r = 2; r < kDepthRefinements; ++r) {
-        begin(false, kept ? front : 1.f);
+        begin(false);
         if (in_range && kept)
             for (int k = 0; k < near_n; ++k)
                 probe(false, near_alpha[k], near_peak[k], near_rs[k]);
