@@ -178,10 +178,10 @@ constexpr float kDepthMinTransmittance = 0.45f;
 constexpr int kGeoThreads = kTileW * kTileH;
 // Gaussians kept per pixel in front of and around the second refinement's
 // bracket (0.1 wide), in thread-local memory. Forward with depth, us, five more
-// walks of the list / this: 500,000 at 1280x720 1,755 / 1,182; 50,000 dense at
-// 1280x960 2,285 / 1,952; 20,000 at 320x243 586 / 348; 200,000 at 700x500
-// 1,263 / 733 (with too few kept, most blocks hold a pixel that has to walk its
-// list again).
+// walks of the list / keeping 48, 64, 96, 128: 500,000 at 1280x720 1,755 /
+// 1,185, 1,177, 1,180, 1,177; 50,000 dense at 1280x960 2,285 / 2,364, 1,981,
+// 1,952-1,966, 1,977; 200,000 at 700x500 1,263 / 746, 744, 733, 733 (with too
+// few, most blocks hold a pixel that has to walk its list again).
 constexpr int kNear = 96;
 
 __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
