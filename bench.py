@@ -260,7 +260,7 @@ def max_over_ranks(v: float, world: int) -> float:
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of these
 # kernels on this workload, from one ncu capture of the same build (not
 # measured by this run); close to the algorithmic bytes, i.e. no re-reads.
-NCU_TRAFFIC_BYTES = {"gaussian_backward_adam": 1_070_964_634, "preprocess": 284_170_770}
+NCU_TRAFFIC_BYTES = {"gaussian_backward_adam": 1_207_971_584, "preprocess": 222_083_072}
 
 # FP32 work of the compositing kernels per evaluated (Gaussian, pixel) pair:
 # forward ~20 FP32 operations + 1 exponential, adjoint ~60 FP32 operations.
@@ -384,8 +384,7 @@ def roofline_entry(stage_ms, counts, n_gauss, peaks):
     # them visible, I instances):
     #  preprocess: every Gaussian reads its 44 B of structure parameters and
     #    writes radius and tile count (8 B); a visible one also reads its SH row
-    #    (192 B) and writes centre, conic, colour, depth key, alpha box and the
-    #    64-byte compositing record (116 B);
+    #    (192 B) and writes its 64-byte record and depth key (68 B);
     #  depth sort (compaction, passes, offset scan): the compaction reads every
     #    Gaussian's tile count and depth (8 B) and writes a visible one's key and
     #    id (8 B); each pass reads and writes key and id (16 B per visible); the
@@ -397,7 +396,7 @@ def roofline_entry(stage_ms, counts, n_gauss, peaks):
     #    bounds 16 B) read + written, 48 B gradient scratch read + written =
     #    1,064 B per Gaussian (culled ones too: their moments decay).
     alg = {
-        "preprocess": 52.0 * n + 308.0 * V,
+        "preprocess": 52.0 * n + 260.0 * V,
         "depth_sort": 8.0 * n + 8.0 * V + pd * 16.0 * V + 12.0 * V,
         "tile_sort": pt * 16.0 * I,
         "gaussian_backward_adam": 1064.0 * n,
