@@ -564,6 +564,7 @@ __global__ void __launch_bounds__(kBGBlock, 4) batch_gaussian_backward48_kernel(
 size_t batch_gaussian_backward_smem(int views) {
     return size_t(views) * sizeof(Camera) + size_t(2) * kBGBlock * kBShStride * sizeof(float);
 }
+constexpr size_t kBGSmemLimit = 227 * 1024; // a CTA's shared memory; neither kernel has static
 size_t batch_gaussian_backward48_smem(int views) {
     return size_t(views) * sizeof(Camera) + size_t(2) * kBGBlock * kBRowStride * sizeof(float);
 }
@@ -962,17 +963,17 @@ void plan(gs_batch* b, const gs_gaussians* g, const gs_camera* cams, int views,
     b->tile_ctr_buf.exact((64 + 2 * kWorkClasses) * sizeof(unsigned), st);
     b->scan_status_buf.exact(std::max<size_t>(scan_status_bytes(int(pairs)), 256), st);
     // the schedule's kernels: grid sizes and attributes
-    const size_t gsmem = batch_gaussian_backward_smem(views);
-    req(gsmem <= 227 * 1024, "too many views for the per-Gaussian backward");
-    const size_t gsmem48 = batch_gaussian_backward48_smem(views);
-    b->rows48_fits = gsmem48 <= 227 * 1024;
-    if (b->rows48_fits)
-        ck(cudaFuncSetAttribute(batch_gaussian_backward48_kernel,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, int(gsmem48)),
+    req(batch_gaussian_backward_smem(views) <= kBGSmemLimit,
+        "too many views for the per-Gaussian backward");
+    b->rows48_fits = batch_gaussian_backward48_smem(views) <= kBGSmemLimit;
+    // A function's limit, shared by every plan on the device: set to the most
+    // any plan may ask for, since a lower one would refuse the launches of a
+    // plan of more views.
+    for (const void* k : {reinterpret_cast<const void*>(batch_gaussian_backward_kernel),
+                          reinterpret_cast<const void*>(batch_gaussian_backward48_kernel)})
+        ck(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(kBGSmemLimit)),
            "smem attribute");
-    ck(cudaFuncSetAttribute(batch_gaussian_backward_kernel,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize, int(gsmem)),
-       "smem attribute");
     with_shape(sc.tile_w, sc.tile_h, b->px, [&]<int TW, int TH, int PX>() {
         const void* fk;
         const void* bk;
