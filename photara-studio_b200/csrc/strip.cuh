@@ -114,16 +114,28 @@ struct StripFeed {
 // columns and rows; the ellipse's rows over the strip's columns (the walk's
 // column interval, tiles.cuh:18-179) sharpen it for tilted ones. A NaN counts
 // as reaching.
+// Both are worked out in 32 bits, and for a tilted needle the determinant
+// cancels: with d = det / (xx zz), the box (from the covariance), det here and
+// the exponent of the per-pixel test are each off by some 2^-22 / d. Below
+// kNeedleDet every band counts as reached. Above it the errors stay under 5e-4
+// of an extent squared in all: the threshold is raised by 2e-3, and the box's
+// extents, at most 1,205 pixels (the covariance is capped), are within the
+// pixel that it is widened by. Without the rule aspects of 1,000 and more lost
+// blends (minor axis 0.05 pixels, aspect 3,000: 46 of 41,818 pixels).
+constexpr float kNeedleDet = 1.f / 1024.f;
+
 template <int TW, int PX>
 __device__ __forceinline__ unsigned strip_bands(const SplatRec& rec, int x0, int y0) {
     using G = StripGeom<TW, PX>;
     const float4 co = rec.co;
     const float2 m = rec.xy;
     const ushort4 box = rec.bounds;
+    const float det = co.x * co.z - co.y * co.y;
+    if (!(det > kNeedleDet * co.x * co.z))
+        return (1u << G::kBands) - 1u;
     if (int(box.x) - 1 >= x0 + TW || int(box.y) + 1 <= x0)
         return 0u;
-    const float det = co.x * co.z - co.y * co.y;
-    const float thr = 2.f * logf(co.w * 255.f);
+    const float thr = 2.004f * logf(co.w * 255.f);
     const float ex = sqrtf(thr * co.z / det), ey = sqrtf(thr * co.x / det);
     const float d0 = fmaxf(-ex, float(x0 - 1) - m.x), d1 = fminf(ex, float(x0 + TW) - m.x);
     const float r0 = sqrtf(fmaxf(0.f, co.z * thr - det * d0 * d0));

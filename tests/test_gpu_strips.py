@@ -96,3 +96,44 @@ def test_long_lists_in_segments_match_whole_lists(count, logit):
                      "refine_weight"):
             x, y = getattr(a, name).cpu().numpy(), getattr(b, name).cpu().numpy()
             assert rel_l2(y, x) <= drift + (1e-4 if name == "opacity_logits" else 1e-5), name
+
+
+@pytest.mark.parametrize("w,h", [(400, 300), (512, 530)])  # 475 and 1,088 tiles
+@pytest.mark.parametrize("minor,aspect", [(0.05, 3000), (0.02, 5000), (0.3, 1000), (0.3, 300),
+                                          (0.5, 70)])
+def test_needles_lose_no_blend(w, h, minor, aspect):
+    """Thin tilted Gaussians (minor axis in pixels), whose 32-bit ellipse has
+    lost its digits: every strip shape blends what the forward of the geometry
+    channels blends, which tests each pixel against the whole list, and both
+    adjoints walk all of it (with a map of ones the densify weights add up to
+    the rendered alpha: float32 terms of 1e-8 to 1, so 1e-6 of the sum)."""
+    n, z, f = 400, 4.0, 500.0
+    g = torch.Generator("cuda").manual_seed(aspect)
+    u = lambda *s: torch.rand(s, device="cuda", generator=g)
+    s = minor * z / f
+    scales = torch.tensor([s * aspect, s, s], device="cuda").log().expand(n, 3).contiguous()
+    q = torch.randn((n, 4), device="cuda", generator=g)
+    half = torch.tensor([0.45 * w * z / f, 0.45 * h * z / f, 0.25], device="cuda")
+    means = ((2 * u(n, 3) - 1) * half + torch.tensor([0.0, 0.0, z], device="cuda")).contiguous()
+    model = gsb.GaussianModel(means, scales, (q / q.norm(dim=1, keepdim=True)).contiguous(),
+                              torch.randn((n, 1), device="cuda", generator=g),
+                              0.3 * torch.randn((n, 16, 3), device="cuda", generator=g), 3)
+    identity = [1.0, 0, 0, 0, 0, 1.0, 0, 0, 0, 0, 1.0, 0, 0, 0, 0, 1.0]
+    cam = gsb.Camera(identity, [0.0, 0.0, 0.0], f, f, w / 2, h / 2, w, h)
+    ones = torch.ones((h, w), device="cuda")
+
+    def weights_add_up(rast, r, **grads):
+        got = rast.backward(model, r, torch.zeros_like(r.color), densify_map=ones, **grads)
+        total = float(r.alpha.double().sum())
+        assert abs(float(got.densify_weight_den.double().sum()) - total) <= 1e-6 * total
+
+    rast = gsb.Rasterizer()
+    whole = rast.forward(model, cam, gsb.RasterizeOptions(active_sh_degree=3, require_depth=True))
+    assert float(whole.alpha.max()) > 0.5
+    weights_add_up(rast, whole, grad_depth=torch.zeros_like(ones),
+                   grad_normal=torch.zeros_like(whole.color))
+    for ppt in (1, 2, 4, 8, None):
+        rast = gsb.Rasterizer(pixels_per_thread=ppt)
+        r = rast.forward(model, cam, gsb.RasterizeOptions(active_sh_degree=3))
+        assert torch.equal(r.color, whole.color) and torch.equal(r.alpha, whole.alpha), ppt
+        weights_add_up(rast, r)
