@@ -231,7 +231,7 @@ GS_API gs_status gs_debug_lookback_probe(gs_context* ctx, int which, unsigned sp
  * pairs the compositing kernels of the last colour training forward evaluate,
  * pairs_out[0] for the forward (pixel not yet saturated when its warp takes
  * the Gaussian), pairs_out[1] for the adjoint (Gaussian at or before the
- * pixel's last contributor); HOST array of 2. Re-renders the forward into
+ * last one taken while the pixel was open); HOST array of 2. Re-renders the forward into
  * color / alpha (identical images) with counting kernels and waits for them. */
 GS_API gs_status gs_debug_composite_pairs(gs_context* ctx, float* color, float* alpha,
                                           unsigned long long* pairs_out);

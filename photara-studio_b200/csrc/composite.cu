@@ -160,8 +160,8 @@ void launch_composite_count_pairs(cudaStream_t s, int tiles, const uint2* ranges
 // Forward with the median-depth and normal channels (render_forward.cu
 // :274-525, blend_tile<GEOMETRY = true>): one thread per pixel of a 16x16
 // tile. Pass 1 is the colour forward (the same per-pixel arithmetic as the
-// colour kernels, so colour, alpha, final transmittance and last contributor
-// are bit-identical to them) plus the alpha-weighted footprint normal and the
+// colour kernels, so colour, alpha and final transmittance are bit-identical to
+// them; the last contributor is the last one blended) plus the alpha-weighted footprint normal and the
 // depth seed (the ray-plane depth of the last Gaussian blended while the
 // transmittance was above 0.5). Pass 2 finds the depth at which the
 // transmittance along the ray crosses 0.5: each Gaussian is a 1D Gaussian

@@ -67,7 +67,8 @@ struct ViewTarget {
     float* color;        // [3][H][W]
     float* alpha;        // [H][W]
     float* pix_T;        // [H][W] final transmittance (NULL: inference only)
-    unsigned* pix_last;  // [H][W] 1 + position of the last blended instance
+    unsigned* pix_last;  // [H][W] 1 + position of the last instance taken while the pixel
+                         // was open: at or behind the last blended one, 0 if none was taken
 };
 
 struct ViewGrads {

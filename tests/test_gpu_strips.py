@@ -137,3 +137,18 @@ def test_needles_lose_no_blend(w, h, minor, aspect):
         r = rast.forward(model, cam, gsb.RasterizeOptions(active_sh_degree=3))
         assert torch.equal(r.color, whole.color) and torch.equal(r.alpha, whole.alpha), ppt
         weights_add_up(rast, r)
+
+
+@pytest.mark.parametrize("ppt", [1, 2, 4, 8, None])
+def test_a_clip_below_the_blend_threshold_blends_and_adjoins_nothing(ppt):
+    """Every opacity is clipped to 0.003 < 1/255: no Gaussian is blended, so
+    none has a last contributor or a gradient."""
+    scene = gsb.make_scene("tiny", seed=3)
+    model, cam = device_model(scene), camera_of(scene)
+    rast = gsb.Rasterizer(pixels_per_thread=ppt)
+    r = rast.forward(model, cam, gsb.RasterizeOptions(
+        active_sh_degree=3, rasterization=gsb.RasterizationPolicy(alpha_clip=0.003)))
+    assert r.rendered_instances > 0 and not bool(r.alpha.any()) and not bool(r.visibility.any())
+    g = rast.backward(model, r, torch.ones_like(r.color), torch.ones_like(r.alpha))
+    for name in ("means", "log_scales", "quaternions", "opacity_logits", "sh", "refine_weight"):
+        assert not bool(getattr(g, name).any()), name
