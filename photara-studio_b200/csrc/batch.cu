@@ -64,6 +64,7 @@ enum BatchCounter : int {
     kBcTotal = 6,     // scan total
     kBcSorted = 7,    // min(instances, capacity): count for the tile sort
     kBcTiles = 8,     // total tiles
+    kBcWild = 9,      // a visible pair's colour is not finite
     kBcInstances64 = 10, // words 10-11: instances requested by the preprocess (u64)
     kBcWords = 16
 };
@@ -109,6 +110,8 @@ __global__ void __launch_bounds__(kBlock) batch_preprocess_kernel(
     const int warp0 = int(threadIdx.x) & ~31;
     store_records(s_rec + warp0, touched > 0, rec,
                   st.rec + size_t(v) * size_t(n) + blockIdx.x * blockDim.x + warp0);
+    if (touched > 0 && !finite_colour(rec.rgb))
+        atomicOr(&counters[kBcWild], 1u);
     const unsigned w_inst = __reduce_add_sync(0xffffffffu, touched);
     const unsigned w_vis = __popc(__ballot_sync(0xffffffffu, touched > 0));
     if (lane_id() == 0 && w_vis) {
@@ -214,12 +217,16 @@ __device__ __forceinline__ unsigned next_item(unsigned& k, unsigned* queue) {
 template <int PX> constexpr int kBatchForwardCtas = PX == 8 ? 20 : PX == 4 ? 28 : 32;
 template <int PX> constexpr int kBatchBackwardCtas = PX == 8 ? 16 : PX == 4 ? 20 : 24;
 
-template <int TW, int TH, int PX, int SCHED>
+// kGuard: with the guarded blend; *wild says which of the two kernels runs.
+template <int TW, int TH, int PX, int SCHED, bool kGuard>
 __global__ void __launch_bounds__(32, kBatchForwardCtas<PX>) batch_forward_kernel(
     const __grid_constant__ CUtensorMap map, unsigned* __restrict__ err, unsigned tiles,
     const uint2* __restrict__ ranges, const unsigned* __restrict__ order, TileLookup L,
     unsigned* __restrict__ queue, float3 bg, float* __restrict__ color, float* __restrict__ alpha,
-    float* __restrict__ pix_T, unsigned* __restrict__ pix_last) {
+    float* __restrict__ pix_T, unsigned* __restrict__ pix_last,
+    const unsigned* __restrict__ wild) {
+    if (PX > 1 && (*wild != 0) != kGuard)
+        return;
     constexpr unsigned kStrips = TH / StripGeom<TW, PX>::kRows;
     __shared__ StripStage s;
     StripFeed feed{s, &map, err};
@@ -237,7 +244,7 @@ __global__ void __launch_bounds__(32, kBatchForwardCtas<PX>) batch_forward_kerne
         const size_t pb = bv.pix_base;
         const ViewTarget o{bv.K.width, bv.K.height, bv.K.alpha_clip, bg, color + 3 * pb,
                            alpha + pb, pix_T + pb, pix_last + pb};
-        if (!composite_forward_strip<TW, PX>(
+        if (!composite_forward_strip<TW, PX, false, false, kGuard>(
                 feed, int(local % gx) * TW,
                 int(local / gx) * TH + int(strip) * StripGeom<TW, PX>::kRows, ranges[tile], order,
                 o, nullptr, L.work, tile * kStrips + strip))
@@ -783,14 +790,19 @@ void enqueue_forward(gs_batch* b, float* color, float* alpha) {
                        kernel<<<b->grid_fwd, 32, 0, s>>>(
                            b->staging.map, b->staging.err, b->total_tiles, b->ranges,
                            b->ivals[b->inst_result], L, b->counters + kBcWork, bg, color, alpha,
-                           b->pix_T, b->pix_last);
+                           b->pix_T, b->pix_last, b->counters + kBcWild);
                    };
-                   if (b->sched.schedule == kSchedStatic)
-                       go(batch_forward_kernel<TW, TH, PX, kSchedStatic>);
-                   else if (b->sched.schedule == kSchedDynamic)
-                       go(batch_forward_kernel<TW, TH, PX, kSchedDynamic>);
-                   else
-                       go(batch_forward_kernel<TW, TH, PX, kSchedHeavyFirst>);
+                   auto either = [&]<bool kGuard>() {
+                       if (b->sched.schedule == kSchedStatic)
+                           go(batch_forward_kernel<TW, TH, PX, kSchedStatic, kGuard>);
+                       else if (b->sched.schedule == kSchedDynamic)
+                           go(batch_forward_kernel<TW, TH, PX, kSchedDynamic, kGuard>);
+                       else
+                           go(batch_forward_kernel<TW, TH, PX, kSchedHeavyFirst, kGuard>);
+                   };
+                   either.template operator()<false>();
+                   if constexpr (PX > 1)
+                       either.template operator()<true>();
                });
     ck(cudaGetLastError(), "batch forward launch");
 }
@@ -978,13 +990,13 @@ void plan(gs_batch* b, const gs_gaussians* g, const gs_camera* cams, int views,
         const void* fk;
         const void* bk;
         if (sc.schedule == kSchedStatic) {
-            fk = reinterpret_cast<const void*>(batch_forward_kernel<TW, TH, PX, kSchedStatic>);
+            fk = reinterpret_cast<const void*>(batch_forward_kernel<TW, TH, PX, kSchedStatic, false>);
             bk = reinterpret_cast<const void*>(batch_backward_kernel<TW, TH, PX, kSchedStatic>);
         } else if (sc.schedule == kSchedDynamic) {
-            fk = reinterpret_cast<const void*>(batch_forward_kernel<TW, TH, PX, kSchedDynamic>);
+            fk = reinterpret_cast<const void*>(batch_forward_kernel<TW, TH, PX, kSchedDynamic, false>);
             bk = reinterpret_cast<const void*>(batch_backward_kernel<TW, TH, PX, kSchedDynamic>);
         } else {
-            fk = reinterpret_cast<const void*>(batch_forward_kernel<TW, TH, PX, kSchedHeavyFirst>);
+            fk = reinterpret_cast<const void*>(batch_forward_kernel<TW, TH, PX, kSchedHeavyFirst, false>);
             bk = reinterpret_cast<const void*>(
                 batch_backward_kernel<TW, TH, PX, kSchedHeavyFirst>);
         }

@@ -54,7 +54,7 @@ struct gs_context {
     // workspace
     DevBuf gauss, grad, scan_status, counters, inst_keys, inst_vals, sort_hist, sort_status,
         sort_counters, ranges, pixel, depth_sort, loss, probe, geo_grad, rec, emit_groups, segment;
-    unsigned* host_counts = nullptr; // pinned [16]: [0, 8) draw counts, [8] error word after the sorts
+    unsigned* host_counts = nullptr; // pinned [16]: [0, 9) frame counters, [12] error word after the sorts
     size_t gauss_cap = 0, grad_cap = 0, inst_cap = 0, pixel_cap = 0, geo_grad_cap = 0;
     GaussianState st{};
     RecStaging staging{};     // tensor map of st.rec for the compositing kernels' TMA gathers
@@ -81,6 +81,7 @@ struct gs_context {
     float* pix_dtdt = nullptr; // dT/dt at the median depth (geometry training forwards)
     unsigned* work_lists = nullptr; // the last colour training forward's strips by adjoint work
     int work_px = 0;                // its pixels per thread (the strips' shape)
+    bool wild = false;              // a colour of the draw list may not be finite
     SegmentStore segments{};        // its checkpoints (levels 0: none kept)
     bool geometry = false;     // the last forward rendered the median-depth / normal channels
     const float* fwd_depth = nullptr;  // its median-depth and normal outputs (caller memory)
@@ -209,8 +210,8 @@ unsigned* device_error_word(gs_context* c) {
 // this while the compositing still runs) and refuses a list whose sort gave up.
 void check_forward_sorts(gs_context* c) {
     ck(cudaEventSynchronize(c->ev_sorted), "sort status sync");
-    if (c->host_counts[8])
-        raise_timeout(c, c->host_counts[8], "in the forward's sorts");
+    if (c->host_counts[12])
+        raise_timeout(c, c->host_counts[12], "in the forward's sorts");
 }
 
 const RecStaging& record_staging(gs_context* c) {
@@ -385,6 +386,7 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
         unsigned* counters = reinterpret_cast<unsigned*>(c->counters.p);
         // counters: [0] instances [1] visible [2] device error [3] scan tile counter
         //           [4] min depth bits [5] max depth bits [6] Gaussian count [7] scan total
+        //           [8] a visible Gaussian's colour is not finite
         launch_frame_counters_init(st, counters);
         const int prev_set = c->ev_set;
         const bool prev_pending = c->ev_pending && c->timing;
@@ -401,7 +403,7 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
                           out->radii, counters);
         ck(cudaGetLastError(), "preprocess launch");
         mark(c, 0, true);
-        ck(cudaMemcpyAsync(c->host_counts, counters, 8 * sizeof(unsigned), cudaMemcpyDeviceToHost,
+        ck(cudaMemcpyAsync(c->host_counts, counters, 9 * sizeof(unsigned), cudaMemcpyDeviceToHost,
                            st),
            "read draw counts");
         ck(cudaEventRecord(c->ev_counts, st), "count event");
@@ -450,6 +452,7 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
         const unsigned visible = c->host_counts[1];
         const unsigned dev_err = c->host_counts[2];
         const unsigned dmin = c->host_counts[4], dmax = c->host_counts[5];
+        c->wild = c->host_counts[8] != 0;
         if (dev_err)
             raise_timeout(c, dev_err, "before this forward's draw counts");
         req(instances < (1u << 30), "instance count exceeds 2^30");
@@ -506,11 +509,11 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
             // The error word of the compaction, depth sort, offset scan and
             // tile sort, for check_forward_sorts (4 bytes; the host waits on
             // it only where the draw list is consumed again).
-            ck(cudaMemcpyAsync(c->host_counts + 8, counters + 2, sizeof(unsigned),
+            ck(cudaMemcpyAsync(c->host_counts + 12, counters + 2, sizeof(unsigned),
                                cudaMemcpyDeviceToHost, st),
                "read sort status");
         } else {
-            c->host_counts[8] = 0;
+            c->host_counts[12] = 0;
             for (int k = 1; k <= 4; ++k) {
                 mark(c, k, false);
                 mark(c, k, true);
@@ -540,7 +543,7 @@ gs_status gs_forward(gs_context* c, const gs_gaussians* g, const gs_camera* cam,
             launch_composite_forward(st, tiles, reinterpret_cast<const uint2*>(c->ranges.p),
                                      c->vals[cur], K, bg, out->color, out->alpha, c->pix_T,
                                      c->pix_last, out->visibility, ppt, record_staging(c),
-                                     c->work_lists, &c->segments);
+                                     ColourGuard{c->wild}, c->work_lists, &c->segments);
         }
         ck(cudaGetLastError(), "composite launch");
         mark(c, 5, true);
@@ -896,15 +899,19 @@ gs_status gs_forward_colors(gs_context* c, const float* colors, const gs_outputs
         req(colors && out && out->color && out->alpha, "invalid colour reuse arguments");
         check_forward_sorts(c);
         const int n = c->g.count;
-        ck(launch_set_colors(c->stream, n, colors, c->st.rec), "colour slots");
+        unsigned* wild = reinterpret_cast<unsigned*>(c->counters.p) + 8;
+        ck(cudaMemsetAsync(wild, 0, sizeof(unsigned), c->stream), "colour flag");
+        ck(launch_set_colors(c->stream, n, colors, c->st.rec, wild), "colour slots");
         c->g.colors = colors;
+        c->wild = true; // not known here
         // empty tiles (ranges zeroed by the forward) composite the background;
         // the checkpoints' colours are written again
         launch_composite_forward(c->stream, c->tiles, reinterpret_cast<const uint2*>(c->ranges.p),
                                  c->vals[c->sorted_buf], c->K, c->bg, out->color, out->alpha,
                                  c->pix_T, c->pix_last, out->visibility,
                                  c->work_lists ? c->work_px : compositing_px(c, c->tiles),
-                                 record_staging(c), nullptr, &c->segments);
+                                 record_staging(c), ColourGuard{false, wild}, nullptr,
+                                 &c->segments);
         ck(cudaGetLastError(), "colour reuse composite launch");
     });
 }
@@ -923,7 +930,7 @@ gs_status gs_pruning_scores(gs_context* c, const float* image, int gaussian_pop,
             return; // nothing drawn: no score
         ck(launch_pruning_scores(c->stream, c->tiles, reinterpret_cast<const uint2*>(c->ranges.p),
                                  c->vals[c->sorted_buf], c->K, c->pix_last, image,
-                                 gaussian_pop ? 1 : 0, scores, record_staging(c)),
+                                 gaussian_pop ? 1 : 0, scores, record_staging(c), c->wild),
            "pruning score launch");
     });
 }

@@ -35,6 +35,10 @@ struct __align__(16) SplatRec {
 };
 static_assert(sizeof(SplatRec) == 64, "one TMA row per record");
 
+// Whether a colour's channels are finite (a false "no" where their sum
+// overflows does no harm: it only selects a slower kernel).
+__device__ __forceinline__ bool finite_colour(float4 c) { return isfinite(c.x + c.y + c.z); }
+
 // Per-Gaussian forward state (structure of arrays, one slot per Gaussian).
 struct GaussianState {
     SplatRec* rec;      // centre, conic, colour, box and tile walk

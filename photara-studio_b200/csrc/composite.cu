@@ -16,21 +16,25 @@ template <int PX> constexpr int kBackwardCtas = PX == 8 ? 16 : PX == 4 ? 20 : 24
 
 // One warp per strip of a reference 16x16 tile (256 / (32 PX) strips per
 // tile). kCount: the same forward that also counts its evaluated pairs. kSeg:
-// it stores the adjoint's checkpoints.
-template <int PX, bool kCount = false, bool kSeg = false>
+// it stores the adjoint's checkpoints. kGuard: with the guarded blend. wild
+// (may be NULL): the device word that says which of the two kernels runs.
+template <int PX, bool kCount = false, bool kSeg = false, bool kGuard = false>
 __global__ void __launch_bounds__(32, kForwardCtas<PX>) composite_forward_kernel(
     const __grid_constant__ CUtensorMap map, unsigned* __restrict__ err,
     const uint2* __restrict__ ranges, const unsigned* __restrict__ order, const Camera K,
     float3 bg, float* __restrict__ out_color, float* __restrict__ out_alpha,
     float* __restrict__ pix_T, unsigned* __restrict__ pix_last, float* __restrict__ visibility,
-    StripOrder sched, Checkpoints cp, unsigned long long* __restrict__ pairs = nullptr) {
+    StripOrder sched, Checkpoints cp, const unsigned* __restrict__ wild,
+    unsigned long long* __restrict__ pairs = nullptr) {
+    if (wild && (*wild != 0) != kGuard)
+        return;
     constexpr int kStrips = kTileH / StripGeom<kTileW, PX>::kRows;
     __shared__ StripStage s;
     StripFeed feed{s, &map, err};
     feed.init();
     const int tile = int(blockIdx.x) / kStrips, strip = int(blockIdx.x) % kStrips;
     const ViewTarget o{K.width, K.height, K.alpha_clip, bg, out_color, out_alpha, pix_T, pix_last};
-    composite_forward_strip<kTileW, PX, kCount, kSeg>(
+    composite_forward_strip<kTileW, PX, kCount, kSeg, kGuard>(
         feed, (tile % K.grid_x) * kTileW,
         (tile / K.grid_x) * kTileH + strip * StripGeom<kTileW, PX>::kRows, ranges[tile], order, o,
         visibility, sched, blockIdx.x, pairs, &cp, tile);
@@ -141,7 +145,7 @@ void launch_composite_count_pairs(cudaStream_t s, int tiles, const uint2* ranges
         const int blocks = tiles * (8 / PX);
         composite_forward_kernel<PX, true><<<blocks, 32, 0, s>>>(
             rs.map, rs.err, ranges, order, K, bg, color, alpha, nullptr, nullptr, nullptr, {}, {},
-            pairs);
+            nullptr, pairs);
         composite_backward_kernel<PX, false, false, true><<<blocks, 32, 0, s>>>(
             rs.map, rs.err, ranges, order, st.grad, K, bg, pix_T, pix_last, color, nullptr,
             nullptr, {}, pairs + 1);
@@ -774,8 +778,8 @@ void launch_composite_backward_geometry(cudaStream_t s, int tiles, const uint2* 
 void launch_composite_forward(cudaStream_t s, int tiles, const uint2* ranges,
                               const unsigned* order, const Camera& K, float3 bg, float* color,
                               float* alpha, float* pix_T, unsigned* pix_last, float* visibility,
-                              int pixels_per_thread, const RecStaging& rs, unsigned* work_lists,
-                              const SegmentStore* segments) {
+                              int pixels_per_thread, const RecStaging& rs, ColourGuard guard,
+                              unsigned* work_lists, const SegmentStore* segments) {
     const bool seg = segments && segments->levels > 0;
     const StripOrder sched = strip_order(seg ? nullptr : work_lists, tiles, pixels_per_thread);
     const Checkpoints cp = seg ? Checkpoints{segments->data, segments->tile_last, segments->levels}
@@ -784,12 +788,19 @@ void launch_composite_forward(cudaStream_t s, int tiles, const uint2* ranges,
         auto go = [&](auto kernel) {
             kernel<<<tiles * (8 / PX), 32, 0, s>>>(rs.map, rs.err, ranges, order, K, bg, color,
                                                    alpha, pix_T, pix_last, visibility, sched, cp,
-                                                   nullptr);
+                                                   PX > 1 ? guard.word : nullptr, nullptr);
+        };
+        auto either = [&]<bool kSeg>() {
+            if constexpr (PX > 1)
+                if (guard.on || guard.word)
+                    go(composite_forward_kernel<PX, false, kSeg, true>);
+            if (PX == 1 || !guard.on || guard.word)
+                go(composite_forward_kernel<PX, false, kSeg, false>);
         };
         if constexpr (PX <= 2)
             if (seg)
-                return go(composite_forward_kernel<PX, false, true>);
-        go(composite_forward_kernel<PX, false, false>);
+                return either.template operator()<true>();
+        either.template operator()<false>();
     };
     if (pixels_per_thread == 1)
         fwd.template operator()<1>();

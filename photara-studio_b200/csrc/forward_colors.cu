@@ -15,20 +15,24 @@ namespace gsb {
 namespace {
 
 __global__ void __launch_bounds__(256) set_colors_kernel(int n, const float* __restrict__ colors,
-                                                        SplatRec* __restrict__ rec) {
+                                                        SplatRec* __restrict__ rec,
+                                                        unsigned* __restrict__ wild) {
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i < n) {
         const float4 c = make_float4(colors[3 * size_t(i)], colors[3 * size_t(i) + 1],
                                      colors[3 * size_t(i) + 2], __uint_as_float(0u));
         rec[i].rgb = c;
+        if (!finite_colour(c))
+            atomicOr(wild, 1u);
     }
 }
 
 } // namespace
 
-cudaError_t launch_set_colors(cudaStream_t s, int n, const float* colors, SplatRec* rec) {
+cudaError_t launch_set_colors(cudaStream_t s, int n, const float* colors, SplatRec* rec,
+                              unsigned* wild) {
     if (n > 0)
-        set_colors_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, colors, rec);
+        set_colors_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, colors, rec, wild);
     return cudaGetLastError();
 }
 

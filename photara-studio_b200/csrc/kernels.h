@@ -241,11 +241,18 @@ struct SegmentStore {
     int levels = 0;                // 0: not used
 };
 constexpr int kWorkListZeroed = 64;
+// Whether a colour of the frame may not be finite, so that the forward takes the
+// guarded blend: known on the host (on), or in a device word, by which one of
+// two launches does the work.
+struct ColourGuard {
+    bool on = false;
+    const unsigned* word = nullptr;
+};
 size_t strip_order_words(int tiles, int pixels_per_thread);
 void launch_composite_forward(cudaStream_t s, int tiles, const uint2* ranges,
                               const unsigned* order, const Camera& K, float3 bg, float* color,
                               float* alpha, float* pix_T, unsigned* pix_last, float* visibility,
-                              int pixels_per_thread, const RecStaging& rs,
+                              int pixels_per_thread, const RecStaging& rs, ColourGuard guard,
                               unsigned* work_lists = nullptr,
                               const SegmentStore* segments = nullptr);
 // Fused L1 + SSIM loss: grad += dL/dpred, *loss_out (may be NULL) = L;
@@ -370,9 +377,11 @@ void launch_composite_backward(cudaStream_t s, int tiles, const uint2* ranges,
 cudaError_t launch_pruning_scores(cudaStream_t s, int tiles, const uint2* ranges,
                                   const unsigned* order, const Camera& K,
                                   const unsigned* pix_last, const float* image, int gaussian_pop,
-                                  float* scores, const RecStaging& rs);
+                                  float* scores, const RecStaging& rs, bool guard);
 
-cudaError_t launch_set_colors(cudaStream_t s, int n, const float* colors, SplatRec* rec);
+// *wild (zeroed before): set if a colour is not finite.
+cudaError_t launch_set_colors(cudaStream_t s, int n, const float* colors, SplatRec* rec,
+                              unsigned* wild);
 
 size_t gaussian_backward_smem(bool fused_sh);
 void launch_gaussian_backward(cudaStream_t s, int n, const float* means, const float* log_scales,

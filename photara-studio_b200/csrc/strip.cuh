@@ -180,6 +180,26 @@ __device__ __forceinline__ unsigned strip_masks(const SplatRec* rec, int cnt, in
     return any;
 }
 
+// A pixel that does not blend a Gaussian multiplies its values by zero, which
+// an infinity or a NaN would turn into a NaN there. Frames with a colour that is
+// not finite (finite_colour, in the preprocess) take a forward with the guarded blend, a
+// kernel of its own: both in one slowed the other down (1M / 1080p 217 -> 230
+// us, by registers and code that the plain loop then shares).
+// The adjoint takes guarded steps in batches with a colour, and strips with a
+// gradient, that is not below this bound (products of two such values and an image's size stay
+// finite).
+constexpr float kTame = 1e15f;
+
+__device__ __forceinline__ bool tame(float a, float b, float c) {
+    return fabsf(a) + fabsf(b) + fabsf(c) < kTame;
+}
+
+// Whether the batch's colours are all below the bound.
+__device__ __forceinline__ bool tame_colours(const SplatRec* rec, int cnt) {
+    const float4 c = rec[min(int(lane_id()), cnt - 1)].rgb;
+    return __all_sync(0xffffffffu, tame(c.x, c.y, c.z));
+}
+
 // Strips by their adjoint work, heaviest first: the forward appends each strip
 // to the list of its work class (four classes per power of two, so within a
 // quarter of each other) and the adjoint's blocks take the classes in
@@ -270,12 +290,13 @@ __device__ __forceinline__ float2 pair_alpha(float4 co, float dx, float xx, floa
 // Selects on values instead of flags kept across the pairs: eight pixels'
 // flags exceed the predicate registers and were moved through general ones
 // (179 ALU instructions per visit of a whole tile).
-// kSeg: also adds the blend to the segment's colour sums.
+// kSeg: also adds the blend to the segment's colour sums. kGuard: the colour
+// reaches the pixels that blend it only (see finite_colour).
 struct SegSums {
     float2 r, g, b;
 };
 
-template <bool kSeg>
+template <bool kSeg, bool kGuard>
 __device__ __forceinline__ int pair_blend(float2 a, float4 c, unsigned pos, float2& T, float2& r,
                                           float2& g, float2& b, unsigned& la, unsigned& lb,
                                           SegSums& seg) {
@@ -283,13 +304,16 @@ __device__ __forceinline__ int pair_blend(float2 a, float4 c, unsigned pos, floa
     const bool ba = !(tt.x < kTransmittanceFloor);
     const bool bb = !(tt.y < kTransmittanceFloor);
     const float2 w = __fmul2_rn(f2(ba ? a.x : 0.f, bb ? a.y : 0.f), T);
-    r = __ffma2_rn(f2s(c.x), w, r);
-    g = __ffma2_rn(f2s(c.y), w, g);
-    b = __ffma2_rn(f2s(c.z), w, b);
+    auto at = [&](float v) {
+        return kGuard ? f2(w.x > 0.f ? v : 0.f, w.y > 0.f ? v : 0.f) : f2s(v);
+    };
+    r = __ffma2_rn(at(c.x), w, r);
+    g = __ffma2_rn(at(c.y), w, g);
+    b = __ffma2_rn(at(c.z), w, b);
     if constexpr (kSeg) {
-        seg.r = __ffma2_rn(f2s(c.x), w, seg.r);
-        seg.g = __ffma2_rn(f2s(c.y), w, seg.g);
-        seg.b = __ffma2_rn(f2s(c.z), w, seg.b);
+        seg.r = __ffma2_rn(at(c.x), w, seg.r);
+        seg.g = __ffma2_rn(at(c.y), w, seg.g);
+        seg.b = __ffma2_rn(at(c.z), w, seg.b);
     }
     T.x = ba ? tt.x : -fabsf(T.x);
     T.y = bb ? tt.y : -fabsf(T.y);
@@ -303,8 +327,9 @@ __device__ __forceinline__ int pair_blend(float2 a, float4 c, unsigned pos, floa
 // alpha test runs on a pixel that has not ended, for the roofline figures.
 // sched (count may be NULL): receives the strip (index `strip`) with its
 // adjoint work. False: the staging gave up (the strip was not written).
-// kSeg: stores the checkpoints and adds the strip to tile_last[tile].
-template <int TW, int PX, bool kCount = false, bool kSeg = false>
+// kSeg: stores the checkpoints and adds the strip to tile_last[tile]. kGuard:
+// the guarded blend (one pixel per thread guards its blend anyway).
+template <int TW, int PX, bool kCount = false, bool kSeg = false, bool kGuard = false>
 __device__ __forceinline__ bool composite_forward_strip(
     StripFeed& feed, int x0, int y0, uint2 range, const unsigned* __restrict__ order,
     const ViewTarget& o, float* __restrict__ visibility, const StripOrder& sched, unsigned strip,
@@ -417,13 +442,15 @@ __device__ __forceinline__ bool composite_forward_strip(
                     const bool bl = !(tt < kTransmittanceFloor);
                     const float w = (bl ? a[u] : 0.f) * T[0].x;
                     const float4 c = rec[j[u]].rgb;
-                    r[0].x += c.x * w;
-                    g[0].x += c.y * w;
-                    b[0].x += c.z * w;
-                    if constexpr (kSeg) {
-                        seg[0].r.x += c.x * w;
-                        seg[0].g.x += c.y * w;
-                        seg[0].b.x += c.z * w;
+                    if (w > 0.f) {
+                        r[0].x += c.x * w;
+                        g[0].x += c.y * w;
+                        b[0].x += c.z * w;
+                        if constexpr (kSeg) {
+                            seg[0].r.x += c.x * w;
+                            seg[0].g.x += c.y * w;
+                            seg[0].b.x += c.z * w;
+                        }
                     }
                     T[0].x = bl ? tt : -fabsf(T[0].x);
                     la[0] = bl ? unsigned(base + j[u] + 1) : la[0];
@@ -458,13 +485,13 @@ __device__ __forceinline__ bool composite_forward_strip(
                         e[p] = pair_alpha(co, dx, xx, nxy, __fadd2_rn(f2s(xy.y), nfy[p]), clip);
 #pragma unroll
                     for (int p = 0; p < NP; ++p)
-                        bl |= pair_blend<kSeg>(e[p], c, pos, T[p], r[p], g[p], b[p], la[p], lb[p],
-                                               seg[p]);
+                        bl |= pair_blend<kSeg, kGuard>(e[p], c, pos, T[p], r[p], g[p], b[p], la[p],
+                                                       lb[p], seg[p]);
                 } else {
 #pragma unroll
                     for (int p = 0; p < NP; ++p)
                         if ((mask[p] >> j) & 1u)
-                            bl |= pair_blend<kSeg>(
+                            bl |= pair_blend<kSeg, kGuard>(
                                 pair_alpha(co, dx, xx, nxy, __fadd2_rn(f2s(xy.y), nfy[p]), clip),
                                 c, pos, T[p], r[p], g[p], b[p], la[p], lb[p], seg[p]);
                 }
@@ -558,8 +585,10 @@ struct PairState {
 // leaving its state unchanged and adding zero. Opacities and colours enter
 // negated (nco = -o, nc = -c), so every difference is one multiply-add; the
 // colour and densify sums come out negated (slot_scale). ra, rb, rc, rd: the
-// mean gradient's norm is |s| |(ra + rb dy, rc + rd dy)|.
-template <bool kRefine, bool kDensify, bool kFirst>
+// mean gradient's norm is |s| |(ra + rb dy, rc + rd dy)|. kGuard: nothing of
+// the Gaussian or of the pixel's gradients reaches an element that does not
+// blend it (see kTame).
+template <bool kRefine, bool kDensify, bool kFirst, bool kGuard = false>
 __device__ __forceinline__ void pair_adjoint(PairState& p, unsigned pos, float4 co, float nco,
                                              float3 nc, float dx, float xx, float nxy, float2 dy,
                                              float clip, float ra, float rb, float rc, float rd,
@@ -572,15 +601,16 @@ __device__ __forceinline__ void pair_adjoint(PairState& p, unsigned pos, float4 
     const float2 nal = f2(fmaxf(-clip, nog.x), fmaxf(-clip, nog.y));
     const float2 oma = __fadd2_rn(f2s(1.f), nal);
     const float2 inv = f2(1.f / oma.x, 1.f / oma.y);
-    const float2 ncdot =
-        __ffma2_rn(f2s(nc.z), p.gz, __ffma2_rn(f2s(nc.y), p.gy, __fmul2_rn(f2s(nc.x), p.gx)));
+    auto hit = [&](float2 v) { return kGuard ? f2(ha ? v.x : 0.f, hb ? v.y : 0.f) : v; };
+    const float2 ncdot = hit(
+        __ffma2_rn(f2s(nc.z), p.gz, __ffma2_rn(f2s(nc.y), p.gy, __fmul2_rn(f2s(nc.x), p.gx))));
     // -dL/dalpha = (S - T_behind c.g) / (1 - alpha), S the colour behind
     // (background included) along the gradient
     const float2 nda = __fmul2_rn(inv, __ffma2_rn(p.T, ncdot, p.sdot));
     p.T = __fmul2_rn(p.T, inv);
     const float2 nw = __fmul2_rn(nal, p.T);
     p.sdot = __ffma2_rn(nw, ncdot, p.sdot);
-    const float2 s = __fmul2_rn(nog, nda);
+    const float2 s = hit(__fmul2_rn(nog, nda));
     const float2 sy = __fmul2_rn(s, dy);
     acc.s = kFirst ? s : __fadd2_rn(acc.s, s);
     acc.sy = kFirst ? sy : __fadd2_rn(acc.sy, sy);
@@ -592,11 +622,11 @@ __device__ __forceinline__ void pair_adjoint(PairState& p, unsigned pos, float4 
         const float2 nrm = f2(sqrtf(q.x), sqrtf(q.y));
         acc.refine = kFirst ? __fmul2_rn(nrm, p.rscale) : __ffma2_rn(nrm, p.rscale, acc.refine);
     }
-    acc.cr = kFirst ? __fmul2_rn(nw, p.gx) : __ffma2_rn(nw, p.gx, acc.cr);
-    acc.cg = kFirst ? __fmul2_rn(nw, p.gy) : __ffma2_rn(nw, p.gy, acc.cg);
-    acc.cb = kFirst ? __fmul2_rn(nw, p.gz) : __ffma2_rn(nw, p.gz, acc.cb);
+    acc.cr = kFirst ? __fmul2_rn(nw, p.gx) : __ffma2_rn(nw, hit(p.gx), acc.cr);
+    acc.cg = kFirst ? __fmul2_rn(nw, p.gy) : __ffma2_rn(nw, hit(p.gy), acc.cg);
+    acc.cb = kFirst ? __fmul2_rn(nw, p.gz) : __ffma2_rn(nw, hit(p.gz), acc.cb);
     if constexpr (kDensify) {
-        acc.dn = kFirst ? __fmul2_rn(p.dmap, nw) : __ffma2_rn(p.dmap, nw, acc.dn);
+        acc.dn = kFirst ? __fmul2_rn(p.dmap, nw) : __ffma2_rn(hit(p.dmap), nw, acc.dn);
         acc.dd = kFirst ? nw : __fadd2_rn(acc.dd, nw);
     }
 }
@@ -770,6 +800,13 @@ __device__ __forceinline__ bool composite_backward_strip(
     const int slot = kDensify ? strip_slot12() : strip_slot10();
     const float scale = slot_scale(slot);
     float* const row = reinterpret_cast<float*>(grad) + max(slot, 0);
+    bool calm = true;
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+        calm = calm && tame(st[p].gx.x, st[p].gy.x, st[p].gz.x) &&
+               tame(st[p].gx.y, st[p].gy.y, st[p].gz.y) &&
+               tame(st[p].sdot.x, st[p].sdot.y, 0.f) && tame(st[p].dmap.x, st[p].dmap.y, 0.f);
+    calm = __all_sync(full, calm);
     unsigned long long evaluated = 0;
     int base = (total - 1) / kStripBatch * kStripBatch;
     unsigned id_next = feed.issue(0, order, range.x + unsigned(base), total - base);
@@ -813,7 +850,7 @@ __device__ __forceinline__ bool composite_backward_strip(
             PairState& t = st[0];
             while (m) {
                 int j[U];
-                bool ok[U];
+                bool ok[U]; // then: the pixel blends it
                 float dx[U], dy[U], og[U], v[U][12];
                 float4 co[U];
 #pragma unroll
@@ -830,17 +867,19 @@ __device__ __forceinline__ bool composite_backward_strip(
                     dy[u] = xy.y + nfy[0].x;
                     const float power = gaussian_power(co[u], dx[u], dy[u]);
                     og[u] = co[u].w * expf(power);
-                    const bool hit = ok[u] && unsigned(base + j[u]) < t.la && !(power > 0.f) &&
-                                     !(fminf(clip, og[u]) < kAlphaFloor);
-                    og[u] = hit ? og[u] : 0.f;
+                    ok[u] = ok[u] && unsigned(base + j[u]) < t.la && !(power > 0.f) &&
+                            !(fminf(clip, og[u]) < kAlphaFloor);
+                    og[u] = ok[u] ? og[u] : 0.f;
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const float4 c = rec[j[u]].rgb;
                     const float al = fminf(clip, og[u]);
                     const float inv = 1.f / (1.f - al);
-                    const float cdot = c.x * t.gx.x + c.y * t.gy.x + c.z * t.gz.x;
-                    const float da = inv * (t.T.x * cdot - t.sdot.x);
+                    // guarded at every pixel (see kTame)
+                    auto hit = [&](float x) { return ok[u] ? x : 0.f; };
+                    const float cdot = hit(c.x * t.gx.x + c.y * t.gy.x + c.z * t.gz.x);
+                    const float da = inv * (t.T.x * cdot - hit(t.sdot.x));
                     t.T.x *= inv;
                     const float w = al * t.T.x;
                     t.sdot.x += w * cdot;
@@ -853,10 +892,10 @@ __device__ __forceinline__ bool composite_backward_strip(
                     v[u][5] = co[u].z * sy + co[u].y * sx;
                     const float rx = v[u][4] * Wf, ry = v[u][5] * Hf;
                     v[u][6] = kRefine ? sqrtf(rx * rx + ry * ry) * t.rscale.x : 0.f;
-                    v[u][7] = kDensify ? -w * t.dmap.x : 0.f;
-                    v[u][8] = -w * t.gx.x;
-                    v[u][9] = -w * t.gy.x;
-                    v[u][10] = -w * t.gz.x;
+                    v[u][7] = kDensify ? -w * hit(t.dmap.x) : 0.f;
+                    v[u][8] = -w * hit(t.gx.x);
+                    v[u][9] = -w * hit(t.gy.x);
+                    v[u][10] = -w * hit(t.gz.x);
                     v[u][11] = kDensify ? -w : 0.f;
                 }
 #pragma unroll
@@ -864,42 +903,48 @@ __device__ __forceinline__ bool composite_backward_strip(
                     reduce_add(j[u], v[u], co[u].w);
             }
         } else {
-            while (m) {
-                const int j = 31 - __clz(int(m));
-                m ^= 1u << j;
-                const unsigned pos = unsigned(base + j);
-                const float2 xy = rec[j].xy;
-                const float4 co = rec[j].co;
-                const float4 c = rec[j].rgb;
-                const float3 nc = make_float3(-c.x, -c.y, -c.z);
-                const float dx = xy.x - fx;
-                const float xx = __fmul_rn(co.x, dx);
-                const float nxy = -__fmul_rn(co.y, dx);
-                const float ra = xx * Wf, rb = co.y * Wf, rc = -nxy * Hf, rd = co.z * Hf;
-                PairSums<kDensify> acc;
-                if ((all >> j) & 1u) {
-                    pair_adjoint<kRefine, kDensify, true>(
-                        st[0], pos, co, -co.w, nc, dx, xx, nxy, __fadd2_rn(f2s(xy.y), nfy[0]),
-                        clip, ra, rb, rc, rd, acc);
+            auto visits = [&]<bool kGuard>() {
+                while (m) {
+                    const int j = 31 - __clz(int(m));
+                    m ^= 1u << j;
+                    const unsigned pos = unsigned(base + j);
+                    const float2 xy = rec[j].xy;
+                    const float4 co = rec[j].co;
+                    const float4 c = rec[j].rgb;
+                    const float3 nc = make_float3(-c.x, -c.y, -c.z);
+                    const float dx = xy.x - fx;
+                    const float xx = __fmul_rn(co.x, dx);
+                    const float nxy = -__fmul_rn(co.y, dx);
+                    const float ra = xx * Wf, rb = co.y * Wf, rc = -nxy * Hf, rd = co.z * Hf;
+                    PairSums<kDensify> acc;
+                    if (!kGuard && ((all >> j) & 1u)) {
+                        pair_adjoint<kRefine, kDensify, true>(
+                            st[0], pos, co, -co.w, nc, dx, xx, nxy, __fadd2_rn(f2s(xy.y), nfy[0]),
+                            clip, ra, rb, rc, rd, acc);
 #pragma unroll
-                    for (int p = 1; p < NP; ++p)
-                        pair_adjoint<kRefine, kDensify, false>(
-                            st[p], pos, co, -co.w, nc, dx, xx, nxy,
-                            __fadd2_rn(f2s(xy.y), nfy[p]), clip, ra, rb, rc, rd, acc);
-                } else {
-                    acc.s = acc.sy = acc.syy = acc.refine = f2s(0.f);
-                    acc.cr = acc.cg = acc.cb = acc.dn = acc.dd = f2s(0.f);
-#pragma unroll
-                    for (int p = 0; p < NP; ++p)
-                        if ((mask[p] >> j) & 1u)
+                        for (int p = 1; p < NP; ++p)
                             pair_adjoint<kRefine, kDensify, false>(
                                 st[p], pos, co, -co.w, nc, dx, xx, nxy,
                                 __fadd2_rn(f2s(xy.y), nfy[p]), clip, ra, rb, rc, rd, acc);
+                    } else {
+                        acc.s = acc.sy = acc.syy = acc.refine = f2s(0.f);
+                        acc.cr = acc.cg = acc.cb = acc.dn = acc.dd = f2s(0.f);
+#pragma unroll
+                        for (int p = 0; p < NP; ++p)
+                            if ((mask[p] >> j) & 1u)
+                                pair_adjoint<kRefine, kDensify, false, kGuard>(
+                                    st[p], pos, co, -co.w, nc, dx, xx, nxy,
+                                    __fadd2_rn(f2s(xy.y), nfy[p]), clip, ra, rb, rc, rd, acc);
+                    }
+                    float v[12];
+                    lane_partials<kDensify>(acc, kRefine, co, dx, v);
+                    reduce_add(j, v, co.w);
                 }
-                float v[12];
-                lane_partials<kDensify>(acc, kRefine, co, dx, v);
-                reduce_add(j, v, co.w);
-            }
+            };
+            if (tame_colours(rec, cnt) && calm)
+                visits.template operator()<false>();
+            else
+                visits.template operator()<true>();
         }
         buf ^= 1;
     }
