@@ -154,8 +154,8 @@ __global__ void __launch_bounds__(kBatchEmitBlock) batch_emit_kernel(
     const BatchView* __restrict__ views, unsigned* __restrict__ keys, unsigned* __restrict__ vals,
     unsigned capacity, int bits, unsigned* __restrict__ hist) {
     __shared__ uint4 s_col[kBatchEmitBlock / 32][32 * kSpanCols];
-    __shared__ unsigned s_hist[3][kMaxRadix]; // tile ids stay below 2^27
-    DigitCounter dc(s_hist, bits);
+    __shared__ unsigned s_hist[3][kMaxRadix];
+    DigitCounter dc(s_hist, hist, bits);
     dc.zero();
     __syncthreads();
     const int warp = int(threadIdx.x >> 5);
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kBatchEmitBlock) batch_emit_kernel(
         },
         keys, vals, capacity, s_col[warp], [&](unsigned key) { dc.count(key); });
     __syncthreads();
-    dc.flush(hist);
+    dc.flush();
 }
 
 // ------------------------------------------------------------- stage 6 --
@@ -765,7 +765,7 @@ void enqueue_forward(gs_batch* b, float* color, float* alpha) {
                 b->group_shift, b->group_cap);
     const unsigned emit_blocks = (b->group_cap + kBatchEmitBlock / 32 - 1) / (kBatchEmitBlock / 32);
     // the emit counts the tile sort's digits (the depth sort's counts are done with)
-    ck(cudaMemsetAsync(hist, 0, 3 * kMaxRadix * sizeof(unsigned), s), "digit counts");
+    ck(cudaMemsetAsync(hist, 0, 4 * kMaxRadix * sizeof(unsigned), s), "digit counts");
     with_tile(b->sched.tile_w, b->sched.tile_h, [&]<int TW, int TH>() {
         batch_emit_kernel<TW, TH><<<emit_blocks, kBatchEmitBlock, 0, s>>>(
             n, b->counters, b->emit_groups, b->group_shift, b->group_cap, order, b->st, b->d_views,

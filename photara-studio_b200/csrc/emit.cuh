@@ -19,14 +19,18 @@ namespace gsb {
 // bits has 2^(9 - w) counters per bin in neighbouring banks, taken by lane:
 // neighbouring instances mostly share their high tile digit, and 32 lanes on
 // one counter are served one by one (emit at 1M / 1080p 68 us on single
-// counters of 7 + 6 bits).
-struct DigitCounter {
+// counters of 7 + 6 bits). Digits beyond the kRows that have shared counters
+// (the fourth of the emits' tile ids: 2^27 tiles and more) go to the global
+// histogram one by one.
+template <int kRows> struct DigitCounter {
     unsigned (*h)[kMaxRadix];
+    unsigned* hist; // [passes][kMaxRadix], global
     RadixPlan plan;
     int w0, c0, w1, c1; // widths and counter bits of the first two digits
     unsigned l0, l1;    // the lane's counter among a bin's
-    __device__ __forceinline__ DigitCounter(unsigned (*hist)[kMaxRadix], int bits)
-        : h(hist), plan(radix_plan(bits)) {
+    __device__ __forceinline__ DigitCounter(unsigned (&rows)[kRows][kMaxRadix],
+                                            unsigned* global, int bits)
+        : h(rows), hist(global), plan(radix_plan(bits)) {
         w0 = plan.width(0);
         c0 = kMaxDigitBits - w0;
         l0 = lane_id() & ((1u << c0) - 1u);
@@ -35,7 +39,7 @@ struct DigitCounter {
         l1 = lane_id() & ((1u << c1) - 1u);
     }
     __device__ __forceinline__ void zero() {
-        for (int k = threadIdx.x; k < plan.passes * kMaxRadix; k += blockDim.x)
+        for (int k = threadIdx.x; k < min(plan.passes, kRows) * kMaxRadix; k += blockDim.x)
             (&h[0][0])[k] = 0;
     }
     __device__ __forceinline__ void count(unsigned key) {
@@ -45,14 +49,19 @@ struct DigitCounter {
             atomicAdd(&h[1][((key << c1) & (kMaxRadix - 1)) | l1], 1u);
             for (int p = 2, at = w1; p < plan.passes; at += plan.width(p), ++p) {
                 const int c = kMaxDigitBits - plan.width(p);
-                atomicAdd(&h[p][(((key >> at) << c) & (kMaxRadix - 1)) |
-                                (lane_id() & ((1u << c) - 1u))],
-                          1u);
+                if (p < kRows)
+                    atomicAdd(&h[p][(((key >> at) << c) & (kMaxRadix - 1)) |
+                                    (lane_id() & ((1u << c) - 1u))],
+                              1u);
+                else
+                    atomicAdd(&hist[p * kMaxRadix +
+                                    ((key >> at) & ((1u << plan.width(p)) - 1u))],
+                              1u);
             }
         }
     }
-    __device__ __forceinline__ void flush(unsigned* __restrict__ hist) {
-        for (int p = 0; p < plan.passes; ++p) {
+    __device__ __forceinline__ void flush() {
+        for (int p = 0; p < min(plan.passes, kRows); ++p) {
             const int w = plan.width(p), c = kMaxDigitBits - w;
             for (int d = threadIdx.x; d < 1 << w; d += blockDim.x) {
                 unsigned v = 0;

@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kBlock) depth_compact_kernel(
     __shared__ unsigned s_hist[4][kMaxRadix];
     __shared__ unsigned s_warp[8];
     __shared__ unsigned s_tile, s_prefix;
-    DigitCounter dc(s_hist, bits);
+    DigitCounter dc(s_hist, hist, bits);
     dc.zero();
     if (threadIdx.x == 0)
         s_tile = atomicAdd(tile_counter, 1u);
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kBlock) depth_compact_kernel(
         }
     }
     __syncthreads();
-    dc.flush(hist);
+    dc.flush();
 }
 
 // Duplicate-with-keys. Warps take the visible Gaussians in depth order in
@@ -154,8 +154,8 @@ __global__ void __launch_bounds__(kEmitBlock) emit_keys_kernel(
     unsigned* __restrict__ hist) {
     // column: (first instance in the 32 Gaussians' range, first tile, tile step, Gaussian)
     __shared__ uint4 s_col[kEmitBlock / 32][32 * kSpanCols];
-    __shared__ unsigned s_hist[3][kMaxRadix]; // tile ids stay below 2^27
-    DigitCounter dc(s_hist, bits);
+    __shared__ unsigned s_hist[3][kMaxRadix];
+    DigitCounter dc(s_hist, hist, bits);
     dc.zero();
     __syncthreads();
     const int warp = int(threadIdx.x >> 5);
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kEmitBlock) emit_keys_kernel(
         r_begin, r_end, order, st, [&](unsigned) { return EmitView{grid_x, grid_y, 0u}; }, keys, values, capacity,
         s_col[warp], [&](unsigned key) { dc.count(key); });
     __syncthreads();
-    dc.flush(hist);
+    dc.flush();
 }
 
 // Per-tile [start, end) from the sorted keys. ranges[] is zeroed beforehand.
