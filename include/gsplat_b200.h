@@ -176,6 +176,8 @@ typedef struct {
 /* Creates a context on `device` enqueuing on `stream` (cudaStream_t, may be 0). */
 GS_API gs_status gs_create(gs_context** out, int device, void* stream);
 GS_API void gs_destroy(gs_context* ctx);
+/* The context's later calls go to `stream`, which first waits for the work that
+ * its calls so far left on another one (a stream being captured does not). */
 GS_API gs_status gs_set_stream(gs_context* ctx, void* stream);
 GS_API const char* gs_last_error(const gs_context* ctx);
 GS_API int gs_abi_version(void);

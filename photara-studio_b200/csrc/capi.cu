@@ -94,6 +94,8 @@ struct gs_context {
     cudaEvent_t ev[2][16] = {}; // stage k: begin 2k, end 2k+1
     cudaEvent_t ev_counts = nullptr; // the draw-count read-back of the forward
     cudaEvent_t ev_sorted = nullptr; // the error word read back after the forward's sorts
+    cudaEvent_t ev_left = nullptr;   // the end of the last call's work on its stream
+    bool left = false;               // ev_left has been recorded
     int ev_set = 0;
     bool ev_pending = false;
     double acc_ms[8] = {};
@@ -102,9 +104,36 @@ struct gs_context {
 
 namespace {
 
-template <typename F> gs_status guarded(gs_context* ctx, F&& f) {
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
+        cudaGetLastError(); // the legacy stream while another one is captured
+        return true;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
+// Records where a call's work ends, so that another stream can wait for it
+// without touching this one, which may be gone or in a capture by then. (A
+// captured call leaves nothing in flight.)
+struct MarkLeft {
+    gs_context* c;
+    bool enqueues;
+    ~MarkLeft() {
+        if (!enqueues || !c->ev_left || capturing(c->stream))
+            return;
+        if (cudaEventRecord(c->ev_left, c->stream) == cudaSuccess)
+            c->left = true;
+        else
+            cudaGetLastError();
+    }
+};
+
+// enqueues: the call puts work on the stream.
+template <typename F> gs_status guarded(gs_context* ctx, F&& f, bool enqueues = true) {
     if (!ctx)
         return GS_ERR_INVALID;
+    MarkLeft mark{ctx, enqueues};
     try {
         ck(cudaSetDevice(ctx->device), "cudaSetDevice");
         f();
@@ -297,6 +326,7 @@ gs_status gs_create(gs_context** out, int device, void* stream) {
                 ck(cudaEventCreate(&e), "event create");
         ck(cudaEventCreateWithFlags(&c->ev_counts, cudaEventDisableTiming), "event create");
         ck(cudaEventCreateWithFlags(&c->ev_sorted, cudaEventDisableTiming), "event create");
+        ck(cudaEventCreateWithFlags(&c->ev_left, cudaEventDisableTiming), "event create");
     });
     if (st != GS_OK) {
         gs_destroy(c);
@@ -329,11 +359,30 @@ void gs_destroy(gs_context* c) {
         cudaEventDestroy(c->ev_counts);
     if (c->ev_sorted)
         cudaEventDestroy(c->ev_sorted);
+    if (c->ev_left)
+        cudaEventDestroy(c->ev_left);
     delete c;
 }
 
 gs_status gs_set_stream(gs_context* c, void* stream) {
-    return guarded(c, [&] { c->stream = static_cast<cudaStream_t>(stream); });
+    if (!c)
+        return GS_ERR_INVALID;
+    const cudaStream_t next = static_cast<cudaStream_t>(stream);
+    if (next == c->stream)
+        return GS_OK;
+    cudaSetDevice(c->device);
+    // the workspace may still be in use on the stream before
+    if (c->left && !capturing(next)) {
+        const cudaError_t e = cudaStreamWaitEvent(next, c->ev_left, 0);
+        if (e != cudaSuccess) {
+            c->error = std::string("gsplat_b200: wait for the last stream: ") +
+                       cudaGetErrorString(e);
+            return GS_ERR_CUDA;
+        }
+    }
+    c->stream = next;
+    c->error.clear();
+    return GS_OK;
 }
 
 const char* gs_last_error(const gs_context* c) { return c ? c->error.c_str() : "null context"; }
@@ -753,7 +802,7 @@ gs_status gs_set_schedule(gs_context* c, int pixels_per_thread) {
                 pixels_per_thread == 4 || pixels_per_thread == 8,
             "pixels_per_thread must be 0 (automatic), 1, 2, 4 or 8");
         c->pixels_per_thread = pixels_per_thread;
-    });
+    }, /*enqueues=*/false);
 }
 
 gs_status gs_debug_draw_list(gs_context* c, unsigned long long* keys_out, unsigned* values_out,
@@ -787,7 +836,7 @@ gs_status gs_enable_stage_timing(gs_context* c, int enable) {
         for (double& v : c->acc_ms)
             v = 0.0;
         c->acc_steps = 0;
-    });
+    }, /*enqueues=*/false);
 }
 
 gs_status gs_stage_times(gs_context* c, float* ms_out, int n) {

@@ -144,17 +144,13 @@ class _Context:
     def __init__(self, pool: "_ContextPool"):
         self.pool = pool
         self.ptr = C.c_void_p()
-        self.stream = None  # the stream of its last use
         lib = L.load()
         L.check(lib.gs_create(C.byref(self.ptr), pool.device, None), None)
 
     def bind_stream(self) -> None:
-        stream = torch.cuda.current_stream(self.pool.device)
-        if self.stream is not None and self.stream != stream and \
-                not torch.cuda.is_current_stream_capturing():
-            stream.wait_stream(self.stream)  # the workspace may still be in use there
-        self.stream = stream
-        L.check(L.load().gs_set_stream(self.ptr, C.c_void_p(stream.cuda_stream)), self.ptr)
+        # waits for what the context's last call left on another stream
+        stream = torch.cuda.current_stream(self.pool.device).cuda_stream
+        L.check(L.load().gs_set_stream(self.ptr, C.c_void_p(stream)), self.ptr)
 
     def release(self) -> None:
         self.pool.give_back(self)
