@@ -110,7 +110,9 @@ __global__ void __launch_bounds__(kThreads) image_loss_kernel(LossArgs a) {
     __shared__ float3 s_dy[kRh * kRw], s_dx[kRh * kRw], s_n[kRh * kRw];
     __shared__ float s_loss[kRh * kRw];
     const size_t pixels = size_t(a.im.width) * a.im.height;
-    const int x0 = int(blockIdx.x) * kTw, y0 = int(blockIdx.y) * kTh;
+    // one grid dimension, row by row (a second one ends at 65,535 blocks)
+    const unsigned across = unsigned(a.im.width + kTw - 1) / kTw;
+    const int x0 = int(blockIdx.x % across) * kTw, y0 = int(blockIdx.x / across) * kTh;
     const int tx0 = int(threadIdx.x) % kTw, ty0 = int(threadIdx.x) / kTw;
     const int x = x0 + tx0, y = y0 + ty0;
     const size_t pixel = size_t(y) * a.im.width + x;
@@ -239,7 +241,7 @@ __global__ void __launch_bounds__(kThreads) image_loss_kernel(LossArgs a) {
         float s = 0.f;
         for (int w = 0; w < kThreads / 32; ++w)
             s += s_terms[w][threadIdx.x];
-        a.partial[(size_t(blockIdx.y) * gridDim.x + blockIdx.x) * 4 + threadIdx.x] = s;
+        a.partial[size_t(blockIdx.x) * 4 + threadIdx.x] = s;
     }
 }
 
@@ -272,11 +274,11 @@ size_t image_loss_partial_floats(int width, int height) {
 cudaError_t launch_image_loss(cudaStream_t s, const ImageLossImages& im,
                               const ImageLossOptions& o, const ImageLossOutputs& out,
                               float photo_weight, float* partial) {
-    const dim3 grid((im.width + kTw - 1) / kTw, (im.height + kTh - 1) / kTh);
+    const unsigned blocks = unsigned(image_loss_partial_floats(im.width, im.height) / 4);
     LossArgs a{im, o, out, photo_weight, out.terms ? partial : nullptr};
-    image_loss_kernel<<<grid, kThreads, 0, s>>>(a);
+    image_loss_kernel<<<blocks, kThreads, 0, s>>>(a);
     if (out.terms)
-        reduce_terms_kernel<<<1, 1024, 0, s>>>(partial, int(grid.x * grid.y), out.terms);
+        reduce_terms_kernel<<<1, 1024, 0, s>>>(partial, int(blocks), out.terms);
     return cudaGetLastError();
 }
 

@@ -148,3 +148,18 @@ def test_deterministic_and_validated():
     with pytest.raises(Exception, match="depth term needs"):
         gsb.compute_training_loss(c["color"], c["target_color"],
                                   options=gsb.TrainingLossOptions(depth_weight=1.0))
+
+
+def test_more_rows_of_blocks_than_a_second_grid_dimension():
+    """65,538 rows of 32 x 8 blocks; ten pixels or fewer across, so without the
+    SSIM term. Bars as against float64 above."""
+    cfg = CONFIGS["masked_geometry"]
+    c = _case(3, 524_300, 21)
+    ours = _run_ours(c, cfg)
+    np_in = {k: (v.cpu().numpy() if torch.is_tensor(v) else v) for k, v in _kwargs(c, cfg).items()}
+    exp = loss_ref.training_loss(c["color"].cpu().numpy(), c["target_color"].cpu().numpy(),
+                                 **np_in)
+    for key in ("color", "alpha", "depth", "normal"):
+        got = getattr(ours, key).cpu().numpy().astype(np.float64)
+        assert np.abs(got - exp[key]).max() <= 2e-4 * np.abs(exp[key]).max(), key
+    assert np.allclose(ours.terms.cpu().numpy(), exp["terms"], rtol=2e-5, atol=1e-8)
