@@ -304,7 +304,7 @@ __device__ __forceinline__ ShAdamConsts sh_adam_consts(const ShAdamArgs& a) {
     k.eps = a.epsilon;
     k.lr = a.lr;
     k.rest_lr = a.rest_lr;
-    k.reg = a.regularization;
+    k.reg = fmaxf(a.regularization, 0.f); // a negative factor or a NaN is no term
     return k;
 }
 

@@ -50,3 +50,36 @@ def test_thread_rows_match_half_warp_rows(n):
     assert bool(((f0 - f1).abs() <= 1e-3 * f0.abs() + 1e-7).all())
     assert int((c0 - c1).abs().max()) <= 1
     assert not torch.equal(p0, model.sh)
+
+
+@pytest.mark.parametrize("move", [lambda t: t.clone(), unaligned])
+def test_a_negative_regularization_factor_is_no_term(monkeypatch, move):
+    """In both layouts; the C ABI takes the factor as it is (the Python layer
+    passes none below 0)."""
+    n = 200
+    scene = gsb.make_scene("tiny", seed=4, count=n)
+    cam = camera_of(scene)
+    g = torch.Generator("cuda").manual_seed(4)
+    state = dict(first=(0.3 * torch.randn((n, 16, 3), device="cuda", generator=g)).half(),
+                 packed=torch.randint(0, 256, (n, 16, 3), device="cuda", generator=g,
+                                      dtype=torch.uint8),
+                 bounds=torch.tensor([18.0, 20.0, 18.0, 21.0], device="cuda").repeat(n, 1))
+    grad = torch.randn((3, cam.height, cam.width), device="cuda", generator=g) * 1e-3
+
+    class Negative(gsb._lib.ShAdam):
+        def __setattr__(self, name, value):
+            super().__setattr__(name, -0.5 if name == "regularization_factor" else value)
+
+    out = []
+    for cls in (gsb._lib.ShAdam, Negative):
+        monkeypatch.setattr(gsb._lib, "ShAdam", cls)
+        m = device_model(scene)
+        m.sh = move(m.sh)
+        st = {k: move(v) if k != "bounds" else v.clone() for k, v in state.items()}
+        rast = gsb.Rasterizer()
+        r = rast.forward(m, cam, gsb.RasterizeOptions(active_sh_degree=3))
+        rast.backward(m, r, grad, None, sh_adam=gsb.SHAdamUpdate(
+            **st, lr=5e-3, rest_lr=1e-3, correction1=0.8, correction2=0.3))
+        out.append((m.sh, st["bounds"]))
+    assert float((out[0][0] - out[1][0]).abs().max()) <= 1e-6
+    assert float((out[0][1] - out[1][1]).abs().max()) <= 1e-5
