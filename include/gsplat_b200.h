@@ -562,9 +562,11 @@ typedef struct gs_batch gs_batch;
 
 typedef struct {
     int tile_w, tile_h;       /* 8x8, 16x16 or 16x32 (width x height) */
-    int pixels_per_thread;    /* 1|2 for 8x8, 2|4 for 16x16 and 16x32 */
+    int pixels_per_thread;    /* 1|2 for 8x8, 2|4 for 16x16 and 16x32; 4 runs as 8 once the
+                                 views hold the pixels of more than 4,800 16x16 tiles */
     int schedule;             /* 0 static stride, 1 dynamic queue, 2 heaviest tiles first */
-    int ctas_per_sm;          /* persistent CTAs per SM; 0 = as many as fit */
+    int ctas_per_sm;          /* tiles in flight per SM (a tile's strips are one-warp CTAs);
+                                 0 = as many as fit */
 } gs_batch_schedule;
 
 typedef struct {
@@ -605,7 +607,8 @@ GS_API gs_status gs_batch_capture(gs_batch* b, float* color, float* alpha, int* 
                                   const gs_model_grads* grads);
 GS_API gs_status gs_batch_replay(gs_batch* b);
 /* Times forward + backward (CUDA events, `iterations` after 2 warm-ups) for
- * every tile shape / pixels-per-thread / schedule candidate, plans the fastest
+ * every tile shape / pixels-per-thread / schedule candidate (as given: 4 pixels
+ * per thread may have run as 8, see gs_batch_schedule), plans the fastest
  * and returns it in *best (*best_ms its time). tried / tried_ms (capacity
  * *n_tried on entry, count on return) receive every candidate; may be NULL. */
 GS_API gs_status gs_batch_autotune(gs_batch* b, const gs_gaussians* g, const gs_camera* cams,

@@ -30,11 +30,13 @@ _SCHEDULE_NAMES = {v: k for k, v in SCHEDULES.items()}
 
 @dataclass
 class BatchSchedule:
+    """Four pixels per thread run as eight once the views hold the pixels of
+    more than 4,800 16x16 tiles (`tuning` lists what was asked for)."""
     tile_w: int = 16
     tile_h: int = 16
     pixels_per_thread: int = 4
     schedule: str = "dynamic"   # static | dynamic | heavy_first
-    ctas_per_sm: int = 0        # 0: as many as fit
+    ctas_per_sm: int = 0        # tiles in flight per SM; 0: as many as fit
 
     def struct(self) -> L.BatchSchedule:
         return L.BatchSchedule(self.tile_w, self.tile_h, self.pixels_per_thread,

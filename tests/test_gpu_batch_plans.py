@@ -1,5 +1,6 @@
-"""Several batched plans alive at once on one device (tolerances of
-test_gpu_batch.py)."""
+"""Batched rendering where plans meet: several plans alive at once, and views
+of enough tiles (above 4,800 of 16x16) that four pixels per thread run as
+eight, against the single-view path (tolerances of test_gpu_batch.py)."""
 import importlib
 
 import numpy as np
@@ -54,3 +55,40 @@ def test_a_later_plan_of_fewer_views_leaves_an_earlier_one_usable(sh_bases):
     for name in NAMES:
         assert rel_l2(getattr(after, name), getattr(before, name)) <= 2e-5, name
         assert rel_l2(getattr(first.grads, name), getattr(before, name)) <= 2e-5, name
+
+
+@pytest.mark.parametrize("tw,th,sched,capacity", [
+    (16, 16, "dynamic", 0), (16, 32, "static", 0),
+    (16, 16, "heavy_first", 0),        # the order lists in a buffer of their own
+    (16, 32, "heavy_first", 1 << 21),  # the order lists in the sort's spare keys
+])
+def test_eight_pixels_per_thread_match_single_views(tw, th, sched, capacity):
+    sizes = ((701, 903), (803, 717), (333, 211))
+    model, cams = _setup(4000, 6, sizes, 4)
+    tiles16 = sum(-(-c.width // 16) * -(-c.height // 16) for c in cams)
+    tiles = sum(-(-c.width // tw) * -(-c.height // th) for c in cams)
+    assert tiles * tw * th // 256 > 4800 and tiles16 > 4800
+    opts = gsb.RasterizeOptions(active_sh_degree=3)
+    br = batch.BatchRasterizer().plan(model, cams, opts, batch.BatchSchedule(tw, th, 4, sched),
+                                      instance_capacity=capacity)
+    res = br.forward()
+    g = torch.Generator("cuda").manual_seed(2)
+    flat = torch.randn(res.color.numel(), device="cuda", generator=g) * 1e-3
+    grads = br.backward(flat)
+    info = br.info()
+    assert info["overflow"] == 0 and info["device_error"] == 0
+    # counts and lists of both orders: 64 classes of the tiles and of the strips
+    strips = th // 16 * tiles
+    assert sched != "heavy_first" or \
+        (64 * (tiles + strips) <= info["instance_capacity"]) == (capacity > 0)
+    rast, total = gsb.Rasterizer(), {}
+    for k, cam in enumerate(cams):
+        r = rast.forward(model, cam, opts)
+        assert float((res.view_color(k) - r.color).abs().max()) <= 1e-6
+        assert float((res.view_alpha(k) - r.alpha).abs().max()) <= 1e-6
+        w, h, off = res.views[k]
+        one = rast.backward(model, r, flat[3 * off:3 * (off + w * h)].view(3, h, w).contiguous())
+        for name in NAMES:
+            total[name] = total.get(name, 0) + getattr(one, name)
+    for name in NAMES:
+        assert rel_l2(getattr(grads, name), total[name]) <= 2e-5, name
