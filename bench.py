@@ -258,8 +258,8 @@ def max_over_ranks(v: float, world: int) -> float:
 
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of these
-# kernels on this workload, from one ncu capture of the same build (not
-# measured by this run); close to the algorithmic bytes, i.e. no re-reads.
+# kernels on this workload, from one ncu capture (not measured by this run);
+# the Gaussian backward's are 8% above its algorithmic bytes (it spills).
 NCU_TRAFFIC_BYTES = {"gaussian_backward_adam": 1_207_971_584, "preprocess": 222_083_072}
 
 # FP32 work of the compositing kernels per evaluated (Gaussian, pixel) pair:

@@ -8,8 +8,9 @@
 //   backward: composite adjoint -> per-Gaussian adjoint (+ fused Adam)
 // Differences by design: the context owns a grow-only workspace instead of
 // caller pool callbacks, every launch goes to the context stream, the camera
-// travels by value, and no snapshot/bucket state is kept (the backward
-// recomputes transmittance per tile from the stored final T).
+// travels by value, and the backward recovers the transmittance per strip from
+// the stored final T instead of bucket snapshots (frames of up to kSegmentTiles
+// tiles store checkpoints of the list segments, strip.cuh).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>

@@ -10,7 +10,8 @@
 namespace gsb {
 
 // Resident warps per SM that the strip kernels are compiled for: the register
-// budget of each pixels-per-thread count without spills.
+// budget of each pixels-per-thread count without spills (the guarded and the
+// counting forward at eight spill 8 bytes).
 template <int PX> constexpr int kForwardCtas = PX == 8 ? 20 : PX == 4 ? 28 : 32;
 template <int PX> constexpr int kBackwardCtas = PX == 8 ? 16 : PX == 4 ? 20 : 24;
 
@@ -112,7 +113,7 @@ static StripOrder strip_order(unsigned* words, int tiles, int pixels_per_thread)
 
 // Test hook for the staging wait: one CTA announces 256 bytes on its
 // mbarrier that no copy delivers, waits at most `limit` suspended waits
-// (as stage_any does), and reports the timeout as stage_any does.
+// (as StripFeed::wait does), and reports the timeout as it does.
 __global__ void stage_probe_kernel(unsigned limit, unsigned* __restrict__ err) {
     __shared__ unsigned long long bar;
     if (threadIdx.x == 0)
@@ -185,7 +186,9 @@ constexpr int kGeoThreads = kTileW * kTileH;
 // walks of the list / keeping 48, 64, 96, 128: 500,000 at 1280x720 1,755 /
 // 1,185, 1,177, 1,180, 1,177; 50,000 dense at 1280x960 2,285 / 2,364, 1,981,
 // 1,952-1,966, 1,977; 200,000 at 700x500 1,263 / 746, 744, 733, 733 (with too
-// few, most blocks hold a pixel that has to walk its list again).
+// few, most blocks hold a pixel that has to walk its list again). The 1,152-byte
+// frames take some 350 MB of the device when the kernel first runs (the driver
+// sizes local memory by the threads that can be resident).
 constexpr int kNear = 96;
 
 __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(
@@ -768,7 +771,10 @@ void launch_composite_backward_geometry(cudaStream_t s, int tiles, const uint2* 
         else
             go(composite_backward_geometry_kernel<PX, false, false>);
     };
-    // more strips where there are too few tiles to fill the GPU
+    // more strips where there are too few tiles to fill the GPU; us at two /
+    // four pixels per thread: 256 tiles 298 / 461, 690 tiles 222 / 297, 1,200
+    // tiles 458 / 439, 1,900 tiles 648 / 667, 3,600 tiles 769 / 723, 8,160 tiles
+    // 1,335 / 1,203
     if (tiles <= 1000)
         bwd.template operator()<2>();
     else

@@ -23,9 +23,10 @@
 // and 96 registers give 5 CTAs, 20 warps, per SM); other strides and degrees
 // one half-warp per row with everything staged (440 bytes: 4 CTAs).
 // Bound: the latency of its loads and of the codec's chains at 20 warps per
-// SM, half issue; it moves its algorithmic bytes. 1M / 1080p 306 -> 268 us,
+// SM, half issue; it moves 1,208 MB for 1,116 MB of algorithmic bytes (96
+// registers spill 44 bytes a thread). 1M / 1080p 306 -> 268 us,
 // 8.4M / 2160p 2,364 -> 2,006 us (4.4 TB/s) against the layout with every row
-// staged at 4 CTAs; 4 CTAs 275 us, 6 CTAs (80 registers, spills) 308 us, CTAs
+// staged at 4 CTAs; 4 CTAs 275 us, 6 CTAs (80 registers, more spills) 308 us, CTAs
 // of 64 and 32 rows 267 and 286 us (2,040 and 2,209 us at 8.4M).
 #include <cuda_fp16.h>
 
@@ -1095,7 +1096,7 @@ __global__ void __launch_bounds__(kRows48 ? kRowsBlock : kGBlock,
     }
 }
 
-size_t gaussian_backward_smem(bool fused_sh, bool rows48) {
+static size_t gaussian_backward_smem(bool fused_sh, bool rows48) {
     if (rows48)
         return size_t(kRowsBlock) * (kRowStride + kWdlStride) * sizeof(float);
     if (!fused_sh)

@@ -158,8 +158,10 @@ cudaError_t launch_pruning_scores(cudaStream_t s, int tiles, const uint2* ranges
         kernel<<<tiles * (8 / PX), 32, 0, s>>>(rs.map, rs.err, ranges, order, pix_last, image,
                                                K.width, K.height, K.grid_x, K.alpha_clip, scores);
     };
-    // more strips where there are too few tiles to fill the GPU, as the
-    // compositing kernels
+    // more strips where there are too few tiles to fill the GPU; us at two / four
+    // / eight pixels per thread: 256 tiles 123 / 173 / 271, 690 tiles 75 / 93 /
+    // 133, 1,200 tiles 131 / 140 / 183, 1,900 tiles 204 / 187 / 215, 3,600 tiles
+    // 210 / 181 / 197, 5,700 tiles 286 / 239 / 242, 8,160 tiles 348 / 279 / 272
     if (tiles <= 1000)
         go.template operator()<2>();
     else if (tiles <= 4800)

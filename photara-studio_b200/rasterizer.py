@@ -272,7 +272,8 @@ class Rasterizer:
     """Drop-in for photara::splat::Rasterizer (CUDA 3DGS pinhole RGB path).
 
     pixels_per_thread selects the compositing schedule (1, 2, 4 or 8; None =
-    chosen per frame from its tile count); results do not depend on it."""
+    chosen per frame from its tile count); images do not depend on it, gradients
+    to rounding."""
 
     def __init__(self, pixels_per_thread: Optional[int] = None):
         self.pixels_per_thread = pixels_per_thread
