@@ -181,8 +181,8 @@ GS_API void gs_destroy(gs_context* ctx);
 GS_API gs_status gs_set_stream(gs_context* ctx, void* stream);
 GS_API const char* gs_last_error(const gs_context* ctx);
 GS_API int gs_abi_version(void);
-/* Bytes of device workspace currently held by the context (without the local
- * memory that the driver keeps for the geometry forward, some 350 MB). */
+/* Bytes of device workspace currently held by the context (without the 40 MB by
+ * which the geometry forward's first launch enlarges the driver's local memory). */
 GS_API size_t gs_workspace_bytes(const gs_context* ctx);
 
 /* ---- rasterizer boundary (api.h:246, :264) ------------------------------------ */

@@ -187,8 +187,8 @@ constexpr int kGeoThreads = kTileW * kTileH;
 // 1,185, 1,177, 1,180, 1,177; 50,000 dense at 1280x960 2,285 / 2,364, 1,981,
 // 1,952-1,966, 1,977; 200,000 at 700x500 1,263 / 746, 744, 733, 733 (with too
 // few, most blocks hold a pixel that has to walk its list again). The 1,152-byte
-// frames take some 350 MB of the device when the kernel first runs (the driver
-// sizes local memory by the threads that can be resident).
+// frames are above the default stack of 1,024 and make the driver enlarge its
+// local memory by 40 MB when the kernel first runs.
 constexpr int kNear = 96;
 
 __global__ void __launch_bounds__(kGeoThreads) composite_geometry_kernel(

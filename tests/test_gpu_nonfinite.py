@@ -1,6 +1,7 @@
 """Infinities and NaN reach only the pixels and Gaussians they are blended
 into: a Gaussian or pixel that does not take part keeps its value (images bit
 for bit; gradients to the order of float atomics, 1e-5 of the largest)."""
+import dataclasses
 import importlib
 
 import pytest
@@ -22,6 +23,9 @@ class _Case:
 
     def __init__(self, ppt, seed, **options):
         scene = gsb.make_scene("tiny", seed=seed)
+        if ppt == "690 tiles":  # the automatic schedule's two pixels, in segments
+            scene, ppt = dataclasses.replace(scene, width=480, height=368, cx=240.0, cy=184.0,
+                                             fx=400.0, fy=400.0), None
         self.model, self.cam = device_model(scene), camera_of(scene)
         self.rast, self.options = gsb.Rasterizer(pixels_per_thread=ppt), options
         self.n = self.model.size()
@@ -58,7 +62,7 @@ def _same(a, b, rows, names):
 
 
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
-@pytest.mark.parametrize("ppt", [1, 2, 4, 8, None])
+@pytest.mark.parametrize("ppt", [1, 2, 4, 8, None, "690 tiles"])
 def test_colour_that_is_not_finite(ppt, value):
     c = _Case(ppt, 5)
     k = c.middle()
@@ -80,7 +84,7 @@ def test_colour_that_is_not_finite(ppt, value):
 
 
 @pytest.mark.parametrize("geometry", [False, True])
-@pytest.mark.parametrize("ppt", [1, 2, 4, 8, None])
+@pytest.mark.parametrize("ppt", [1, 2, 4, 8, None, "690 tiles"])
 def test_pixel_gradient_that_is_not_finite(ppt, geometry):
     c = _Case(ppt, 6, require_depth=geometry)
     r = c.render(c.colors)
