@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kBlock) batch_preprocess_kernel(
     store_records(s_rec + warp0, touched > 0, rec,
                   st.rec + size_t(v) * size_t(n) + blockIdx.x * blockDim.x + warp0);
     if (touched > 0 && !finite_colour(rec.rgb))
-        atomicOr(&counters[kBcWild], 1u);
+        counters[kBcWild] = 1u; // every writer stores the same
     const unsigned w_inst = __reduce_add_sync(0xffffffffu, touched);
     const unsigned w_vis = __popc(__ballot_sync(0xffffffffu, touched > 0));
     if (lane_id() == 0 && w_vis) {

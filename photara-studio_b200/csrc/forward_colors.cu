@@ -23,7 +23,7 @@ __global__ void __launch_bounds__(256) set_colors_kernel(int n, const float* __r
                                      colors[3 * size_t(i) + 2], __uint_as_float(0u));
         rec[i].rgb = c;
         if (!finite_colour(c))
-            atomicOr(wild, 1u);
+            *wild = 1u; // every writer stores the same
     }
 }
 

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kBlock) preprocess_kernel(
     store_records(s_rec + warp0, touched > 0, rec, st.rec + blockIdx.x * blockDim.x + warp0);
     const unsigned full = 0xffffffffu;
     if (touched > 0 && !finite_colour(rec.rgb))
-        atomicOr(&counters[8], 1u);
+        counters[8] = 1u; // every writer stores the same
     const unsigned w_inst = __reduce_add_sync(full, touched);
     const unsigned w_vis = __popc(__ballot_sync(full, touched > 0));
     const unsigned w_min = __reduce_min_sync(full, touched > 0 ? depth_bits : 0xffffffffu);
